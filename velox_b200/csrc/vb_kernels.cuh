@@ -92,6 +92,8 @@ struct GemvArgs {
     unsigned long long* trace = nullptr;  // 3-slot timestamp record of this launch (tuned kernels only)
 };
 cudaError_t gemv(const LaunchCfg& lc, const GemvArgs& a, int path);
+// vb_gemv_canon.cu: every format from its canonical layout, fp32 arithmetic
+cudaError_t gemv_canon(const LaunchCfg& lc, const GemvArgs& a);
 
 // vb_gemv_fast.cu
 bool tile_q4_supported(uint32_t rows, uint32_t K);
