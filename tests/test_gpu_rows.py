@@ -1,10 +1,51 @@
-"""Matrix-vector products of every format against exact sums, at the sizes where their row groups and passes end."""
+"""Products of a few rows of x (mma.sync kernel) and single rows of every format: one decode step of a batch against the
+CPU checker, at the sizes where tiles, column groups, weight passes and cluster splits end."""
 import numpy as np
 import pytest
 
+import helpers as H
 from oracle import oracle as O
+from velox_b200 import lib as L
+from velox_b200.modelspec import LLAMA3_8B_INT4
 
 pytestmark = pytest.mark.gpu
+
+# 2^-11 of an fp16 cache and of nothing else: logits of N(0, 0.02) heads over unit rows of 512 stay below ~2.5, two layers
+TOL = 5e-3
+FMTS = {"q4g32": (L.FMT_Q4G32, L.FMT_F16), "q4_0": (L.FMT_Q4G64REF, L.FMT_Q4G64REF), "f16": (L.FMT_F16, L.FMT_F16), "bf16": (L.FMT_BF16, L.FMT_BF16),
+        "f32": (L.FMT_F32, L.FMT_F32)}
+
+
+@pytest.mark.parametrize("fmt", sorted(FMTS))
+@pytest.mark.parametrize("batch", [1, 2, 3, 5, 9, 17])
+def test_batch_step_matches_checker(fmt, batch):
+    w, emb = FMTS[fmt]
+    # K of 512 and 1408 (11 blocks of 128: not a multiple of any split), 4112 head rows (257 tiles of 16)
+    spec = LLAMA3_8B_INT4.scaled(name="rows-" + fmt, d_model=512, n_layers=2, n_q_heads=8, n_kv_heads=2, head_dim=64, ffn_dim=1408, vocab=4112,
+                                 weight_fmt=w, head_fmt=w, embed_fmt=emb)
+    eng = H.build_engine(spec, 31, 32, max_batch=batch)
+    rng = np.random.default_rng(batch)
+    prompts = [rng.integers(0, spec.vocab, size=1 + i % 5).astype(np.uint32) for i in range(batch)]
+    toks = rng.integers(0, spec.vocab, size=batch)
+    for slot, p in enumerate(prompts):
+        eng.reserve(slot, 32)
+        eng.prefill(p, slot)
+    for slot, p in enumerate(prompts):
+        if slot % 4 != 3 or batch < 4:  # every fourth slot sits the step out
+            eng.set_state(slot, int(toks[slot]), len(p))
+        else:
+            eng.set_state(slot, 0, len(p), False)
+    eng.decode(1)
+    for slot in sorted({0, batch // 2, batch - 1}):
+        if slot % 4 == 3 and batch >= 4:
+            continue
+        ora, _ = H.build_oracle(spec, 31, 32)
+        for pos, t in enumerate(prompts[slot]):
+            ora.forward_step(int(t), pos)
+        ora.forward_step(int(toks[slot]), len(prompts[slot]))
+        assert float(np.max(np.abs(eng.logits(slot) - ora.logits))) <= TOL, (fmt, batch, slot)
+    eng.close()
+
 
 @pytest.mark.parametrize("fmt", ["f32", "f16", "bf16", "q4g32", "q4g64ref", "i8pc"])
 @pytest.mark.parametrize("in_dim,out_dim,batch", [(64, 1, 1), (64, 7, 2), (576, 33, 1), (1088, 130, 8), (2112, 5, 11), (8192, 19, 4)])

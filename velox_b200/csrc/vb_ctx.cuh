@@ -106,6 +106,8 @@ struct vb_ctx {
     // activations
     float *hidden = nullptr, *qkv = nullptr, *q = nullptr, *attn_out = nullptr, *act = nullptr, *logits = nullptr;
     float* attn_scratch = nullptr;
+    unsigned char* frag_ws = nullptr;  // x of a product in fragment order (vb_gemv_mma.cu)
+    uint64_t frag_ws_bytes = 0;
     float* cand_v = nullptr;
     uint32_t* cand_i = nullptr;
 

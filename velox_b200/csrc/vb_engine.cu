@@ -70,7 +70,9 @@ void set_tied_head(vb_ctx* c) {
     h.m.rows = c->vocab;
     h.m.data = (const unsigned char*)h.m.data + wmat_data_bytes(h.m.fmt, c->vocab_off, h.m.cols);
     if (h.m.scales) h.m.scales = (const unsigned char*)h.m.scales + wmat_scale_bytes(h.m.fmt, c->vocab_off, h.m.cols);
-    h.m.tiled = h.m.tiled_scales = h.m.v3 = h.m.v3_scales = nullptr;
+    h.m.tiled = h.m.tiled_scales = h.m.v3_scales = nullptr;
+    // the int4 tiles of the whole table are the head's (a rank's slice has none of its own)
+    if (c->d.tp_size > 1 || !(h.m.fmt == VB_FMT_Q4G32 || h.m.fmt == VB_FMT_Q4G64REF)) h.m.v3 = nullptr;
 }
 
 // Lay the arena out in execution order.  Wq|Wk|Wv (and their scales) are adjacent so that the fused QKV
@@ -84,15 +86,16 @@ int32_t plan_arena(vb_ctx* c) {
     const bool lean = (c->d.flags & VB_FLAG_LEAN_WEIGHTS) != 0;
     auto add_group = [&](std::initializer_list<int> roles, int layer) {
         std::vector<Slot> g;
-        bool tile_all = true, i8_all = true;  // all members int4 g32 / all int8 per-channel, in tileable shapes
+        bool tile_all = true, i8_all = true;  // all members int4 (group-64: not in a lean arena) / all int8 per-channel, in tileable shapes
         for (int role : roles) {
             uint32_t rows, cols; int32_t fmt;
             if (!role_shape(c, role, &rows, &cols, &fmt)) continue;
             Tensor& t = c->tensor(role, layer);
             t.m.fmt = fmt; t.m.rows = rows; t.m.cols = cols;
             g.push_back({role, layer, ~0ULL, ~0ULL, 0, 0, ~0ULL, false});
-            if (fmt != VB_FMT_Q4G32 || !tile_q4_supported(rows, cols)) tile_all = false;
+            if (!(fmt == VB_FMT_Q4G32 || (fmt == VB_FMT_Q4G64REF && !lean)) || !tile_q4_supported(rows, cols)) tile_all = false;
             if (fmt != VB_FMT_I8PC || !tile_q4_supported(rows, cols)) i8_all = false;
+            if (role == VB_ROLE_EMBED && !c->d.tied_lm_head) tile_all = i8_all = false;  // rows are looked up, never multiplied
         }
         if (g.empty()) return;
         const bool lean_group = lean && (tile_all || i8_all);  // only the integer tensor-core layout is kept
@@ -116,7 +119,7 @@ int32_t plan_arena(vb_ctx* c) {
             off = align256(off);
         }
         if (tile_all) {
-            if (!lean_group) {
+            if (!lean_group && c->tensor(g[0].role, layer).m.fmt == VB_FMT_Q4G32) {
                 // tile-major copies for the fp16 tensor-core kernel, members adjacent again (fused QKV = one tiled matrix)
                 for (Slot& s : g) { s.has_tiled = true; s.tiled = off; s.tiled_scales = off; off += packed_bytes(s); }
                 off = align256(off);
@@ -157,9 +160,10 @@ int32_t plan_arena(vb_ctx* c) {
                 swiglu_v3_off.push_back(off);
                 off += 2 * (wmat_data_bytes(tg.m.fmt, tg.m.rows, tg.m.cols) + wmat_scale_bytes(tg.m.fmt, tg.m.rows, tg.m.cols));
                 off = align256(off);
-            } else if (tg.m.fmt == VB_FMT_I8PC && tile_q4_supported(tg.m.rows, tg.m.cols)) {
+            } else if ((tg.m.fmt == VB_FMT_I8PC && tile_q4_supported(tg.m.rows, tg.m.cols)) ||
+                       (tg.m.fmt == VB_FMT_Q4G64REF && !lean && tg.m.rows % 8 == 0 && tg.m.cols % 128 == 0)) {
                 swiglu_off.push_back(~0ULL);
-                swiglu_v3_off.push_back(off);  // 2*rows x cols of blocks, then 2*rows scales
+                swiglu_v3_off.push_back(off);  // 2*rows x cols of blocks (int8: then 2*rows scales)
                 off += 2 * (wmat_data_bytes(tg.m.fmt, tg.m.rows, tg.m.cols) + wmat_scale_bytes(tg.m.fmt, tg.m.rows, tg.m.cols));
                 off = align256(off);
             } else {
@@ -422,7 +426,9 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
     auto product = [&](const GemvArgs& ga) -> cudaError_t {
         if (io.i8_ws && gemm_i8_supported(ga)) return gemm_i8(lcfg(c, true), ga, io.i8_ws, io.i8_ws_bytes, true);
         if (io.tc_ws) return gemm_tc(lcfg(c, true), ga, io.tc_ws, io.tc_ws_bytes, true);
-        return gemv(lcfg(c, true), ga, c->gemv_path);
+        GemvArgs gg = ga;
+        gg.frag_ws = c->frag_ws; gg.frag_ws_bytes = c->frag_ws_bytes;
+        return gemv(lcfg(c, true), gg, c->gemv_path);
     };
     for (uint32_t l = 0; l < d.n_layers; ++l) {
         const int L = (int)l;
@@ -496,6 +502,7 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
         h.norm_w = c->tensor(VB_ROLE_FINAL_NORM, 0).m.data; h.norm_fmt = c->tensor(VB_ROLE_FINAL_NORM, 0).m.fmt; h.eps = d.rms_eps;
         h.w = c->tensor(VB_ROLE_LM_HEAD, 0).m;
         h.trace = next_trace(); h.max_ring = c->head_ring;
+        h.frag_ws = c->frag_ws; h.frag_ws_bytes = c->frag_ws_bytes;
         if (io.i8_ws && gemm_i8_supported(h)) VB_TRY(gemm_i8(lcfg(c, true), h, io.i8_ws, io.i8_ws_bytes, true));
         else if (io.tc_ws && gemm_tc_supported(h)) VB_TRY(gemm_tc(lcfg(c, true), h, io.tc_ws, io.tc_ws_bytes, true));
         else VB_TRY(gemv(lcfg(c, true), h, c->gemv_path));
@@ -659,6 +666,8 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
         VB_CREATE_TRY(dev_alloc(&c->tp_pair, B * 8));
         VB_CREATE_TRY(dev_alloc(&c->tp_pairs, B * 8 * tp));
     }
+    c->frag_ws_bytes = gemv_mma_workspace_bytes(std::max(std::max(d.d_model, c->ffn), c->qdim));
+    VB_CREATE_TRY(dev_alloc(&c->frag_ws, c->frag_ws_bytes));
     VB_CREATE_TRY(dev_alloc(&c->attn_scratch, attn_scratch_floats(c->hq, d.head_dim, d.max_batch, c->n_splits)));
     VB_CREATE_CUDA(cudaMemsetAsync(c->attn_scratch, 0, attn_scratch_floats(c->hq, d.head_dim, d.max_batch, c->n_splits) * 4, c->stream));
     VB_CREATE_TRY(dev_alloc(&c->cand_v, B * argmax_chunks(c->vocab)));
@@ -693,7 +702,7 @@ int32_t vb_destroy(vb_ctx* c) {
     void* frees[] = {c->arena, c->kv_pool, c->block_table_dev, c->state, c->pf_state, c->pf_tokens, c->hidden, c->qkv, c->q,
                      c->attn_out, c->act, c->logits, c->attn_scratch, c->cand_v, c->cand_i, c->rope_inv_freq, c->trace, c->partial, c->tp_pair, c->tp_pairs,
                      c->pfc_state, c->pfc_table, c->pfc_hidden, c->pfc_qkv, c->pfc_q, c->pfc_attn, c->pfc_act, c->tc_ws, c->f16_pool, c->i8_tiles_pool, c->sample_probs,
-                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws};
+                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws, c->frag_ws};
     for (void* p : frees) if (p) cudaFree(p);
     if (c->ring_host) cudaFreeHost(c->ring_host);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -755,7 +764,8 @@ static int32_t finish_load(vb_ctx* c, Tensor* t, int32_t role, int32_t layer, co
     LaunchCfg lc = lcfg(c, false);
     lc.counter = nullptr;
     if (t->m.tiled) VB_CUDA(tile_q4(lc, const_cast<void*>(t->m.tiled), const_cast<void*>(t->m.tiled_scales), cn.data, cn.scales, t->m.rows, t->m.cols));
-    if (t->m.v3 && t->m.fmt == VB_FMT_Q4G32) VB_CUDA(tile_q4_v3(lc, const_cast<void*>(t->m.v3), cn.data, cn.scales, t->m.rows, t->m.cols));
+    const bool q4 = t->m.fmt == VB_FMT_Q4G32 || t->m.fmt == VB_FMT_Q4G64REF;
+    if (t->m.v3 && q4) VB_CUDA(tile_q4_v3(lc, const_cast<void*>(t->m.v3), cn.data, cn.scales, t->m.fmt, t->m.rows, t->m.cols));
     if (t->m.v3 && t->m.fmt == VB_FMT_I8PC)
         VB_CUDA(tile_i8_v3(lc, const_cast<void*>(t->m.v3), const_cast<void*>(t->m.v3_scales), cn.data, cn.scales, t->m.rows, t->m.cols));
     if (role == VB_ROLE_WGATE || role == VB_ROLE_WUP) {
@@ -763,7 +773,7 @@ static int32_t finish_load(vb_ctx* c, Tensor* t, int32_t role, int32_t layer, co
         const void* il = c->tensor(VB_ROLE_WGATE, layer).m.tiled_swiglu;
         if (il) VB_CUDA(tile_q4_swiglu(lc, const_cast<void*>(il), cn.data, cn.scales, t->m.rows, t->m.cols, which));
         const void* il3 = c->tensor(VB_ROLE_WGATE, layer).m.v3_swiglu;
-        if (il3 && t->m.fmt == VB_FMT_Q4G32) VB_CUDA(tile_q4_v3_swiglu(lc, const_cast<void*>(il3), cn.data, cn.scales, t->m.rows, t->m.cols, which));
+        if (il3 && q4) VB_CUDA(tile_q4_v3_swiglu(lc, const_cast<void*>(il3), cn.data, cn.scales, t->m.fmt, t->m.rows, t->m.cols, which));
         if (il3 && t->m.fmt == VB_FMT_I8PC) {
             unsigned char* sc = (unsigned char*)const_cast<void*>(il3) + 2 * wmat_data_bytes(t->m.fmt, t->m.rows, t->m.cols);
             VB_CUDA(tile_i8_v3_swiglu(lc, const_cast<void*>(il3), sc, cn.data, cn.scales, t->m.rows, t->m.cols, which));

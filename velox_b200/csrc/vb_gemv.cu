@@ -15,7 +15,7 @@ cudaError_t gemv_fast_init();  // vb_gemv_fast.cu
 
 cudaError_t gemv_init() {
     cudaError_t e;
-    if ((e = gemv_imma_init()) != cudaSuccess) return e;
+    if ((e = gemv_imma_init()) != cudaSuccess || (e = gemv_mma_init()) != cudaSuccess) return e;
     return gemv_fast_init();
 }
 
@@ -29,7 +29,9 @@ cudaError_t gemv(const LaunchCfg& lc, const GemvArgs& a, int path) {
     if (a.batch == 0 || a.w.rows == 0) return cudaSuccess;
     if (path != 0) {
         bool handled = false;
-        cudaError_t e = gemv_imma(lc, a, &handled);
+        cudaError_t e = gemv_mma(lc, a, &handled);
+        if (handled || e != cudaSuccess) return e;
+        e = gemv_imma(lc, a, &handled);
         if (handled || e != cudaSuccess) return e;
         e = gemv_fast(lc, a, &handled);
         if (handled || e != cudaSuccess) return e;

@@ -676,7 +676,22 @@ __global__ void k_tile_q4_v3_scales(__half* __restrict__ out, const __half* __re
     }
 }
 
-static cudaError_t tile_v3_half(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, uint32_t n_tiles,
+// group-64 weights keep the words; a block's 128 scale bytes are 8 x {(scale, minimum) of row g for its two groups, the same
+// of row g + 8}
+__global__ void k_tile_q4_v3_pairs(uint32_t* __restrict__ out, const uint32_t* __restrict__ canon, uint32_t n_tiles, uint32_t K,
+                                   uint32_t rows_per_tile, uint32_t row_off, uint32_t half) {
+    const uint32_t KT = K / 128;
+    const uint64_t n = (uint64_t)n_tiles * KT * 16;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t h = i & 1, g = (i >> 1) & 7;
+        const uint64_t blk = i >> 4;
+        const uint32_t kt = blk % KT, rt = blk / KT;
+        const uint64_t row = (uint64_t)rt * rows_per_tile + row_off + g;
+        out[blk * (IM_BLK_BYTES / 4) + 256 + g * 4 + half * 2 + h] = canon[row * (K / 64) + kt * 2 + h];
+    }
+}
+
+static cudaError_t tile_v3_half(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, int32_t fmt, uint32_t n_tiles,
                                 uint32_t K, uint32_t rows_per_tile, uint32_t row_off, uint32_t half) {
     const uint64_t nw = (uint64_t)n_tiles * (K / 128) * 128;
     unsigned blocks = (unsigned)((nw + 255) / 256 > 148 * 32 ? 148 * 32 : (nw + 255) / 256);
@@ -685,19 +700,21 @@ static cudaError_t tile_v3_half(const LaunchCfg& lc, void* tiled, const void* ca
     if (e != cudaSuccess) return e;
     const uint64_t ns = (uint64_t)n_tiles * (K / 128) * 32;
     blocks = (unsigned)((ns + 255) / 256 > 148 * 32 ? 148 * 32 : (ns + 255) / 256);
+    if (fmt == VB_FMT_Q4G64REF)
+        return launch(lc, k_tile_q4_v3_pairs, dim3(blocks), dim3(256), 0, (uint32_t*)tiled, (const uint32_t*)canon_scales, n_tiles, K, rows_per_tile, row_off, half);
     return launch(lc, k_tile_q4_v3_scales, dim3(blocks), dim3(256), 0, (__half*)tiled, (const __half*)canon_scales, n_tiles, K,
                   rows_per_tile, row_off, half);
 }
 
-cudaError_t tile_q4_v3(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, uint32_t rows, uint32_t K) {
-    cudaError_t e = tile_v3_half(lc, tiled, canon, canon_scales, rows / 16, K, 16, 0, 0);
+cudaError_t tile_q4_v3(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, int32_t fmt, uint32_t rows, uint32_t K) {
+    cudaError_t e = tile_v3_half(lc, tiled, canon, canon_scales, fmt, rows / 16, K, 16, 0, 0);
     if (e != cudaSuccess) return e;
-    return tile_v3_half(lc, tiled, canon, canon_scales, rows / 16, K, 16, 8, 1);
+    return tile_v3_half(lc, tiled, canon, canon_scales, fmt, rows / 16, K, 16, 8, 1);
 }
 // gate (which = 0) or up (which = 1) into the interleaved SwiGLU matrix: tile i = gate rows 8i..8i+7 | up rows 8i..8i+7
-cudaError_t tile_q4_v3_swiglu(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, uint32_t rows, uint32_t K,
+cudaError_t tile_q4_v3_swiglu(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, int32_t fmt, uint32_t rows, uint32_t K,
                               int which) {
-    return tile_v3_half(lc, tiled, canon, canon_scales, rows / 8, K, 8, 0, (uint32_t)which);
+    return tile_v3_half(lc, tiled, canon, canon_scales, fmt, rows / 8, K, 8, 0, (uint32_t)which);
 }
 
 constexpr int IM_NB = 4;   // rows of x per weight pass of the multi-row flavour ...

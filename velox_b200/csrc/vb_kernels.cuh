@@ -90,10 +90,16 @@ struct GemvArgs {
     bool* pushed = nullptr;          // out: set when the kernel that ran did send them
     bool* reduced = nullptr;         // out: set when it also finished the exchange (TpPush::reduce_hidden)
     unsigned long long* trace = nullptr;  // 3-slot timestamp record of this launch (tuned kernels only)
+    void* frag_ws = nullptr;         // != null: workspace of gemv_mma (gemv_mma_workspace_bytes of the widest in_dim), 16-byte aligned
+    uint64_t frag_ws_bytes = 0;
 };
 cudaError_t gemv(const LaunchCfg& lc, const GemvArgs& a, int path);
 // vb_gemv_canon.cu: every format from its canonical layout, fp32 arithmetic
 cudaError_t gemv_canon(const LaunchCfg& lc, const GemvArgs& a);
+// vb_gemv_mma.cu: a few rows of x on mma.sync (int4 tiles, fp16 / bf16 canonical); needs frag_ws
+cudaError_t gemv_mma_init();
+uint64_t gemv_mma_workspace_bytes(uint32_t max_in_dim);
+cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& a, bool* handled);
 
 // vb_gemv_fast.cu
 bool tile_q4_supported(uint32_t rows, uint32_t K);
@@ -114,8 +120,8 @@ cudaError_t tile_i8_v3(const LaunchCfg& lc, void* blocks, void* scales, const vo
                        uint32_t K);
 cudaError_t tile_i8_v3_swiglu(const LaunchCfg& lc, void* blocks, void* scales, const void* canon, const void* canon_scales, uint32_t rows,
                               uint32_t K, int which);
-cudaError_t tile_q4_v3(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, uint32_t rows, uint32_t K);
-cudaError_t tile_q4_v3_swiglu(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, uint32_t rows, uint32_t K,
+cudaError_t tile_q4_v3(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, int32_t fmt, uint32_t rows, uint32_t K);
+cudaError_t tile_q4_v3_swiglu(const LaunchCfg& lc, void* tiled, const void* canon, const void* canon_scales, int32_t fmt, uint32_t rows, uint32_t K,
                               int which);
 extern bool imma_enabled;
 extern bool imma_multirow;

@@ -119,6 +119,7 @@ int32_t verify_pass(vb_ctx* c, int32_t slot, const uint32_t* cand, uint32_t B, u
     h.norm_w = c->tensor(VB_ROLE_FINAL_NORM, 0).m.data; h.norm_fmt = c->tensor(VB_ROLE_FINAL_NORM, 0).m.fmt; h.eps = c->d.rms_eps;
     h.w = c->tensor(VB_ROLE_LM_HEAD, 0).m;
     h.max_ring = c->head_ring;
+    h.frag_ws = c->frag_ws; h.frag_ws_bytes = c->frag_ws_bytes;
     VB_CUDA(gemv(lcfg(c, true), h, c->gemv_path));
     VB_CUDA(argmax(lcfg(c, true), d_win, c->spec_logits, c->vocab, B, c->spec_cand_v, c->spec_cand_i, nullptr, nullptr, 0));
     VB_CUDA(cudaMemcpyAsync(winners, d_win, B * 4, cudaMemcpyDeviceToHost, c->stream));
