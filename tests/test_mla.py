@@ -136,3 +136,47 @@ def test_mla_block_from_library_ops_matches_checker(vb):
         n = start[b] + 12
         diff = np.abs((got_cache[b, :n].astype(np.uint32) << 16).view(np.float32) - caches[b][:n])
         assert np.max(diff) <= 2e-2 * max(1.0, float(np.max(np.abs(caches[b][:n]))))   # a bf16 ulp where fp32 sums differ in the last bit
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,n_in,n_out,batch,rows_out", [(3, 128, 512, 1, 0), (3, 512, 128, 17, 1), (2, 16, 16, 8, 0), (2, 48, 80, 33, 1), (1, 512, 2064, 9, 0), (5, 20, 24, 3, 1)])
+def test_head_product_widths_and_batches(vb, heads, n_in, n_out, batch, rows_out):
+    """Tiles of 16 outputs and 8 / 16 batch rows, parts of W_h, and the widths that are not whole 16s (the last case)."""
+    from velox_b200.engine import DeviceBuffer as dev
+    rng = np.random.default_rng(n_in + batch)
+    w = O.bf16_round(rng.standard_normal((heads, n_out, n_in) if rows_out else (heads, n_in, n_out)).astype(np.float32))
+    x = rng.standard_normal((batch, heads, n_in)).astype(np.float32)
+    d_w, d_x, d_y = dev.from_numpy(O.to_bf16_bits(w)), dev.from_numpy(x), dev(batch * heads * n_out * 4)
+    vb.check(vb.load().vb_op_mla_head_product(d_y.ptr, d_x.ptr, d_w.ptr, heads, n_in, n_out, batch, rows_out, None))
+    vb.check(vb.load().vb_dev_sync())
+    want = np.einsum("bhk,hok->bho" if rows_out else "bhk,hko->bho", x.astype(np.float64), w.astype(np.float64))
+    # fp32 sums of n_in products of unit normals: n_in roundings of 2^-24 of a partial sum below 6 sqrt(n_in)
+    assert np.max(np.abs(d_y.to_numpy(np.float32, (batch, heads, n_out)) - want)) <= n_in * 2.0 ** -24 * 6 * np.sqrt(n_in)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,lens", [(128, [1, 63, 64, 65, 3000, 0, 128, 127]), (7, [200] * 90), (200, [5000, 64, 1])])
+def test_mla_runs_of_tiles_that_cross_sequences(vb, heads, lens):
+    """The equal runs of 64-row tiles: sequences of one tile and of many runs, an empty one, more sequences than runs, two blocks
+    of heads.  Products of bf16 operands, probabilities rounded to bf16: 2^-8 of values below 5."""
+    from velox_b200.engine import DeviceBuffer as dev
+    lib = vb.load()
+    vb.check(lib.vb_op_mla_set_path(1))
+    rng = np.random.default_rng(heads)
+    B, max_ctx, scale = len(lens), max(lens), 1.0 / np.sqrt(192.0)
+    q = O.bf16_round(rng.standard_normal((B, heads, DC + DR)).astype(np.float32))
+    cache = O.bf16_round(rng.standard_normal((B, max_ctx, DC + DR)).astype(np.float32))
+    d_q, d_cache, d_len = dev.from_numpy(q), dev.from_numpy(O.to_bf16_bits(cache)), dev.from_numpy(np.array(lens, np.uint32))
+    need = lib.vb_op_mla_decode_scratch_bytes(B, heads, max_ctx, 0)
+    d_scratch, d_out = dev(need), dev(B * heads * DC * 4)
+    vb.check(lib.vb_op_mla_decode(d_out.ptr, d_q.ptr, d_cache.ptr, d_len.ptr, B, heads, max_ctx, max_ctx, scale, 0, d_scratch.ptr, need, None))
+    vb.check(lib.vb_dev_sync())
+    got = d_out.to_numpy(np.float32, (B, heads, DC))
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert np.all(got[b] == 0.0)
+            continue
+        s = (q[b] @ cache[b, :n].T) * scale
+        p = np.exp(s - s.max(axis=1, keepdims=True))
+        want = (p / p.sum(axis=1, keepdims=True)) @ cache[b, :n, :DC]
+        assert np.max(np.abs(got[b] - want)) <= 2.0 ** -8 * 5, b

@@ -153,8 +153,9 @@ bool gemm_i8_supported(const GemvArgs& a);
 // absorbed multi-head latent attention on tcgen05 (vb_mla_tc.cu); `extra` = status word + bf16 copy of q, 16-byte aligned
 extern bool mla_use_tc;
 uint64_t mla_tc_extra_scratch_bytes(uint32_t batch, uint32_t n_heads);
-cudaError_t mla_decode_tc(const LaunchCfg& lc, const float* q, const void* cache, const uint32_t* ctx_len, float* partial, void* extra,
-                          uint32_t batch, uint32_t n_heads, uint32_t n_splits, uint32_t split_tokens, uint64_t cache_stride, float scale);
+uint64_t mla_tc_partial_bytes(uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens);
+cudaError_t mla_decode_tc(const LaunchCfg& lc, float* out, const float* q, const void* cache, const uint32_t* ctx_len, float* partial, void* extra,
+                          uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens, uint64_t cache_stride, float scale);
 uint64_t gemm_i8_workspace_bytes(uint32_t in_dim);
 // int8 [rows][K] -> tile-major copy in shared-memory order (WMat::i8_tiles); K a multiple of 128
 uint64_t gemm_i8_tiles_bytes(uint32_t rows, uint32_t K);

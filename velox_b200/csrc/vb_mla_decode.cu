@@ -189,14 +189,8 @@ __global__ void __launch_bounds__(ML_THREADS, 1) k_mla_decode(MlaArgs a) {
 
 // out[b][h][:] = sum over the live slices of partial * exp(m - M) / L; grid (n_heads, B), 128 threads x 4 dimensions
 __global__ void __launch_bounds__(128) k_mla_merge(float* __restrict__ out, const float* __restrict__ partial, const uint32_t* __restrict__ ctx_len,
-                                                   uint32_t n_heads, uint32_t n_splits, uint32_t split_tokens, const uint32_t* __restrict__ status) {
+                                                   uint32_t n_heads, uint32_t n_splits, uint32_t split_tokens) {
     const uint32_t h = blockIdx.x, b = blockIdx.y;
-    if (status && *status) {
-        // a wait in the tensor-core kernel ran out: the partials are not to be trusted, and the caller must see it
-        float* o = out + ((size_t)b * n_heads + h) * ML_V + threadIdx.x * 4;
-        o[0] = o[1] = o[2] = o[3] = __int_as_float(0x7FC00000);
-        return;
-    }
     const uint32_t ctx = ctx_len[b];
     const uint32_t live = ctx == 0 ? 0 : min(n_splits, (ctx + split_tokens - 1) / split_tokens);
     const float* base = partial + (((size_t)b * n_splits) * n_heads + h) * (ML_V + 2);
@@ -252,6 +246,113 @@ __global__ void __launch_bounds__(256) k_mla_head_product(float* __restrict__ ds
     }
 }
 
+// The same products on mma.sync (m16n8k16, bf16 operands, fp32 accumulate) for widths in whole 16s: A = 16 output columns of W_h,
+// B = 8 batch rows, x as three bf16 parts whose sum is the fp32 value.  A block makes [128 outputs][64 batch rows] of a head: 16
+// warps of 16 outputs x 32 rows, K in chunks of 64, W_h through three stages of cp.async, x through registers (converted on the
+// way to shared memory, the next chunk's loads in flight meanwhile).  W_h and x are read once per such tile; mma and ldmatrix
+// take about the same time (12 and 7 per warp and K step).
+// 128 heads, batch 64: 512 -> 128 17 us, 128 -> 512 21 us (the kernel above, which reads W_h element by element and once for
+// every 16 rows: 198 and 84 us; 32 KB of W_h per block and 16 rows at a time, x converted anew by every block: 45 and 25 us).
+constexpr int HP_O = 128, HP_B = 64, HP_K = 64, HP_THREADS = 512, HP_XROW = HP_K + 8;  // (rows 16 bytes apart modulo 128: no bank conflicts)
+__device__ __forceinline__ void hp_ldsm4(uint32_t (&r)[4], uint32_t addr, bool trans) {
+    if (trans) asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    else asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <bool W_ROWS_ARE_OUT>
+__global__ void __launch_bounds__(HP_THREADS, 2) k_mla_head_mma(float* __restrict__ dst, const float* __restrict__ src, const __nv_bfloat16* __restrict__ w,
+                                                                uint32_t n_heads, uint32_t n_in, uint32_t n_out, uint32_t batch) {
+    // a W stage: [128 outputs][64 of K] or [64 of K][128 outputs], rows padded by 8 elements
+    constexpr uint32_t W_ROWS = W_ROWS_ARE_OUT ? HP_O : HP_K, W_COLS = W_ROWS_ARE_OUT ? HP_K : HP_O, W_ROW = W_COLS + 8, W_STAGE = W_ROWS * W_ROW * 2;
+    constexpr uint32_t X_PART = HP_B * HP_XROW * 2, X_STAGE = 3 * X_PART;
+    extern __shared__ __align__(16) unsigned char hp_smem[];
+    const uint32_t h = blockIdx.x, o0 = blockIdx.y * HP_O, b0 = blockIdx.z * HP_B;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, mat = lane >> 3, r8 = lane & 7;
+    const uint32_t ws = (uint32_t)__cvta_generic_to_shared(hp_smem), xs = ws + 3 * W_STAGE;
+    const __nv_bfloat16* wh = w + (size_t)h * n_in * n_out;
+    const uint32_t n_chunks = (n_in + HP_K - 1) / HP_K;
+    auto load_w = [&](uint32_t c) {  // zeros outside the matrix
+#pragma unroll
+        for (uint32_t i = threadIdx.x; i < W_ROWS * W_COLS / 8; i += HP_THREADS) {
+            const uint32_t r = i / (W_COLS / 8), p = i % (W_COLS / 8) * 8;
+            const uint32_t o = W_ROWS_ARE_OUT ? o0 + r : o0 + p, k = W_ROWS_ARE_OUT ? c * HP_K + p : c * HP_K + r;
+            const bool in = c < n_chunks && o < n_out && k < n_in;
+            const __nv_bfloat16* from = in ? (W_ROWS_ARE_OUT ? wh + (size_t)o * n_in + k : wh + (size_t)k * n_out + o) : w;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ws + (c % 3) * W_STAGE + (r * W_ROW + p) * 2), "l"(from), "r"(in ? 16u : 0u) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // x: thread -> batch row threadIdx / 16 (+ 32), four elements of K
+    float4 xr[2];
+    auto load_x = [&](uint32_t c) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t b = b0 + threadIdx.x / 16 + i * 32, k = c * HP_K + threadIdx.x % 16 * 4;
+            xr[i] = (c < n_chunks && b < batch && k < n_in) ? *reinterpret_cast<const float4*>(src + ((size_t)b * n_heads + h) * n_in + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    load_w(0);
+    load_w(1);
+    load_x(0);
+    const uint32_t m0 = (warp & 7) * 16, n0 = (warp >> 3) * 32;  // this warp's outputs and batch rows
+    const bool work = o0 + m0 < n_out && b0 + n0 < batch;
+    const uint32_t pairs = work ? (min(batch - b0 - n0, 32u) + 15) / 16 : 0;
+    float d[4][4] = {};
+    const uint32_t a_at = W_ROWS_ARE_OUT ? ((m0 + (mat & 1) * 8 + r8) * W_ROW + (mat >> 1) * 8) * 2 : (((mat >> 1) * 8 + r8) * W_ROW + m0 + (mat & 1) * 8) * 2;
+    const uint32_t b_at = ((n0 + (mat >> 1) * 8 + r8) * HP_XROW + (mat & 1) * 8) * 2;  // rows n..n+7 (K lo, K hi), rows n+8..n+15
+    for (uint32_t c = 0; c < n_chunks; ++c) {
+        const uint32_t xb = xs + (c & 1) * X_STAGE, wb = ws + (c % 3) * W_STAGE;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float4 v = xr[i];
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+                const __nv_bfloat162 p = __floats2bfloat162_rn(v.x, v.y), q = __floats2bfloat162_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(hp_smem + (xb - ws) + part * X_PART + ((threadIdx.x / 16 + i * 32) * HP_XROW + threadIdx.x % 16 * 4) * 2) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&p), *reinterpret_cast<const uint32_t*>(&q));
+                v.x -= __low2float(p); v.y -= __high2float(p); v.z -= __low2float(q); v.w -= __high2float(q);
+            }
+        }
+        load_x(c + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // chunk c is there, and every warp is done with chunk c - 1
+        load_w(c + 2);
+        if (work) {
+#pragma unroll
+            for (uint32_t k = 0; k < HP_K; k += 16) {
+                uint32_t A[4];
+                hp_ldsm4(A, wb + a_at + (W_ROWS_ARE_OUT ? k : k * W_ROW) * 2, !W_ROWS_ARE_OUT);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) {
+#pragma unroll
+                    for (uint32_t np = 0; np < 2; ++np) {
+                        if (np < pairs) {
+                            uint32_t B[4];
+                            hp_ldsm4(B, xb + part * X_PART + b_at + (np * 16 * HP_XROW + k) * 2, false);
+#pragma unroll
+                            for (int n = 0; n < 2; ++n) {
+                                float* e = d[2 * np + n];
+                                asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                                    : "+f"(e[0]), "+f"(e[1]), "+f"(e[2]), "+f"(e[3]) : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(B[2 * n]), "r"(B[2 * n + 1]));
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (work) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t b = b0 + n0 + n * 8 + 2 * t + (i & 1), o = o0 + m0 + g + 8 * (i >> 1);
+                if (b < batch) dst[((size_t)b * n_heads + h) * n_out + o] = d[n][i];
+            }
+    }
+}
+constexpr int hp_smem_bytes(bool rows_out) { return 3 * (rows_out ? HP_O * (HP_K + 8) : HP_K * (HP_O + 8)) * 2 + 2 * 3 * HP_B * HP_XROW * 2; }
+
 }  // namespace
 
 }  // namespace vb
@@ -260,15 +361,16 @@ using namespace vb;
 
 extern "C" {
 
+// the partial outputs of the mma.sync kernel's slices or of the tcgen05 kernel's pieces; split_tokens as the caller gave it
 static uint64_t mla_partial_bytes(uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens) {
-    const uint64_t n_splits = ((uint64_t)max_ctx + split_tokens - 1) / split_tokens;
-    const uint64_t b = (uint64_t)batch * (n_splits ? n_splits : 1) * n_heads * (ML_V + 2) * 4;
-    return (b + 1023) / 1024 * 1024;
+    const uint32_t slice = split_tokens ? split_tokens : 1024;
+    const uint64_t n_splits = ((uint64_t)max_ctx + slice - 1) / slice;
+    const uint64_t a = (uint64_t)batch * (n_splits ? n_splits : 1) * n_heads * (ML_V + 2) * 4, b = mla_tc_partial_bytes(batch, n_heads, max_ctx, split_tokens);
+    return ((a > b ? a : b) + 1023) / 1024 * 1024;
 }
 
 uint64_t vb_op_mla_decode_scratch_bytes(uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens) {
-    if (split_tokens == 0) split_tokens = 1024;
-    // the slices' partial outputs, then the tensor-core path's status word and bf16 copy of q
+    // the partial outputs, then the tensor-core path's status word and bf16 copy of q
     return mla_partial_bytes(batch, n_heads, max_ctx, split_tokens) + mla_tc_extra_scratch_bytes(batch, n_heads);
 }
 
@@ -283,11 +385,19 @@ int32_t vb_op_mla_decode(float* out, const float* q, const void* latent_cache, c
                          void* stream) {
     VB_REQUIRE(out && q && latent_cache && ctx_len && scratch, "vb_op_mla_decode: null pointer");
     VB_REQUIRE(batch > 0 && n_heads > 0 && max_ctx > 0 && cache_stride_rows >= max_ctx, "vb_op_mla_decode: empty problem or cache stride below max_ctx");
-    if (split_tokens == 0) split_tokens = 1024;
     VB_REQUIRE(split_tokens % ML_TILE == 0, "vb_op_mla_decode: split_tokens=%u is not a multiple of %d", split_tokens, ML_TILE);
     VB_REQUIRE(((uintptr_t)latent_cache & 15) == 0 && ((uintptr_t)q & 7) == 0 && ((uintptr_t)scratch & 15) == 0, "vb_op_mla_decode: unaligned pointer");
     VB_REQUIRE(scratch_bytes >= vb_op_mla_decode_scratch_bytes(batch, n_heads, max_ctx, split_tokens), "vb_op_mla_decode: scratch of %llu bytes is too small",
                (unsigned long long)scratch_bytes);
+    LaunchCfg lc;
+    lc.stream = (cudaStream_t)stream;
+    if (mla_use_tc) {
+        // tcgen05 path: both products on the 5th-generation tensor cores (vb_mla_tc.cu)
+        void* extra = reinterpret_cast<unsigned char*>(scratch) + mla_partial_bytes(batch, n_heads, max_ctx, split_tokens);
+        VB_CUDA(mla_decode_tc(lc, out, q, latent_cache, ctx_len, (float*)scratch, extra, batch, n_heads, max_ctx, split_tokens, cache_stride_rows, scale));
+        return VB_OK;
+    }
+    if (split_tokens == 0) split_tokens = 1024;
     static bool opted = false;
     if (!opted) {
         VB_CUDA(cudaFuncSetAttribute(k_mla_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ML_SMEM));
@@ -297,20 +407,9 @@ int32_t vb_op_mla_decode(float* out, const float* q, const void* latent_cache, c
     a.q = q; a.cache = (const __nv_bfloat16*)latent_cache; a.ctx_len = ctx_len; a.partial = (float*)scratch;
     a.n_heads = n_heads; a.split_tokens = split_tokens; a.n_splits = (max_ctx + split_tokens - 1) / split_tokens;
     a.cache_stride = cache_stride_rows; a.scale = scale;
-    LaunchCfg lc;
-    lc.stream = (cudaStream_t)stream;
-    if (mla_use_tc) {
-        // tcgen05 path: both products on the 5th-generation tensor cores (vb_mla_tc.cu)
-        void* extra = reinterpret_cast<unsigned char*>(scratch) + mla_partial_bytes(batch, n_heads, max_ctx, split_tokens);
-        VB_CUDA(mla_decode_tc(lc, q, latent_cache, ctx_len, (float*)scratch, extra, batch, n_heads, a.n_splits, split_tokens, cache_stride_rows, scale));
-        VB_CUDA(launch(lc, k_mla_merge, dim3(n_heads, batch), dim3(128), 0, out, (const float*)scratch, ctx_len, n_heads, a.n_splits, split_tokens,
-                       (const uint32_t*)extra));
-        return VB_OK;
-    }
     const dim3 grid(a.n_splits, (n_heads + ML_HEADS_PER_BLOCK - 1) / ML_HEADS_PER_BLOCK, batch);
     VB_CUDA(launch(lc, k_mla_decode, grid, dim3(ML_THREADS), ML_SMEM, a));
-    VB_CUDA(launch(lc, k_mla_merge, dim3(n_heads, batch), dim3(128), 0, out, (const float*)scratch, ctx_len, n_heads, a.n_splits, split_tokens,
-                   (const uint32_t*)nullptr));
+    VB_CUDA(launch(lc, k_mla_merge, dim3(n_heads, batch), dim3(128), 0, out, (const float*)scratch, ctx_len, n_heads, a.n_splits, split_tokens));
     return VB_OK;
 }
 
@@ -329,6 +428,19 @@ int32_t vb_op_mla_head_product(float* dst, const float* src, const void* w_bf16,
     if (batch == 0) return VB_OK;
     LaunchCfg lc;
     lc.stream = (cudaStream_t)stream;
+    // whole 16s and 16-byte rows: the tensor-core kernel
+    if (n_in % 16 == 0 && n_out % 16 == 0 && (((uintptr_t)src | (uintptr_t)w_bf16) & 15) == 0) {
+        static bool opted_hp = false;
+        if (!opted_hp) {
+            VB_CUDA(cudaFuncSetAttribute(k_mla_head_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(true)));
+            VB_CUDA(cudaFuncSetAttribute(k_mla_head_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(false)));
+            opted_hp = true;
+        }
+        const dim3 g3(n_heads, (n_out + HP_O - 1) / HP_O, (batch + HP_B - 1) / HP_B);
+        if (w_rows_are_out) VB_CUDA(launch(lc, k_mla_head_mma<true>, g3, dim3(HP_THREADS), hp_smem_bytes(true), dst, src, (const __nv_bfloat16*)w_bf16, n_heads, n_in, n_out, batch));
+        else VB_CUDA(launch(lc, k_mla_head_mma<false>, g3, dim3(HP_THREADS), hp_smem_bytes(false), dst, src, (const __nv_bfloat16*)w_bf16, n_heads, n_in, n_out, batch));
+        return VB_OK;
+    }
     const dim3 grid(n_heads, (batch + 15) / 16);
     const size_t smem = (size_t)16 * n_in * 4;
     if (w_rows_are_out) VB_CUDA(launch(lc, k_mla_head_product<true>, grid, dim3(256), smem, dst, src, (const __nv_bfloat16*)w_bf16, n_heads, n_in, n_out, batch));
