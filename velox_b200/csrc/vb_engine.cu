@@ -996,10 +996,11 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // the batched kernels read the weights once for the chunk, K/V of all rows are appended before attention and row
     // j attends positions 0..first+j, so the result is the causal one.  (The reference's batched prefill driver:
     // velox_cuda_runner_k2.cu:1614-1704.)  Sharded contexts and the last token take the per-token path below.
+    // Prompts of up to half a chunk go token by token: the same bits as the same tokens fed one step at a time.
     uint32_t done = 0;
     const bool use_tc = c->prefill_gemm && c->d.tp_size <= 1 && n_tokens > c->prefill_gemm_min && c->prefill_rows >= 1 && tc_products_ok(c);
     const uint32_t P = use_tc ? std::min(c->prefill_rows, n_tokens - 1) : c->prefill_chunk;
-    if (use_tc || (P >= 2 && P <= 32 && c->d.tp_size <= 1 && n_tokens > P)) {
+    if (use_tc || (P >= 2 && P <= 32 && c->d.tp_size <= 1 && 2 * n_tokens > P)) {
         const uint32_t cap = use_tc ? c->prefill_rows : P;  // rows the chunk buffers hold
         if ((rc = ensure_chunk_buffers(c, cap)) != VB_OK) return rc;
         if (use_tc && ((rc = ensure_f16_copies(c)) != VB_OK || (rc = ensure_tc_ws(c, cap, false)) != VB_OK)) return rc;
@@ -1007,10 +1008,10 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
                        (const int32_t*)(c->block_table_dev + (size_t)slot * c->max_blocks), c->max_blocks));
         StepIO io{c->pfc_hidden, c->pfc_qkv, c->pfc_q, c->pfc_attn, c->pfc_act, nullptr, c->pfc_table, P, false};
         if (use_tc) { io.tc_ws = tc_ws_aligned(c); io.tc_ws_bytes = c->tc_ws_bytes; io.causal_chunk = true; }
-        // the last token always takes the per-token path below (it produces the logits); the tensor-core chunks may be
-        // ragged (every row of a chunk is live), the batched-kernel chunks are whole
-        while (use_tc ? done + 1 < n_tokens : done + P < n_tokens) {
-            const uint32_t n = use_tc ? std::min(P, n_tokens - 1 - done) : P;
+        // the last token always takes the per-token path below (it produces the logits); the last chunk may be ragged (token by
+        // token instead, a 120-token prompt of the 72B shape spent 66 ms on its last 8)
+        while (done + 1 < n_tokens) {
+            const uint32_t n = std::min(P, n_tokens - 1 - done);
             io.B = n; io.first = done;
             VB_CUDA(launch(lcfg(c, false), k_set_chunk_state, dim3((n + 127) / 128), dim3(128), 0, c->pfc_state, (const uint32_t*)c->pf_tokens, done, n, n));
             VB_CUDA(enqueue_step(c, c->pfc_state, false, io));

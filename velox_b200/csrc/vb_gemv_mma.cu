@@ -588,9 +588,20 @@ cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& g, bool* handled) {
     const bool swiglu = g.epilogue == EPI_SWIGLU, q4 = g.w.fmt == VB_FMT_Q4G32 || g.w.fmt == VB_FMT_Q4G64REF;
     const uint32_t K = g.w.cols;
     if (!g.frag_ws || gemv_mma_workspace_bytes(K) > g.frag_ws_bytes || g.push.links) return cudaSuccess;
-    // One row of x: the kernels that stage it themselves save a launch, except for group-64 weights, which have none.
-    // Two rows of 16-bit weights: still no more than the FMA kernel does beside the stream (it is ahead to 2, behind at 4).
-    if (g.w.fmt == VB_FMT_Q4G32 ? g.batch < 2 : q4 ? g.batch < 1 : g.batch < 3) return cudaSuccess;
+    const uint64_t weights = (uint64_t)g.w.rows * K * (swiglu ? 2 : 1);
+    if (g.w.fmt == VB_FMT_Q4G32) {
+        // One row: the integer kernel stages x itself and needs one launch.  2..4 rows are one pass of its multi-row flavour too,
+        // faster (8B shape: O 6.2 against 8.2 us, gate/up 17.5 / 22.9, head 55 / 64) unless its tiles fill the last round of
+        // SMs badly (QKV: 384 tiles on 296 places, 14.7 / 10.4) or four rows of x are long to stage (down: 19.7 / 15.8).
+        if (g.batch < 2) return cudaSuccess;
+        const uint32_t tiles = (swiglu ? 2 : 1) * g.w.rows / 16, places = 2 * 148, rounds = (tiles + places - 1) / places;
+        if (g.batch <= 4 && K <= 8192 && tiles * 4 >= rounds * places * 3) return cudaSuccess;
+    } else {
+        // The fp32 kernel needs one launch and no conversion: ahead on small matrices (135M model, group-64, one row: 2.8 against
+        // 6.4 us) and with one or two rows of 16-bit weights (it streams those at 5..6 TB/s).
+        if (!q4 && g.batch < 3) return cudaSuccess;
+        if (weights * g.batch < 8000000ull) return cudaSuccess;
+    }
     MmArgs a;
     if (q4) {
         a.w = (const unsigned char*)(swiglu ? g.w.v3_swiglu : g.w.v3);
