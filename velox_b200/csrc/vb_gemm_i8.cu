@@ -107,7 +107,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     unsigned char* gen = smem_raw + (base - smem_u32(smem_raw));
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + STAGES * STAGE_BYTES + (2 * STAGES + 1) * 8);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int row0 = blockIdx.y * I8_BM;
     const int nk_all = (int)((p.K + I8_BK - 1) / I8_BK);
     const int kb_first = (int)(((long long)nk_all * blockIdx.z) / gridDim.z), kb_last = (int)(((long long)nk_all * (blockIdx.z + 1)) / gridDim.z);
@@ -130,7 +130,8 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+      if (elect_one()) {
         // weights do not depend on the kernel before this one: the whole ring of weight tiles is requested before the
         // dependency wait, the planes of x (written by the conversion kernel in front) after it
         const int pre = nk < STAGES ? nk : STAGES;
@@ -167,13 +168,16 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             }
             tma_2d(st + W_TILES * I8_W_BYTES, &map_x, kx, 0, full);
         }
-    } else if (warp == 1 && lane == 0) {
+      }
+    } else if (warp == 1) {
+        // the warp waits together, an elected lane issues (vb_tma.cuh)
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!wait_abort(bars + s * 8, ph, abort_flag)) break;
+            if (!__all_sync(0xFFFFFFFFu, wait_abort(bars + s * 8, ph, abort_flag))) break;
             fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
+            if (elect_one()) {
             const uint64_t da = smem_desc_sw128(st), da2 = smem_desc_sw128(st + I8_W_BYTES), db = smem_desc_sw128(st + W_TILES * I8_W_BYTES);
 #pragma unroll
             for (int k = 0; k < I8_BK / 32; ++k) {  // 32 bytes further along the swizzled row: +2 in the address field
@@ -182,8 +186,10 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                 if (DUAL) mma_i8(tmem + I8_BN, da2 + 2u * k, db + 2u * k, acc);
             }
             commit_to(bars + (STAGES + s) * 8);
+            if (kb == nk - 1) commit_to(bar_accum);
+            }
+            __syncwarp();
         }
-        commit_to(bar_accum);
     }
     __syncwarp();
     pdl_wait();               // every thread: the epilogue reads the residual stream and x scales of earlier kernels

@@ -31,13 +31,10 @@ constexpr int BM = 128;      // weight rows per tile (UMMA M)
                              // rows of x per tile (UMMA N): 128 or 256, a template parameter of the kernel
 constexpr int BK = 64;       // K extent of a stage: 64 fp16 = one 128-byte swizzle row
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KB: one box of 128 rows
-// ring depth so that the stages fill 192 KB: (weight tiles + x tiles) x 16 KB per stage
-__host__ __device__ constexpr int stage_bytes_for(bool dual, int bn) { return (dual ? 2 : 1) * TILE_BYTES + bn * BK * 2; }
-// PER_SM = 1: the ring fills 192 KB; PER_SM = 2: 96 KB, so that two blocks share an SM and one block's prologue
-// and epilogue overlap the other's main loop
-__host__ __device__ constexpr int stages_for(bool dual, int bn, int per_sm = 1) { return (192 / per_sm) * 1024 / stage_bytes_for(dual, bn); }
-constexpr int SMEM_BYTES_HALF = 96 * 1024 + 1024 + 256;
-constexpr int SMEM_BYTES = 192 * 1024 + 1024 /* alignment slack */ + 256 /* barriers */;
+// the ring of stages fills 192 KB; PER_SM = 2: 96 KB, so that two blocks share an SM and one block's prologue and epilogue
+// overlap the other's main loop
+constexpr int RING_BYTES = 192 * 1024;
+__host__ __device__ constexpr int smem_bytes_for(int per_sm) { return RING_BYTES / per_sm + 1024 /* alignment slack */ + 256 /* barriers */; }
 
 // instruction descriptor of tcgen05.mma kind::f16: fp32 accumulate (bits 4-5 = 1), A and B fp16 (formats 0),
 // both K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24
@@ -99,26 +96,26 @@ struct GemmParams {
     // counter sums the partials in split order (the same bits whoever is last) and runs the epilogue
     float* part;          // [split][tile][BN / 32][32][128]
     uint32_t* counters;   // [tile], zero between launches (the last block puts the zero back)
-    // Operand splitting (prefill chunks): fp16 holds 11 significant bits, and over 32 layers and thousands of cached
+    // Operand splitting (prefill chunks, template parameters XP and WP): fp16 holds 11 significant bits, and over 32 layers and thousands of cached
     // positions that rounding reaches the logits (2.8e-2 at 2048 rows of the 8B shape).  x_parts = 2: x = x_hi + x_lo,
     // both fp16, x_lo rows lie `x_lo_row` rows below x_hi in the same tensor map; w_parts = 2: W = W_hi + W_lo likewise
     // (second tensor maps).  The products W_hi.x_hi + W_hi.x_lo + W_lo.x_hi accumulate into the same tensor-memory
     // columns, so the epilogue does not change; what is dropped (W_lo.x_lo) is 2^-22 of the result.
-    uint32_t x_parts, w_parts, x_lo_row;
-    uint32_t stages;      // ring depth for this operand set
+    uint32_t x_lo_row;
 };
 
-template <bool DUAL, int BN, int PER_SM = 1>
+// XP, WP: parts of x and of the weights (1 or 2); compile-time, so that every descriptor is a base plus a constant
+template <bool DUAL, int BN, int PER_SM, int XP, int WP>
 __global__ void __launch_bounds__(128, PER_SM)
 k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
           const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wl, const __grid_constant__ CUtensorMap map_wl2,
           const GemmParams p) {
     constexpr int W_TILES = DUAL ? 2 : 1, X_TILES = BN / 128;  // BN = 32: one box of 32 rows
     constexpr int X_BYTES = BN * BK * 2;                        // one part of the x operand of a stage
-    const int STAGES = (int)p.stages;
-    const int WP = (int)p.w_parts, XP = (int)p.x_parts;
-    const int STAGE_BYTES = W_TILES * WP * TILE_BYTES + XP * X_BYTES;  // [W hi (,W2 hi)][W lo (,W2 lo)][x hi][x lo]
-    const int X_OFF = W_TILES * WP * TILE_BYTES;
+    constexpr int STAGE_BYTES = W_TILES * WP * TILE_BYTES + XP * X_BYTES;  // [W hi (,W2 hi)][W lo (,W2 lo)][x hi][x lo]
+    constexpr int STAGES = RING_BYTES / PER_SM / STAGE_BYTES;
+    static_assert(STAGES >= 2, "ring depth");
+    constexpr int X_OFF = W_TILES * WP * TILE_BYTES;
     constexpr uint32_t IDESC = idesc_for(BN);
     constexpr uint32_t TMEM_COLS = DUAL ? 2 * BN : BN;
     extern __shared__ unsigned char smem_raw[];
@@ -129,7 +126,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + STAGES * STAGE_BYTES + (2 * STAGES + 1) * 8);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // the tiles of x are the fastest block index: the blocks that share a weight tile run together and it comes
     // from DRAM once
     const int row0 = blockIdx.y * BM, tok0 = blockIdx.x * BN;
@@ -156,8 +153,9 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     pdl_wait();  // x (and converted weights) come from the kernels before this one
     pdl_launch_dependents();
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---- producer: TMA copies into the ring ----
+        if (elect_one())
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
@@ -177,31 +175,34 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                 if (X_TILES == 2) tma_load_2d(st + X_OFF + xp * X_BYTES + TILE_BYTES, &map_x, kx, xr + 128, full);  // rows 128..255: the next 16 groups of 8
             }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- tensor-core issue ----
+    } else if (warp == 1) {
+        // ---- tensor-core issue: the warp waits together, an elected lane issues (see vb_tma.cuh) ----
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!wait_or_abort(bars + s * 8, ph, abort_flag)) break;
+            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag))) break;
             tc_fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
-            const uint64_t da = smem_desc(st), da2 = smem_desc(st + TILE_BYTES), db = smem_desc(st + X_OFF);
-            const uint64_t dal = smem_desc(st + W_TILES * TILE_BYTES), dal2 = smem_desc(st + (W_TILES + 1) * TILE_BYTES), dbl = smem_desc(st + X_OFF + X_BYTES);
+            if (elect_one()) {
+                const uint64_t da = smem_desc(st), da2 = smem_desc(st + TILE_BYTES), db = smem_desc(st + X_OFF);
+                const uint64_t dal = smem_desc(st + W_TILES * TILE_BYTES), dal2 = smem_desc(st + (W_TILES + 1) * TILE_BYTES), dbl = smem_desc(st + X_OFF + X_BYTES);
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {  // 16 fp16 = 32 bytes further along the swizzled row: +2 in the address field
-                const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
-                mma_f16(tmem, da + 2u * k, db + 2u * k, IDESC, acc);
-                if (XP == 2) mma_f16(tmem, da + 2u * k, dbl + 2u * k, IDESC, 1u);
-                if (WP == 2) mma_f16(tmem, dal + 2u * k, db + 2u * k, IDESC, 1u);
-                if (DUAL) {
-                    mma_f16(tmem + BN, da2 + 2u * k, db + 2u * k, IDESC, acc);
-                    if (XP == 2) mma_f16(tmem + BN, da2 + 2u * k, dbl + 2u * k, IDESC, 1u);
-                    if (WP == 2) mma_f16(tmem + BN, dal2 + 2u * k, db + 2u * k, IDESC, 1u);
+                for (int k = 0; k < BK / 16; ++k) {  // 16 fp16 = 32 bytes further along the swizzled row: +2 in the address field
+                    const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
+                    mma_f16(tmem, da + 2u * k, db + 2u * k, IDESC, acc);
+                    if (XP == 2) mma_f16(tmem, da + 2u * k, dbl + 2u * k, IDESC, 1u);
+                    if (WP == 2) mma_f16(tmem, dal + 2u * k, db + 2u * k, IDESC, 1u);
+                    if (DUAL) {
+                        mma_f16(tmem + BN, da2 + 2u * k, db + 2u * k, IDESC, acc);
+                        if (XP == 2) mma_f16(tmem + BN, da2 + 2u * k, dbl + 2u * k, IDESC, 1u);
+                        if (WP == 2) mma_f16(tmem + BN, dal2 + 2u * k, db + 2u * k, IDESC, 1u);
+                    }
                 }
+                mma_commit(bars + (STAGES + s) * 8);  // the stage is free again once these products have read it
+                if (kb == nk - 1) mma_commit(bar_accum);
             }
-            mma_commit(bars + (STAGES + s) * 8);  // the stage is free again once these products have read it
+            __syncwarp();
         }
-        mma_commit(bar_accum);
     }
     __syncwarp();
 
@@ -451,24 +452,23 @@ bool gemm_tc_split_k = true;  // vb_set_option("decode_split_k", 0): one block p
 int gemm_tc_split = 2;  // vb_set_option("prefill_split", n): prefill chunks multiply 0: fp16(x).fp16(W); 1: x as hi + lo; 2: x and W as hi + lo
 bool gemm_tc_wide = false;  // vb_set_option("prefill_wide", 1): 256 rows of x per tile when a chunk has more than 128 (measured slower at 512 rows: fewer blocks than SMs)
 
+template <bool DUAL, int BN, int PER_SM, int XP, int WP>
+static cudaError_t tc_opt_in() {
+    return cudaFuncSetAttribute(k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_for(PER_SM));
+}
+template <bool DUAL, int BN, int PER_SM, int XP, int WP>
+static cudaError_t tc_launch(const LaunchCfg& lc, const dim3& grid, const CUtensorMap* m, const GemmParams& p) {
+    return launch(lc, k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, grid, dim3(128), smem_bytes_for(PER_SM), m[0], m[1], m[2], m[3], m[4], p);
+}
+
 cudaError_t gemm_tc_init() {
     if (g_tc_init) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<false, 128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_HALF);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<true, 128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_HALF);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_tc<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+#define VB_TC(...) if ((e = tc_opt_in<__VA_ARGS__>()) != cudaSuccess) return e
+    VB_TC(false, 32, 1, 1, 1); VB_TC(true, 32, 1, 1, 1);
+    VB_TC(false, 128, 2, 1, 1); VB_TC(false, 128, 2, 2, 1); VB_TC(false, 128, 1, 2, 2);
+    VB_TC(true, 128, 2, 1, 1); VB_TC(true, 128, 1, 2, 1); VB_TC(true, 128, 1, 2, 2);
+#undef VB_TC
     g_tc_init = true;
     return cudaSuccess;
 }
@@ -550,13 +550,14 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
         wh[i] = hi;
         wl[i] = lo;
     }
-    CUtensorMap mw, mw2, mx, mwl, mwl2;
-    if (!make_map(&mw, wh[0], out_dim, K) || !make_map(&mx, xh, rows_pad * x_parts, K, narrow ? 32 : BM)) return cudaErrorNotSupported;
-    if (dual) { if (!make_map(&mw2, wh[1], out_dim, K)) return cudaErrorNotSupported; } else mw2 = mw;
-    mwl = mw; mwl2 = mw2;
+    CUtensorMap maps[5];  // W, W2, x, W lo, W2 lo
+    if (!make_map(&maps[0], wh[0], out_dim, K) || !make_map(&maps[2], xh, rows_pad * x_parts, K, narrow ? 32 : BM)) return cudaErrorNotSupported;
+    maps[1] = maps[0];
+    if (dual && !make_map(&maps[1], wh[1], out_dim, K)) return cudaErrorNotSupported;
+    maps[3] = maps[0]; maps[4] = maps[1];
     if (w_parts == 2) {
-        if (!make_map(&mwl, wl[0], out_dim, K)) return cudaErrorNotSupported;
-        if (dual && !make_map(&mwl2, wl[1], out_dim, K)) return cudaErrorNotSupported;
+        if (!make_map(&maps[3], wl[0], out_dim, K)) return cudaErrorNotSupported;
+        if (dual && !make_map(&maps[4], wl[1], out_dim, K)) return cudaErrorNotSupported;
     }
     GemmParams p;
     p.dst = a.dst + a.dst_offset;
@@ -570,11 +571,7 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
     fast_error_word(&p.err);
     p.counters = reinterpret_cast<uint32_t*>(workspace);
     p.part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(workspace) + WS_COUNTER_BYTES);
-    p.x_parts = x_parts; p.w_parts = w_parts; p.x_lo_row = (uint32_t)rows_pad;
-    auto stages_of = [&](int bn, int ring_kb) {
-        const int stage = (dual ? 2 : 1) * (int)w_parts * TILE_BYTES + (int)x_parts * bn * BK * 2;
-        return ring_kb * 1024 / stage;
-    };
+    p.x_lo_row = (uint32_t)rows_pad;
     if (narrow) {
         // few row tiles (QKV, O, down of a decode batch: 28-36 blocks on 148 SMs): split K so that every SM streams
         const uint32_t tiles = (out_dim + BM - 1) / BM, nk = (K + BK - 1) / BK;
@@ -584,27 +581,13 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
             if ((uint64_t)splits * tiles * 128 * 32 * 4 > WS_PART_BYTES || tiles * 4 > WS_COUNTER_BYTES) splits = 1;
         }
         const dim3 grid(1, tiles, splits);
-        p.stages = (uint32_t)stages_of(32, 192);
-        if (dual) return launch(lc, k_gemm_tc<true, 32>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
-        return launch(lc, k_gemm_tc<false, 32>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
-    }
-    // 256 rows of x per tile (half the weight traffic per flop) once there are more than 128 rows
-    if (n_rows > 128 && gemm_tc_wide && stages_of(256, 192) >= 2) {
-        const dim3 grid((unsigned)((rows_pad + 255) / 256), (out_dim + BM - 1) / BM);
-        p.stages = (uint32_t)stages_of(256, 192);
-        if (dual) return launch(lc, k_gemm_tc<true, 256>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
-        return launch(lc, k_gemm_tc<false, 256>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
+        return dual ? tc_launch<true, 32, 1, 1, 1>(lc, grid, maps, p) : tc_launch<false, 32, 1, 1, 1>(lc, grid, maps, p);
     }
     const dim3 grid((unsigned)(rows_pad / 128), (out_dim + BM - 1) / BM);
-    if (gemm_tc_two_per_sm && stages_of(128, 96) >= 2) {  // half the ring per block, two blocks per SM
-        p.stages = (uint32_t)stages_of(128, 96);
-        if (dual) return launch(lc, k_gemm_tc<true, 128, 2>, grid, dim3(128), SMEM_BYTES_HALF, mw, mw2, mx, mwl, mwl2, p);
-        return launch(lc, k_gemm_tc<false, 128, 2>, grid, dim3(128), SMEM_BYTES_HALF, mw, mw2, mx, mwl, mwl2, p);
-    }
-    p.stages = (uint32_t)stages_of(128, 192);
-    if (p.stages < 2) return cudaErrorInvalidConfiguration;
-    if (dual) return launch(lc, k_gemm_tc<true, 128>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
-    return launch(lc, k_gemm_tc<false, 128>, grid, dim3(128), SMEM_BYTES, mw, mw2, mx, mwl, mwl2, p);
+    // two blocks per SM where half a ring still holds two stages
+    if (x_parts == 1) return dual ? tc_launch<true, 128, 2, 1, 1>(lc, grid, maps, p) : tc_launch<false, 128, 2, 1, 1>(lc, grid, maps, p);
+    if (w_parts == 1) return dual ? tc_launch<true, 128, 1, 2, 1>(lc, grid, maps, p) : tc_launch<false, 128, 2, 2, 1>(lc, grid, maps, p);
+    return dual ? tc_launch<true, 128, 1, 2, 2>(lc, grid, maps, p) : tc_launch<false, 128, 1, 2, 2>(lc, grid, maps, p);
 }
 
 }  // namespace vb

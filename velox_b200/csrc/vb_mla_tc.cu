@@ -27,7 +27,7 @@
 // What a tensor instruction costs (M 128, K 16, measured back to back): N / 2 clocks of arithmetic; with A from shared memory at
 // least 4 KB + the B tile at 128 bytes a clock: 45 clocks at N 16, 53 at N 64, 67 at N 128; with A from tensor memory N / 2 at
 // every N.  Hence 64 tokens a tile (16: three times the clocks per token) and as much of Q as fits in tensor memory: 16 x 53 +
-// 20 x 33 + 4 x 129 = 2.0 k clocks a tile.  These rates need the issuing lane chosen by elect.sync and descriptors known at
+// 20 x 33 + 4 x 129 = 2.0 k clocks a tile.  These rates need the issuing lane chosen by elect.sync (vb_tma.cuh) and descriptors known at
 // compile time up to a base: issued by `lane == 0` from a loop with run-time column blocks the same instructions came 183 clocks
 // apart and the kernel took 270 us instead of 177.
 // Measured, 64 sequences of 1024..8192 tokens (mean 4609): 132 us with conversion (6) and merge (14), 3.2 k clocks a tile, tensor
@@ -111,12 +111,6 @@ __device__ __forceinline__ void tmem_ld_wait(float (&r)[N]) {  // (the registers
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&r)[32]) {
     tmem_ld32_nowait(taddr, r);
     tmem_ld_wait(r);
-}
-// one lane of the (converged) warp, always the same one
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-    return p != 0;
 }
 __device__ __forceinline__ float exp2_fast(float x) {
     float r;

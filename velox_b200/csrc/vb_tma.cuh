@@ -32,6 +32,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (clock64() - t0 > 2000000000LL) return false;
     }
 }
+// One lane of the (converged) warp, always the same one.  Tensor-core and TMA instructions take their operands from uniform
+// registers: under `lane == 0` the compiler has to make them uniform instruction by instruction (the latent attention's 36
+// products of a tile came 183 clocks apart instead of ~55), after elect.sync it knows that one lane runs.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tma_load_1d(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(bar) : "memory");
