@@ -203,7 +203,8 @@ int32_t vb_trace_read(vb_ctx* ctx, uint64_t* out, uint32_t max_records, uint32_t
  *   "attn_mma"       1: tensor-core attention for the fp16 cache; 0: the scalar fp32 path
  *   "fuse_append"    1: bias + RoPE + KV append inside the attention kernel
  *   "prefill_chunk"  prompt tokens that go through the layers together in vb_prefill (16; 1 = token by token)
- *   "prefill_gemm"   1: prompts longer than "prefill_gemm_min" (48) tokens go through the layers in chunks of up to
+ *   "prefill_gemm"   1: prompts longer than "prefill_gemm_min" (16 for int4 group-32 and int8 weights, else 48) tokens go
+ *                    through the layers in chunks of up to
  *                    "prefill_rows" (2048) tokens whose products run on the tcgen05 tensor cores; 0: batched kernels
  *   "prefill_split"  how those chunk products treat the 11 significant bits of fp16 operands: 2 (default): x and the
  *                    weights fp16 cannot hold exactly are multiplied as hi + lo parts (3 tensor-core products, results equal

@@ -6,6 +6,7 @@ import pytest
 import helpers as H
 from oracle import oracle as O
 from velox_b200 import lib as L
+from velox_b200.engine import Engine
 from velox_b200.modelspec import LLAMA3_8B_INT4
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +64,29 @@ def test_canonical_matvec(vb, oracle, fmt, in_dim, out_dim, batch):
     exact = x.astype(np.float64) @ oracle.dequantize(data, scales, c, out_dim, in_dim).astype(np.float64).T
     # fp32 sums of in_dim terms of std 0.02 each: in_dim roundings of 2^-24 of a partial sum below 5 * 0.02 * sqrt(in_dim)
     assert np.max(np.abs(got - exact)) <= in_dim * 2.0 ** -24 * 5 * 0.02 * np.sqrt(in_dim)
+
+
+@pytest.mark.parametrize("fmt,lean", [("q4g32", False), ("q4g32", True), ("i8", False)])
+@pytest.mark.parametrize("n", [17, 33, 34, 65, 66, 129, 140])
+def test_prompt_products_from_tensor_memory(fmt, lean, n):
+    """Prompts whose n - 1 chunk rows are the edges of the row tiles (16, 32, 64, 128) and one more, against the CPU checker.
+    K of 1024 (split over a cluster), 384 and 1408 / 1472, 576 QKV rows (half a tile over).  Steps at shrinking positions
+    look at the cached rows again, each with few others to dilute it."""
+    w, ffn = (L.FMT_Q4G32, 1408) if fmt == "q4g32" else (L.FMT_I8PC, 1472)
+    spec = LLAMA3_8B_INT4.scaled(name="prompt-" + fmt, d_model=1024, n_layers=2, n_q_heads=12, n_kv_heads=3, head_dim=32, ffn_dim=ffn, vocab=1024,
+                                 weight_fmt=w, head_fmt=w)
+    eng = Engine(spec, max_seq_len=160, lean_weights=lean)
+    eng.load_synthetic(41)
+    eng.reserve(0, 160)
+    prompt = H.prompt_tokens(spec, 41, n)
+    eng.prefill(prompt)
+    ora, _ = H.build_oracle(spec, 41, 160)
+    for pos, t in enumerate(prompt):
+        ora.forward_step(int(t), pos)
+    assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL
+    for pos in (n - 1, n // 2, 16, 2, 1):
+        eng.set_state(0, 7, pos)
+        eng.decode(1)
+        ora.forward_step(7, pos)
+        assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
+    eng.close()

@@ -84,13 +84,16 @@ struct vb_ctx {
     int32_t* pfc_table = nullptr;         // [chunk][max_blocks], every row = the sequence's block-table row
     float *pfc_hidden = nullptr, *pfc_qkv = nullptr, *pfc_q = nullptr, *pfc_attn = nullptr, *pfc_act = nullptr;
     uint32_t pfc_rows = 0;                // rows the buffers above hold
-    // prompts of at least `prefill_gemm_min` tokens: chunks of up to `prefill_rows` tokens whose four products per layer
-    // run on the tcgen05 tensor cores (vb_gemm_tc.cu); the workspace holds their fp16 operands
+    // prompts of more than `prefill_gemm_min` tokens: chunks of up to `prefill_rows` tokens whose four products per layer
+    // run on the tcgen05 tensor cores (vb_gemm_tc.cu); the workspace holds their fp16 operands.  int4 group-32 and int8 weights
+    // from `prefill_ts_min` on (vb_gemm_ts.cu: x in parts as fine as those of the kernels for few rows; equal time at 16 rows)
     bool prefill_gemm = true;
     bool decode_gemm = false;   // decode steps of wide batches through the same tensor-core GEMMs (one row per slot)
     bool decode_gemm_auto = false;  // switched on by vb_create, not by the caller: falls back silently when unsupported
     bool prefill_flash = true;  // causal tile attention for those chunks (vb_attn_prefill.cu) instead of one launch row per token
-    uint32_t prefill_rows = 2048, prefill_gemm_min = 48;
+    uint32_t prefill_rows = 2048, prefill_gemm_min = 48, prefill_ts_min = 16;
+    void* ts_ws = nullptr;      // x of a prefill chunk as fp16 parts (vb_gemm_ts.cu)
+    uint64_t ts_ws_bytes = 0;
     void* tc_ws = nullptr;
     uint64_t tc_ws_bytes = 0;
     void* i8_tiles_pool = nullptr;  // tile-major int8 copies of the layer matrices and the head for those products (WMat::i8_tiles)
@@ -141,6 +144,8 @@ struct StepIO {
     const int32_t* block_table;
     uint32_t B;
     bool fused_append;  // false: K/V of all rows are appended by a kernel of their own before attention
+    void* ts_ws = nullptr;  // != null: the layer products run as tensor-core GEMMs that dequantise on the way (vb_gemm_ts.cu)
+    uint64_t ts_ws_bytes = 0;
     void* tc_ws = nullptr;  // != null: the layer products run as tensor-core GEMMs with this workspace
     uint64_t tc_ws_bytes = 0;
     void* i8_ws = nullptr;  // != null: decode batches over int8 weights take the integer tensor-core kernel

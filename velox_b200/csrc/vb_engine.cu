@@ -246,6 +246,37 @@ bool tc_products_ok(vb_ctx* c) {
     return true;
 }
 
+// The same for the products that dequantise into tensor memory (vb_gemm_ts.cu), with the default operand parts.  They read only
+// the packed weights, so they win while the weights are what takes time, and they are the only ones a lean context can run.
+// Four layers of the 8B int4 shape and a last token, ms: 64 rows 1.23 (fp16 copies: 1.58; sixteen rows at a time: 3.3), 128
+// rows 1.55 (1.69), 160 rows 2.37 (2.00); the 7B int8 shape: 64 rows 1.23 (1.85), 128 1.28 (1.95), 200 2.07 (2.19), 256 2.12 (2.22).
+uint32_t ts_rows_max(const vb_ctx* c) { return c->d.weight_fmt == VB_FMT_I8PC ? 256 : 128; }
+bool ts_products_ok(vb_ctx* c) {
+    if (gemm_tc_split != 2) return false;  // fewer parts: the products of vb_gemm_tc.cu
+    const int roles[] = {VB_ROLE_WQ, VB_ROLE_WO, VB_ROLE_WGATE, VB_ROLE_WDOWN};
+    for (int role : roles) {
+        GemvArgs a;
+        a.w = c->tensor(role, 0).m;
+        if (role == VB_ROLE_WQ) a.w.rows = c->qkv_rows;
+        if (role == VB_ROLE_WGATE) { a.w2 = c->tensor(VB_ROLE_WUP, 0).m; a.epilogue = EPI_SWIGLU; }
+        if (!gemm_ts_supported(a)) return false;
+    }
+    return true;
+}
+int32_t ensure_ts_ws(vb_ctx* c, uint32_t rows) {
+    const uint64_t need = gemm_ts_workspace_bytes(std::max(std::max(c->d.d_model, c->ffn), c->qdim), rows);
+    if (c->ts_ws_bytes >= need) return VB_OK;
+    if (c->ts_ws) cudaFree(c->ts_ws);
+    c->ts_ws = nullptr; c->ts_ws_bytes = 0;
+    if (cudaMalloc(&c->ts_ws, need) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("cannot allocate %llu bytes for the rows of a prefill chunk", (unsigned long long)need);
+        return VB_ERR_OOM;
+    }
+    c->ts_ws_bytes = need;
+    return VB_OK;
+}
+
 // Workspace of the tensor-core products for `rows` rows of x (fp16 operands): the largest of a layer's four
 // products, and of the lm_head when `with_head`.
 int32_t ensure_tc_ws(vb_ctx* c, uint32_t rows, bool with_head) {
@@ -424,6 +455,7 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
         return nccl_allreduce_sum_f32(c->nccl, io.hidden, (size_t)B * d.d_model, c->stream) == VB_OK ? cudaSuccess : cudaErrorUnknown;
     };
     auto product = [&](const GemvArgs& ga) -> cudaError_t {
+        if (io.ts_ws) return gemm_ts(lcfg(c, true), ga, io.ts_ws, io.ts_ws_bytes);
         if (io.i8_ws && gemm_i8_supported(ga)) return gemm_i8(lcfg(c, true), ga, io.i8_ws, io.i8_ws_bytes, true);
         if (io.tc_ws) return gemm_tc(lcfg(c, true), ga, io.tc_ws, io.tc_ws_bytes, true);
         GemvArgs gg = ga;
@@ -702,7 +734,7 @@ int32_t vb_destroy(vb_ctx* c) {
     void* frees[] = {c->arena, c->kv_pool, c->block_table_dev, c->state, c->pf_state, c->pf_tokens, c->hidden, c->qkv, c->q,
                      c->attn_out, c->act, c->logits, c->attn_scratch, c->cand_v, c->cand_i, c->rope_inv_freq, c->trace, c->partial, c->tp_pair, c->tp_pairs,
                      c->pfc_state, c->pfc_table, c->pfc_hidden, c->pfc_qkv, c->pfc_q, c->pfc_attn, c->pfc_act, c->tc_ws, c->f16_pool, c->i8_tiles_pool, c->sample_probs,
-                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws, c->frag_ws};
+                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws, c->frag_ws, c->ts_ws};
     for (void* p : frees) if (p) cudaFree(p);
     if (c->ring_host) cudaFreeHost(c->ring_host);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -998,16 +1030,24 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // velox_cuda_runner_k2.cu:1614-1704.)  Sharded contexts and the last token take the per-token path below.
     // Prompts of up to half a chunk go token by token: the same bits as the same tokens fed one step at a time.
     uint32_t done = 0;
-    const bool use_tc = c->prefill_gemm && c->d.tp_size <= 1 && n_tokens > c->prefill_gemm_min && c->prefill_rows >= 1 && tc_products_ok(c);
-    const uint32_t P = use_tc ? std::min(c->prefill_rows, n_tokens - 1) : c->prefill_chunk;
+    const bool gemm_ok = c->prefill_gemm && c->d.tp_size <= 1 && c->prefill_rows >= 1;
+    const bool tc_ok = gemm_ok && n_tokens > c->prefill_gemm_min && tc_products_ok(c);
+    const uint32_t rows = std::min(c->prefill_rows, n_tokens - 1);
+    const bool use_ts = gemm_ok && n_tokens > c->prefill_ts_min && ts_products_ok(c) && (!tc_ok || rows <= ts_rows_max(c));
+    const bool use_tc = use_ts || tc_ok;
+    const uint32_t P = use_tc ? rows : c->prefill_chunk;
     if (use_tc || (P >= 2 && P <= 32 && c->d.tp_size <= 1 && 2 * n_tokens > P)) {
-        const uint32_t cap = use_tc ? c->prefill_rows : P;  // rows the chunk buffers hold
+        uint32_t cap = P;  // rows the chunk buffers hold: a power of two, so that prompts of growing length rarely grow them
+        if (use_tc) { cap = 128; while (cap < P) cap *= 2; }
         if ((rc = ensure_chunk_buffers(c, cap)) != VB_OK) return rc;
-        if (use_tc && ((rc = ensure_f16_copies(c)) != VB_OK || (rc = ensure_tc_ws(c, cap, false)) != VB_OK)) return rc;
+        if (use_ts) { if ((rc = ensure_ts_ws(c, cap)) != VB_OK) return rc; }
+        else if (use_tc && ((rc = ensure_f16_copies(c)) != VB_OK || (rc = ensure_tc_ws(c, cap, false)) != VB_OK)) return rc;
         VB_CUDA(launch(lcfg(c, false), k_fill_chunk_table, dim3(P), dim3(128), 0, c->pfc_table,
                        (const int32_t*)(c->block_table_dev + (size_t)slot * c->max_blocks), c->max_blocks));
         StepIO io{c->pfc_hidden, c->pfc_qkv, c->pfc_q, c->pfc_attn, c->pfc_act, nullptr, c->pfc_table, P, false};
-        if (use_tc) { io.tc_ws = tc_ws_aligned(c); io.tc_ws_bytes = c->tc_ws_bytes; io.causal_chunk = true; }
+        if (use_ts) { io.ts_ws = c->ts_ws; io.ts_ws_bytes = c->ts_ws_bytes; }
+        else if (use_tc) { io.tc_ws = tc_ws_aligned(c); io.tc_ws_bytes = c->tc_ws_bytes; }
+        io.causal_chunk = use_tc;
         // the last token always takes the per-token path below (it produces the logits); the last chunk may be ragged (token by
         // token instead, a 120-token prompt of the 72B shape spent 66 ms on its last 8)
         while (done + 1 < n_tokens) {
@@ -1276,7 +1316,7 @@ int32_t vb_set_option(vb_ctx* c, const char* name, int64_t value) {
     }
     if (!strcmp(name, "prefill_wide")) { gemm_tc_wide = value != 0; return VB_OK; }
     if (!strcmp(name, "prefill_flash")) { c->prefill_flash = value != 0; return VB_OK; }
-    if (!strcmp(name, "prefill_gemm_min")) { c->prefill_gemm_min = (uint32_t)value; return VB_OK; }
+    if (!strcmp(name, "prefill_gemm_min")) { c->prefill_gemm_min = c->prefill_ts_min = (uint32_t)value; return VB_OK; }
     if (!strcmp(name, "prefill_rows")) {
         VB_REQUIRE(value >= 1 && value <= 4096, "vb_set_option: prefill_rows must be in [1, 4096]");
         c->prefill_rows = (uint32_t)value;

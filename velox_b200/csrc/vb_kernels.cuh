@@ -144,6 +144,11 @@ uint64_t gemm_tc_workspace_bytes(uint32_t out_dim, uint32_t in_dim, uint32_t n_r
 // counters_zeroed: the caller zeroed the head of the workspace once (allows the split-K path)
 cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uint64_t workspace_bytes, bool counters_zeroed = false);
 
+// vb_gemm_ts.cu: many rows of x, weights dequantised into tensor memory; the workspace holds the parts of x
+bool gemm_ts_supported(const GemvArgs& a);
+uint64_t gemm_ts_workspace_bytes(uint32_t in_dim, uint32_t n_rows);
+cudaError_t gemm_ts(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uint64_t workspace_bytes);
+
 // vb_gemm_i8.cu: decode batches (<= 32 rows) over int8 per-channel weights on the integer tensor cores, weights read
 // where they lie (one byte per weight), exact arithmetic; workspace head (gemm_i8_workspace_zero_bytes) zero before first use
 extern bool gemm_i8_enabled;
