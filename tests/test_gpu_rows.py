@@ -90,3 +90,27 @@ def test_prompt_products_from_tensor_memory(fmt, lean, n):
         ora.forward_step(7, pos)
         assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
     eng.close()
+
+
+@pytest.mark.parametrize("head_dim,group", [(32, 2), (64, 3), (128, 1), (128, 8), (256, 2)])
+@pytest.mark.parametrize("splits", [1, 3, 7, 11, 16])
+def test_attention_slices(head_dim, group, splits):
+    """Decode attention cut into any number of slices (odd ones: the merge's slices of the head dimension are uneven), against
+    the CPU checker where a slice, a 16-row block or a warp's chunk ends.  Positions shrink: a step overwrites its own row."""
+    spec = LLAMA3_8B_INT4.scaled(name="slices", d_model=256, n_layers=2, n_q_heads=2 * group, n_kv_heads=2, head_dim=head_dim, ffn_dim=256, vocab=512,
+                                 weight_fmt=L.FMT_F16, head_fmt=L.FMT_F16)
+    eng = H.build_engine(spec, 51, 320)
+    eng.set_option("attn_splits", splits)
+    eng.reserve(0, 320)
+    prompt = H.prompt_tokens(spec, 51, 300)
+    eng.prefill(prompt)
+    ora, _ = H.build_oracle(spec, 51, 320)
+    for pos, t in enumerate(prompt):
+        ora.forward_step(int(t), pos)
+    assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL
+    for pos in (299, 257, 256, 255, 130, 33, 16, 15, 1, 0):
+        eng.set_state(0, 5, pos)
+        eng.decode(1)
+        ora.forward_step(5, pos)
+        assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
+    eng.close()

@@ -14,8 +14,8 @@
 // heads of the group, reduces the per-lane partial dot products with a transposing butterfly (one value per
 // lane instead of one reduction per value); online-softmax state (m, l, acc) per query head in fp32 throughout.
 // The splits of one (sequence, head group) form a
-// thread-block cluster: each block pushes slice j of its partial into block j's shared memory (distributed
-// shared memory stores) and, after one cluster barrier, every block merges its slice of the head dimension
+// thread-block cluster: each block pushes slice j of its partial into block j's shared memory (asynchronous
+// stores that count themselves off at a barrier there), then every block merges its slice of the head dimension
 // locally -- no global round trip, no atomics, a fixed merge order.
 // In the engine the kernel also does what the reference runs as separate kernels before attention
 // (fused_rope_kernel and the KV write of fused_qkv, src/runners/tinystories_smollm.cu:189-318): bias, RoPE of
@@ -29,6 +29,8 @@
 // per layer [block][K|V][kv_head][block_tokens][D].
 #include <cooperative_groups.h>
 #include <stdlib.h>
+
+#include <type_traits>
 
 #include "vb_internal.cuh"
 #include <cuda.h>
@@ -46,7 +48,8 @@ constexpr int ATTN_WARPS = 8;
 // (the legacy tensor path takes ~64 clocks per mma.sync per scheduler: a 16-token tile is 32 of them) and moves the
 // full-depth logits from 0.0149 to 0.0160 of the checker's: the two products stay
 constexpr bool ATTN_SPLIT_P = true;
-constexpr int ATTN_MAX_SPLITS = 8;  // portable thread-block cluster size
+constexpr int ATTN_MAX_SPLITS = 8;  // portable thread-block cluster size (any number of splits up to it)
+constexpr int ATTN_CLUSTER = 16;    // the largest cluster of the device (a power of two: it divides every head dimension)
 constexpr int ATTN_SPEC_BLOCKS = ATTN_WARPS * 32;  // block-table rows up to this long are fetched whole, before the position is known
 
 struct AttnKArgs {
@@ -207,7 +210,9 @@ struct AttnSmem {
     static constexpr int CH_FIT = (MMA ? 32768 : 16384) / (D * (int)sizeof(KVT));
     static constexpr int CH = CH_FIT > CH_CAP ? CH_CAP : CH_FIT;
     static constexpr size_t kv_bytes = (size_t)2 * 2 * CH * RS * sizeof(KVT);  // [buffer][K|V][CH][RS]
-    static constexpr size_t acc_bytes = (size_t)ATTN_WARPS * GM * D * sizeof(float);
+    // mma.sync path: only the low halves of Q; the warps' partials take the place of the staged rows at the end
+    static constexpr size_t acc_bytes = MMA == 1 ? (size_t)16 * D : (size_t)ATTN_WARPS * GM * D * sizeof(float);
+    static_assert(MMA != 1 || (size_t)ATTN_WARPS * GM * D * sizeof(float) <= kv_bytes, "partials");
     // tensor-core paths: staging aligned to 1024 bytes; tcgen05 path: + the Q and P operands (4 KB each)
     static constexpr size_t total = kv_bytes + acc_bytes + (MMA ? 1024 : 0) + (MMA == 2 ? 8192 : 0);
 };
@@ -226,9 +231,12 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     __shared__ float q_s[GM][D];
     __shared__ float sc_s[MMA ? 1 : ATTN_WARPS][32];   // scalar path: a warp's scores
     __shared__ float part_ml[ATTN_WARPS][GM][2];
-    __shared__ float gath[GM * (D + 32)];   // partials of all splits for this block's slice of the head dimension
+    // partials of all splits for this block's slice of the head dimension: [split][GM] {M, L}, then [split][GM][slice]
+    __shared__ __align__(16) float gath[GM * (2 * ATTN_CLUSTER + D + ATTN_CLUSTER)];
+    __shared__ __align__(8) unsigned long long push_bar;  // completes when all of them have arrived
     __shared__ float rope_cs[D / 2], rope_sn[D / 2];
-    __shared__ __align__(8) unsigned long long kv_bar[2];  // one transaction barrier per staging buffer
+    // one transaction barrier per staging buffer; mma.sync path: one per buffer and warp, at [buffer * ATTN_WARPS + warp]
+    __shared__ __align__(8) unsigned long long kv_bar[MMA == 1 ? 2 * ATTN_WARPS : 2];
     __shared__ int32_t blk_s[ATTN_SPEC_BLOCKS];             // the sequence's block-table row (short tables only)
     __shared__ __align__(16) KVT new_kv[2][D];  // the appended token's K and V (fused mode)
     __shared__ __align__(8) unsigned long long tc_bar[2];  // tcgen05 path: S ready, P . V done (one completion per chunk each)
@@ -237,10 +245,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     unsigned char* dyn_base = MMA ? dyn_smem + ((1024u - (smem_u32(dyn_smem) & 1023u)) & 1023u) : dyn_smem;
     KVT* kv_s = reinterpret_cast<KVT*>(dyn_base);
-    float* part_acc = reinterpret_cast<float*>(dyn_base + SM::kv_bytes);  // [ATTN_WARPS][GM][D]
-    // tensor-core path: until the warps' partials are written there (after the last chunk's barrier), the same bytes hold
-    // the low halves of Q (q - fp16(q)) as B fragments, the same for every warp: [k step][lane], 16 * D bytes
-    uint2* qlo_s = reinterpret_cast<uint2*>(part_acc);
+    float* part_acc = reinterpret_cast<float*>(dyn_base + (MMA == 1 ? 0 : SM::kv_bytes));  // [ATTN_WARPS][GM][D]
+    // mma.sync path: the low halves of Q (q - fp16(q)) as B fragments, the same for every warp: [k step][lane], 16 * D bytes
+    uint2* qlo_s = reinterpret_cast<uint2*>(dyn_base + SM::kv_bytes);
     // tcgen05 path: the B operands, [q_hi (8 heads) | q_lo (8 heads)] as 16 rows x 128 dimensions (two 64-column halves, 128-byte
     // swizzle) and [p_hi | p_lo] as 16 rows x 128 tokens (core matrices of 8 rows x 16 bytes)
     unsigned char* qop = dyn_base + SM::kv_bytes + SM::acc_bytes;
@@ -271,6 +278,13 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     const bool appender = a.qkv_raw && t_lo <= pos && pos < t_hi;
     // every block of the cluster must be running before anyone writes into its shared memory: arrive now,
     // wait just before the pushes (the barrier's latency hides behind the attention itself)
+    const uint32_t per_d = ((uint32_t)D + ka.n_splits - 1) / ka.n_splits;  // this block merges dimensions d_lo .. d_hi - 1
+    const uint32_t d_lo = min((uint32_t)D, split * per_d), d_hi = min((uint32_t)D, d_lo + per_d);
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&push_bar), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(smem_u32(&push_bar), ka.n_splits * ng * (d_hi > d_lo ? (d_hi - d_lo) * 4 + 8 : 0));
+    }
     cg::cluster_group cluster = cg::this_cluster();
     cluster.barrier_arrive();
     // tensor-core path: S^T = K Q^T (16 tokens x 8 heads per mma) and O^T = V^T P^T (16 dims x 8 heads), so the
@@ -307,7 +321,20 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
         const uint32_t NT = ATTN_WARPS * 32;
         const uint32_t me = (threadIdx.x + NT - rot) % NT;
         const uint32_t row_bytes = D * (uint32_t)sizeof(KVT);
-        if constexpr (MMA) {
+        if constexpr (MMA == 1) {
+            // every warp fetches its own 16 tokens of the chunk, one tiled copy per lane (K or V, 64-column half): 16 rows of
+            // 128 bytes, swizzled
+            const uint32_t tok = c0 + warp * 16u, i = (lane + 32u - rot) % 32u;
+            if (warp < CH / 16 && tok < t_hi && i < 2 * HV) {
+                const uint32_t wbar = smem_u32(&kv_bar[buf * ATTN_WARPS + warp]), h = i % HV, kv = i / HV;
+                if (i == 0) mbar_expect_tx(wbar, 2 * HV * 2048u);
+                const int32_t blk = spec_table ? blk_s[tok / 16u] : a.block_table[(size_t)b * a.max_blocks + tok / 16u];
+                const int y = (int)(a.kv_map_row0 + (((uint32_t)blk * 2 + kv) * a.Hkv + kvh) * 16u);
+                const uint32_t dst = smem_u32(kb) + ((kv * HV + h) * CH + warp * 16u) * 128u;
+                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                             ::"r"(dst), "l"(&ka.kv_map), "r"((int)(h * 64u)), "r"(y), "r"(wbar) : "memory");
+            }
+        } else if constexpr (MMA) {
             // one tiled copy per (KV block, K or V, 64-column half): 16 rows of 128 bytes, swizzled
             const uint32_t nb = (n_tok + 15u) / 16u;
             if (me == 0) mbar_expect_tx(bar, nb * 2 * HV * 2048u);
@@ -359,8 +386,8 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     constexpr int QIT = (GM * (int)half + ATTN_WARPS * 32 - 1) / (ATTN_WARPS * 32);  // (head, pair) items per thread
     float bq1[QIT], bq2[QIT], bk1 = 0.f, bk2 = 0.f, bv1 = 0.f, bv2 = 0.f;
     if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&kv_bar[0]), 1);
-        mbar_init(smem_u32(&kv_bar[1]), 1);
+#pragma unroll
+        for (int i = 0; i < (MMA == 1 ? 2 * ATTN_WARPS : 2); ++i) mbar_init(smem_u32(&kv_bar[i]), 1);
         if constexpr (MMA == 2) { mbar_init(smem_u32(&tc_bar[0]), 1); mbar_init(smem_u32(&tc_bar[1]), 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -376,9 +403,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     uint32_t tmem = 0;
     if constexpr (MMA == 2) { at_fence_after(); tmem = tc_tmem_slot; }
     if (early) {
-        // the requests for the first two chunks, spread over the block (one copy per thread or fewer)
+        // the requests for the first two chunks (one copy per thread or fewer)
         if (n_ch > 0) stage_chunk(0, 0, 0);
-        if (n_ch > 1) stage_chunk(1, 1, ATTN_WARPS * 16);
+        if (n_ch > 1) stage_chunk(1, 1, MMA == 1 ? 8 : ATTN_WARPS * 16);
     }
     if (a.qkv_raw && warp != 0) {
         // rotary angles of this position (one sincos per frequency, shared by all heads)
@@ -411,7 +438,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     trace_mark(a.trace, 1);
     if (!early) {
         if (n_ch > 0) stage_chunk(0, 0, 0);
-        if (n_ch > 1) stage_chunk(1, 1, ATTN_WARPS * 16);
+        if (n_ch > 1) stage_chunk(1, 1, MMA == 1 ? 8 : ATTN_WARPS * 16);
     }
 
     if (has_tokens) {
@@ -515,6 +542,93 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
         }
 
         // ---- the slice, CH tokens at a time through the two buffers (both were requested above) ----------------
+        if constexpr (MMA == 1) {
+            // Each warp walks through its own 16 tokens of every chunk: own barriers, no block-wide step until the merge.  (With
+            // block-wide chunks a buffer was requested again only when the slowest warp was through with it: a layer of the 8B
+            // shape at 7900 cached rows 68.7 us, so 63.8; a third buffer gave another 0.3.)
+            const uint32_t mi = lane >> 3, r8 = lane & 7, tok0 = warp * 16;
+            for (uint32_t c = 0; c < n_ch; ++c) {
+                const uint32_t c0 = t_lo + c * CH, buf = c & 1, t0 = c0 + tok0;
+                if (warp >= CH / 16 || t0 >= t_hi) break;
+                if (!mbar_wait(smem_u32(&kv_bar[buf * ATTN_WARPS + warp]), (c >> 1) & 1) && a.err) atomicOr(a.err, 0x400u);
+                KVT* kb = kv_s + (size_t)buf * 2 * CH * RS;
+                // the copies moved a whole KV block: rows past the context's end hold whatever the pool held (they are
+                // multiplied with probability 0 and must be numbers), and the new token's row is older than this step
+                const uint32_t n_valid = min(16u, t_hi - t0);
+                const bool patch = appender && t0 <= pos && pos < t0 + 16u;
+                if (patch || n_valid != 16u) {
+                    for (uint32_t i = lane; i < (16u - n_valid) * 2 * ROW16; i += 32) {
+                        const uint32_t piece = i % ROW16, rowi = i / ROW16, kv = rowi & 1, r = tok0 + n_valid + (rowi >> 1);
+                        reinterpret_cast<uint4*>(kb + ((size_t)(kv * HV + (piece >> 3)) * CH + r) * 64)[piece & 7] = make_uint4(0, 0, 0, 0);
+                    }
+                    if (patch) {
+                        const uint32_t r = pos - c0;
+                        for (uint32_t i = lane; i < 2 * ROW16; i += 32) {
+                            const uint32_t kv = i / ROW16, piece = i % ROW16;
+                            reinterpret_cast<uint4*>(kb + ((size_t)(kv * HV + (piece >> 3)) * CH + r) * 64)[(piece & 7) ^ (r & 7)] =
+                                reinterpret_cast<const uint4*>(new_kv[kv])[piece];
+                        }
+                    }
+                    __syncwarp();
+                }
+                // scores of 16 tokens x 8 heads
+                float sc4[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sl4[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // against the high and the low halves of Q
+                // row (tok0 + (mi & 1) * 8 + r8) of K, 16-byte piece q = 2 * ks + (mi >> 1) of its D / 8: half q >> 3,
+                // piece (q & 7) ^ r8 of the 128-byte row
+                const uint32_t k_row = smem_u32(kb) + (tok0 + (mi & 1) * 8 + r8) * 128u;
+#pragma unroll
+                for (int ks = 0; ks < MT; ++ks) {
+                    uint32_t af[4];
+                    const uint32_t q = 2u * ks + (mi >> 1);
+                    ldsm_x4(af, k_row + (q >> 3) * (CH * 128u) + (((q & 7u) ^ r8) << 4));
+                    const uint2 ql = qlo_s[ks * 32 + lane];
+                    mma_f16_16816(sc4, af, qb[ks][0], qb[ks][1]);
+                    mma_f16_16816(sl4, af, ql.x, ql.y);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sc4[e] += sl4[e];
+                // this thread: tokens tA = lane / 4 and tA + 8 of the tile, heads 2 * (lane & 3) and + 1
+                const uint32_t tA = c0 + tok0 + (lane >> 2);
+                const bool vA = tA < t_hi, vB = tA + 8 < t_hi;
+                const float s0 = vA ? sc4[0] * ka.scale : -INFINITY, s1 = vA ? sc4[1] * ka.scale : -INFINITY;
+                const float s2 = vB ? sc4[2] * ka.scale : -INFINITY, s3 = vB ? sc4[3] * ka.scale : -INFINITY;
+                float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
+#pragma unroll
+                for (int off = 4; off < 32; off <<= 1) {
+                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, off));
+                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, off));
+                }
+                const float nm0 = fmaxf(m2[0], mx0), nm1 = fmaxf(m2[1], mx1);
+                const float al0 = (m2[0] == -INFINITY) ? 0.0f : __expf(m2[0] - nm0);
+                const float al1 = (m2[1] == -INFINITY) ? 0.0f : __expf(m2[1] - nm1);
+                const float p0 = (nm0 == -INFINITY) ? 0.0f : __expf(s0 - nm0), p2 = (nm0 == -INFINITY) ? 0.0f : __expf(s2 - nm0);
+                const float p1 = (nm1 == -INFINITY) ? 0.0f : __expf(s1 - nm1), p3 = (nm1 == -INFINITY) ? 0.0f : __expf(s3 - nm1);
+                l2[0] = fmaf(l2[0], al0, p0 + p2);
+                l2[1] = fmaf(l2[1], al1, p1 + p3);
+                m2[0] = nm0; m2[1] = nm1;
+                // P^T as B fragments (k = token, n = head): transpose the two 8x8 halves of the score tile
+                const uint32_t pb0 = movmatrix_trans(pack_half2(p0, p1));
+                const uint32_t pb1 = movmatrix_trans(pack_half2(p2, p3));
+                const uint32_t pl0 = movmatrix_trans(pack_half2(p0 - half_round(p0), p1 - half_round(p1)));
+                const uint32_t pl1 = movmatrix_trans(pack_half2(p2 - half_round(p2), p3 - half_round(p3)));
+                const uint32_t v_row = smem_u32(kb) + HV * (CH * 128u) + (tok0 + (mi >> 1) * 8 + r8) * 128u;
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    o_t[mt][0] *= al0; o_t[mt][2] *= al0; o_t[mt][1] *= al1; o_t[mt][3] *= al1;
+                    uint32_t af[4];
+                    const uint32_t q = 2u * mt + (mi & 1);
+                    ldsm_x4_trans(af, v_row + (q >> 3) * (CH * 128u) + (((q & 7u) ^ r8) << 4));
+                    mma_f16_16816(o_t[mt], af, pb0, pb1);
+                    if constexpr (ATTN_SPLIT_P) mma_f16_16816(o_t[mt], af, pl0, pl1);
+                }
+                __syncwarp();  // the warp is done with the buffer: it takes the chunk after next
+                if (c + 2 < n_ch) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    stage_chunk(c + 2, buf, 0);
+                }
+            }
+            __syncthreads();  // every staged row is read: their place takes the warps' partials
+        } else
         for (uint32_t c = 0; c < n_ch; ++c) {
             const uint32_t c0 = t_lo + c * CH, buf = c & 1;
             if (!mbar_wait(smem_u32(&kv_bar[buf]), (c >> 1) & 1) && a.err) atomicOr(a.err, 0x400u);
@@ -627,60 +741,6 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
                 // the staging buffer, the P operand and S^T are free again once that product is done
                 if (!mbar_wait(o_bar, c & 1) && a.err) atomicOr(a.err, 0x1000u);
                 at_fence_after();
-            } else if constexpr (MMA) {
-                const uint32_t n_tiles = (c_hi - c0 + 15) / 16;
-                const uint32_t mi = lane >> 3, r8 = lane & 7;
-                for (uint32_t tile = warp; tile < n_tiles; tile += ATTN_WARPS) {
-                    const uint32_t tok0 = tile * 16;
-                    // scores of 16 tokens x 8 heads
-                    float sc4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    // row (tok0 + (mi & 1) * 8 + r8) of K, 16-byte piece q = 2 * ks + (mi >> 1) of its D / 8: half q >> 3,
-                    // piece (q & 7) ^ r8 of the 128-byte row
-                    const uint32_t k_row = smem_u32(kb) + (tok0 + (mi & 1) * 8 + r8) * 128u;
-#pragma unroll
-                    for (int ks = 0; ks < MT; ++ks) {
-                        uint32_t af[4];
-                        const uint32_t q = 2u * ks + (mi >> 1);
-                        ldsm_x4(af, k_row + (q >> 3) * (CH * 128u) + (((q & 7u) ^ r8) << 4));
-                        const uint2 ql = qlo_s[ks * 32 + lane];
-                        mma_f16_16816(sc4, af, qb[ks][0], qb[ks][1]);
-                        mma_f16_16816(sc4, af, ql.x, ql.y);
-                    }
-                    // this thread: tokens tA = lane / 4 and tA + 8 of the tile, heads 2 * (lane & 3) and + 1
-                    const uint32_t tA = c0 + tok0 + (lane >> 2);
-                    const bool vA = tA < c_hi, vB = tA + 8 < c_hi;
-                    const float s0 = vA ? sc4[0] * ka.scale : -INFINITY, s1 = vA ? sc4[1] * ka.scale : -INFINITY;
-                    const float s2 = vB ? sc4[2] * ka.scale : -INFINITY, s3 = vB ? sc4[3] * ka.scale : -INFINITY;
-                    float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
-#pragma unroll
-                    for (int off = 4; off < 32; off <<= 1) {
-                        mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, off));
-                        mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, off));
-                    }
-                    const float nm0 = fmaxf(m2[0], mx0), nm1 = fmaxf(m2[1], mx1);
-                    const float al0 = (m2[0] == -INFINITY) ? 0.0f : __expf(m2[0] - nm0);
-                    const float al1 = (m2[1] == -INFINITY) ? 0.0f : __expf(m2[1] - nm1);
-                    const float p0 = (nm0 == -INFINITY) ? 0.0f : __expf(s0 - nm0), p2 = (nm0 == -INFINITY) ? 0.0f : __expf(s2 - nm0);
-                    const float p1 = (nm1 == -INFINITY) ? 0.0f : __expf(s1 - nm1), p3 = (nm1 == -INFINITY) ? 0.0f : __expf(s3 - nm1);
-                    l2[0] = fmaf(l2[0], al0, p0 + p2);
-                    l2[1] = fmaf(l2[1], al1, p1 + p3);
-                    m2[0] = nm0; m2[1] = nm1;
-                    // P^T as B fragments (k = token, n = head): transpose the two 8x8 halves of the score tile
-                    const uint32_t pb0 = movmatrix_trans(pack_half2(p0, p1));
-                    const uint32_t pb1 = movmatrix_trans(pack_half2(p2, p3));
-                    const uint32_t pl0 = movmatrix_trans(pack_half2(p0 - half_round(p0), p1 - half_round(p1)));
-                    const uint32_t pl1 = movmatrix_trans(pack_half2(p2 - half_round(p2), p3 - half_round(p3)));
-                    const uint32_t v_row = smem_u32(kb) + HV * (CH * 128u) + (tok0 + (mi >> 1) * 8 + r8) * 128u;
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        o_t[mt][0] *= al0; o_t[mt][2] *= al0; o_t[mt][1] *= al1; o_t[mt][3] *= al1;
-                        uint32_t af[4];
-                        const uint32_t q = 2u * mt + (mi & 1);
-                        ldsm_x4_trans(af, v_row + (q >> 3) * (CH * 128u) + (((q & 7u) ^ r8) << 4));
-                        mma_f16_16816(o_t[mt], af, pb0, pb1);
-                        if constexpr (ATTN_SPLIT_P) mma_f16_16816(o_t[mt], af, pl0, pl1);
-                    }
-                }
             } else
             for (uint32_t t0 = c0 + warp * TCH; t0 < c_hi; t0 += ATTN_WARPS * TCH) {
                 float kr[TCH][EPL], vr[TCH][EPL];
@@ -809,48 +869,76 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     }
     __syncthreads();
     // ---- ... and push it to the blocks of the cluster (the splits of one sequence and head group): block j
-    // merges slice j of the head dimension, so every value goes to exactly one block's shared memory.  One
-    // cluster barrier later each block holds all it needs locally: no global round trip, no atomics, a fixed
-    // merge order, and nobody reads remote memory after the barrier (blocks may leave at once).
+    // merges slice j of the head dimension, so every value goes to exactly one block's shared memory.  The stores
+    // count themselves off at the receiver's transaction barrier, so a block goes on when ITS values are there, without
+    // a second cluster barrier: no global round trip, no atomics, a fixed merge order, and nobody reads remote memory (blocks may leave at
+    // once: a block that still waits is alive, and nothing is sent to one that does not).
     cluster.barrier_wait();
     const uint32_t n = ka.n_splits;  // == cluster size along y
-    const uint32_t per_d = (D + n - 1) / n;
-    const uint32_t gstride = per_d + 2;  // per (source split, head): M, L, per_d accumulators
-    for (uint32_t i = threadIdx.x; i < GM * D; i += blockDim.x) {
-        const uint32_t g = i / D, d = i % D;
-        float M = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < ATTN_WARPS; ++w) M = fmaxf(M, part_ml[w][g][0]);
-        float L = 0.0f, A = 0.0f;
-#pragma unroll
-        for (int w = 0; w < ATTN_WARPS; ++w) {
-            const float mw = part_ml[w][g][0];
-            const float f = (mw == -INFINITY) ? 0.0f : __expf(mw - M);
-            L = fmaf(part_ml[w][g][1], f, L);
-            A = fmaf(part_acc[((size_t)w * GM + g) * D + d], f, A);
-        }
-        if (g < ng) {
-            const uint32_t owner = d / per_d, dd = d - owner * per_d;
-            float* dst = cluster.map_shared_rank(gath, owner) + ((size_t)split * GM + g) * gstride;
-            dst[2 + dd] = A;
-            if (dd == 0) { dst[0] = M; dst[1] = L; }
-        }
-    }
-    cluster.sync();
-    const uint32_t d_lo = split * per_d, d_hi = min((uint32_t)D, d_lo + per_d);
-    for (uint32_t i = threadIdx.x; i < ng * per_d; i += blockDim.x) {
-        const uint32_t g = i / per_d, dd = i % per_d, d = d_lo + dd;
-        if (d < d_hi) {
+    float* gacc = gath + 2 * ATTN_CLUSTER * GM;  // [split][GM][per_d]
+    const uint32_t gath_a = smem_u32(gath), gacc_a = smem_u32(gacc), bar_a = smem_u32(&push_bar);
+    auto push = [&](auto vec) {
+        constexpr int V = decltype(vec)::value;  // consecutive dimensions a thread merges and sends
+        for (uint32_t i = threadIdx.x; i < GM * D / V; i += blockDim.x) {
+            const uint32_t g = i / (D / V), d = i % (D / V) * V;
             float M = -INFINITY;
-            for (uint32_t r = 0; r < n; ++r) M = fmaxf(M, gath[((size_t)r * GM + g) * gstride]);
-            float L = 0.0f, A = 0.0f;
-            for (uint32_t r = 0; r < n; ++r) {
-                const float* src = gath + ((size_t)r * GM + g) * gstride;
-                const float f = (src[0] == -INFINITY) ? 0.0f : __expf(src[0] - M);
-                L = fmaf(src[1], f, L);
-                A = fmaf(src[2 + dd], f, A);
+#pragma unroll
+            for (int w = 0; w < ATTN_WARPS; ++w) M = fmaxf(M, part_ml[w][g][0]);
+            float L = 0.0f, A[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) A[e] = 0.0f;
+#pragma unroll
+            for (int w = 0; w < ATTN_WARPS; ++w) {
+                const float mw = part_ml[w][g][0];
+                const float f = (mw == -INFINITY) ? 0.0f : __expf(mw - M);
+                L = fmaf(part_ml[w][g][1], f, L);
+                const float* pa = &part_acc[((size_t)w * GM + g) * D + d];
+                if constexpr (V == 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(pa);
+                    A[0] = fmaf(v.x, f, A[0]); A[1] = fmaf(v.y, f, A[1]); A[2] = fmaf(v.z, f, A[2]); A[3] = fmaf(v.w, f, A[3]);
+                } else {
+                    A[0] = fmaf(pa[0], f, A[0]);
+                }
             }
-            a.out[(size_t)b * a.Hq * D + (size_t)(kvh * ka.G + g0 + g) * D + d] = (L > 0.0f) ? (A / L) : 0.0f;
+            if (g < ng) {
+                const uint32_t owner = d / per_d, dd = d - owner * per_d;
+                uint32_t bar, acc, ml;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(bar_a), "r"(owner));
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(acc) : "r"(gacc_a + ((split * GM + g) * per_d + dd) * 4), "r"(owner));
+                if constexpr (V == 4)
+                    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                                 ::"r"(acc), "r"(__float_as_uint(A[0])), "r"(__float_as_uint(A[1])), "r"(__float_as_uint(A[2])), "r"(__float_as_uint(A[3])), "r"(bar) : "memory");
+                else
+                    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(acc), "r"(__float_as_uint(A[0])), "r"(bar) : "memory");
+                if (dd == 0) {
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ml) : "r"(gath_a + (split * GM + g) * 8), "r"(owner));
+                    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                                 ::"r"(ml), "r"(__float_as_uint(M)), "r"(__float_as_uint(L)), "r"(bar) : "memory");
+                }
+            }
+        }
+    };
+    if (per_d % 4 == 0) push(std::integral_constant<int, 4>{});
+    else push(std::integral_constant<int, 1>{});
+    // bounded like the copies' waits; the peers' own waits come first, so it gets twice their limit
+    if (threadIdx.x < ((ng * per_d + 31) & ~31u)) {
+        bool here = mbar_wait(bar_a, 0) || mbar_wait(bar_a, 0);
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        if (!here && a.err) atomicOr(a.err, 0x2000u);
+        for (uint32_t i = threadIdx.x; here && i < ng * per_d; i += blockDim.x) {
+            const uint32_t g = i / per_d, dd = i % per_d, d = d_lo + dd;
+            if (d < d_hi) {
+                float M = -INFINITY;
+                for (uint32_t r = 0; r < n; ++r) M = fmaxf(M, gath[(r * GM + g) * 2]);
+                float L = 0.0f, A = 0.0f;
+                for (uint32_t r = 0; r < n; ++r) {
+                    const float2 ml = *reinterpret_cast<const float2*>(gath + (r * GM + g) * 2);
+                    const float f = (ml.x == -INFINITY) ? 0.0f : __expf(ml.x - M);
+                    L = fmaf(ml.y, f, L);
+                    A = fmaf(gacc[(r * GM + g) * per_d + dd], f, A);
+                }
+                a.out[(size_t)b * a.Hq * D + (size_t)(kvh * ka.G + g0 + g) * D + d] = (L > 0.0f) ? (A / L) : 0.0f;
+            }
         }
     }
     trace_exit(a.trace);
@@ -885,14 +973,14 @@ bool attn_use_mma = true;  // fp16 caches with head_dim <= 256: QK^T and PV on t
 template <typename KVT, int EPL, int GM, int MMA>
 static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka) {
     ka.g_chunks = (ka.G + GM - 1) / GM;
-    const size_t smem = AttnSmem<KVT, EPL, GM, MMA>::total;
     dim3 grid(ka.a.Hkv * ka.g_chunks, ka.n_splits, ka.a.batch);
+    const size_t smem = AttnSmem<KVT, EPL, GM, MMA>::total;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(ATTN_WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = lc.stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = ka.n_splits; attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
@@ -900,6 +988,12 @@ static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
+    }
+    if (EPL <= 2 && MMA == 1) {
+        // 66 KB: three blocks would fit an SM, and the driver would give shared memory all of it; the products around this kernel
+        // stream their weights through L1 and wait for the split to change back (6 layers of the 135M shape 156 us, so 146)
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = 72;
     }
     cfg.attrs = attr;
     if (lc.counter) ++*lc.counter;
@@ -951,14 +1045,17 @@ template <typename KVT, int EPL, int GM>
 static cudaError_t opt_in_one() {
     cudaError_t e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)AttnSmem<KVT, EPL, GM, 0>::total);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if constexpr (sizeof(KVT) == 2 && EPL >= 2 && EPL <= 8) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)AttnSmem<KVT, EPL, GM, 1>::total);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if constexpr (EPL == 4) {
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)AttnSmem<KVT, EPL, GM, 2>::total);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         }
     }
     return e;

@@ -654,6 +654,10 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
         const uint32_t g = c->hq / c->hkv, pairs = d.max_batch * c->hkv * ((g + 7) / 8);
         const uint32_t fit = pairs ? 148u / pairs : 8u;  // one block per SM: two 128-token staging buffers take most of its shared memory
         if (c->n_splits > (fit ? fit : 1u)) c->n_splits = fit ? fit : 1u;
+        // A few pairs and long contexts: clusters of 16.  Eight of them do not find room at once on this part (10 blocks each
+        // do, for 1 % at 7900 rows and minus 1 % at 500), four do; below ~3000 rows the wider merge costs what it gives (us per
+        // step, 8 -> 16 splits, 4 layers of the 7B shape, 4 KV heads: 512 rows 333 -> 335, 4096 350 -> 338, 7900 365 -> 352).
+        if (pairs <= 4 && d.max_seq_len >= 4096) c->n_splits = 16;
     }
     c->tokens_per_split = attn_tokens_per_split(d.max_seq_len);
     c->t.resize((size_t)VB_ROLE_COUNT * d.n_layers);
@@ -1333,7 +1337,7 @@ int32_t vb_set_option(vb_ctx* c, const char* name, int64_t value) {
         return VB_OK;
     }
     if (!strcmp(name, "attn_splits")) {
-        VB_REQUIRE(value >= 1 && value <= 8, "vb_set_option: attn_splits is 1..8 (a thread-block cluster)");
+        VB_REQUIRE(value >= 1 && value <= 16, "vb_set_option: attn_splits is 1..16 (a thread-block cluster)");
         c->n_splits = (uint32_t)value;
         return VB_OK;
     }
