@@ -118,16 +118,30 @@ __device__ __forceinline__ void im_stage_chunk(unsigned char* __restrict__ xq, i
     float p = 1.0f;
     if (gmax > 0.0f && gmax < 3.0e38f) p = __fdividef(32000.0f, gmax);
     if (!(p < 3.0e38f)) p = 1.0f;
-    int X[8], s = 0;
-    uint32_t hw[2] = {0u, 0u}, lw[2] = {0u, 0u};
+    float y[8], odd = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { y[i] = v[i] * p; odd = fmaf(y[i], 0.0f, odd); }
+    if (odd != 0.0f || !(gmax < 3.0e38f)) {  // NaN counts as 0, infinities and what p = 1 leaves too large go to the end of the range
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = y[i] == y[i] ? fmaxf(-32639.0f, fminf(32639.0f, y[i])) : 0.0f;
+    }
+    // (Conversion, clamp, shifts and masks element by element were ~110 instructions, this is ~50: 0.6 us of a 41 us layer of the
+    // 8B int4 shape, 0.7 of the 7B int8 one, all of it time in which HBM idles.)
+    // Adding 1.5 * 2^23 leaves rint(y) in the low bits: the low 16 are X modulo 2^16, whose low byte is L as a signed byte; byte
+    // 1 of X + 128 is H.  Byte permutes then collect four planes' bytes in three instructions each.
+    uint32_t xb[8], hb[8];
+    int s = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        X[i] = __float2int_rn(v[i] * p);
-        X[i] = max(-32639, min(32639, X[i]));
-        s += X[i];
-        const int H = (X[i] + 128) >> 8, L = X[i] - (H << 8);
-        hw[i >> 2] |= (uint32_t)(H & 0xFF) << (8 * (i & 3));
-        lw[i >> 2] |= (uint32_t)(L & 0xFF) << (8 * (i & 3));
+        xb[i] = __float_as_uint(__fadd_rn(y[i], 12582912.0f));
+        hb[i] = xb[i] + 128u;
+        s += (int)(xb[i] - 0x4B400000u);
+    }
+    uint32_t hw[2], lw[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        lw[i] = __byte_perm(__byte_perm(xb[4 * i], xb[4 * i + 1], 0x0040), __byte_perm(xb[4 * i + 2], xb[4 * i + 3], 0x0040), 0x5410);
+        hw[i] = __byte_perm(__byte_perm(hb[4 * i], hb[4 * i + 1], 0x0051), __byte_perm(hb[4 * i + 2], hb[4 * i + 3], 0x0051), 0x5410);
     }
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
