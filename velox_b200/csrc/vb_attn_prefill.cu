@@ -51,7 +51,8 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t h = blockIdx.y, kvh = h / (Hq / Hkv);
-    const uint32_t r0 = blockIdx.x * QROWS;
+    // the last rows have the most to look at: they start first, so that the short ones fill the tail
+    const uint32_t r0 = (gridDim.x - 1 - blockIdx.x) * QROWS;
     const uint32_t rows_here = min((uint32_t)QROWS, n - r0);
     const uint32_t kv_len = first + r0 + rows_here;                 // positions 0..kv_len-1 are visible to the last row
     const uint32_t n_tiles = (kv_len + KTILE - 1) / KTILE;
