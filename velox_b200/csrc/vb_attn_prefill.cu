@@ -39,20 +39,20 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <int D>
-__global__ void __launch_bounds__(128)
+template <int D, int PER_SM>
+__global__ void __launch_bounds__(128, PER_SM)
 k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __half* __restrict__ kv_layer,
                const int32_t* __restrict__ table_row, uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens,
-               float scale) {
+               uint32_t bt_shift, float scale) {
     constexpr int ROWB = (D + 8) * 2;            // bytes per staged row
     constexpr int TILEB = KTILE * ROWB;          // one K or V tile
     constexpr int CHUNKS = D / 8;                // 16-byte pieces per row
     extern __shared__ __align__(16) unsigned char smem[];  // [2 buffers][K tile | V tile]
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t h = blockIdx.y, kvh = h / (Hq / Hkv);
-    // the last rows have the most to look at: they start first, so that the short ones fill the tail
-    const uint32_t r0 = (gridDim.x - 1 - blockIdx.x) * QROWS;
+    const uint32_t h = blockIdx.x, kvh = h / (Hq / Hkv);
+    // the last rows have the most to look at: those of all heads start first, so that the short ones fill the tail
+    const uint32_t r0 = (gridDim.y - 1 - blockIdx.y) * QROWS;
     const uint32_t rows_here = min((uint32_t)QROWS, n - r0);
     const uint32_t kv_len = first + r0 + rows_here;                 // positions 0..kv_len-1 are visible to the last row
     const uint32_t n_tiles = (kv_len + KTILE - 1) / KTILE;
@@ -63,13 +63,16 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
     auto stage = [&](uint32_t tile, uint32_t buf) {
         const uint32_t t0 = tile * KTILE;
         const uint32_t dstK = sbase + buf * 2 * TILEB, dstV = dstK + TILEB;
-        for (uint32_t i = threadIdx.x; i < KTILE * CHUNKS; i += 128) {
+#pragma unroll
+        for (uint32_t it = 0; it < KTILE * CHUNKS / 128; ++it) {
+            const uint32_t i = threadIdx.x + it * 128;
             const uint32_t tok = i / CHUNKS, c = i % CHUNKS;
             const uint32_t pos = t0 + tok;
             const bool valid = pos < kv_len;
             const uint32_t p = valid ? pos : 0u;
-            const int32_t blk = table_row[p / block_tokens];
-            const __half* kp = kv_layer + ((((size_t)blk * 2 + 0) * Hkv + kvh) * block_tokens + p % block_tokens) * D + c * 8;
+            const uint32_t bi = bt_shift < 32 ? p >> bt_shift : p / block_tokens;
+            const int32_t blk = table_row[bi];
+            const __half* kp = kv_layer + ((((size_t)blk * 2 + 0) * Hkv + kvh) * block_tokens + (p - bi * block_tokens)) * D + c * 8;
             const __half* vp = kp + (size_t)Hkv * block_tokens * D;
             cp_async16(dstK + tok * ROWB + c * 16, kp, valid);
             cp_async16(dstV + tok * ROWB + c * 16, vp, valid);
@@ -114,10 +117,12 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
         if (t0 <= first + r0 + warp * 16 + 15) {
             float s[KTILE / 8][4];
 #pragma unroll
-            for (int j = 0; j < KTILE / 8; ++j) {
-                s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
+            for (int j = 0; j < KTILE / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
+            // eight chains of products side by side (head dimension outside)
 #pragma unroll
-                for (int kt = 0; kt < D / 16; kt += 2) {
+            for (int kt = 0; kt < D / 16; kt += 2) {
+#pragma unroll
+                for (int j = 0; j < KTILE / 8; ++j) {
                     uint32_t b0, b1, b2, b3;
                     ldsm_x4(sK + (8 * j + (lane & 7)) * ROWB + (16 * kt + 8 * (lane >> 3)) * 2, b0, b1, b2, b3);
                     mma16816(s[j], qa[kt], b0, b1);
@@ -180,19 +185,32 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
     }
 }
 
-template <int D>
-cudaError_t launch_prefill(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
+template <int D, int PER_SM>
+cudaError_t launch_prefill_n(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
                            uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens) {
     constexpr int SMEM = 2 * 2 * KTILE * (D + 8) * 2;
     static bool opted = false;
     if (!opted) {
-        cudaError_t e = cudaFuncSetAttribute(k_attn_prefill<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e == cudaSuccess && PER_SM == 3) e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (e != cudaSuccess) return e;
         opted = true;
     }
     const float scale = 1.0f / sqrtf((float)D);
-    return launch(lc, k_attn_prefill<D>, dim3((n + QROWS - 1) / QROWS, Hq), dim3(128), SMEM, out, q, kv_layer, table_row, first, n, Hq,
-                  Hkv, block_tokens, scale);
+    uint32_t bt_shift = 32;  // block_tokens as a power of two, 32: it is none
+    if ((block_tokens & (block_tokens - 1)) == 0) for (bt_shift = 0; (1u << bt_shift) < block_tokens;) ++bt_shift;
+    return launch(lc, k_attn_prefill<D, PER_SM>, dim3(Hq, (n + QROWS - 1) / QROWS), dim3(128), SMEM, out, q, kv_layer, table_row, first, n, Hq,
+                  Hkv, block_tokens, bt_shift, scale);
+}
+
+// Three blocks per SM (168 registers, the whole shared memory) once there are blocks for more than two: 2.5 us a layer are lost
+// to the other kernels' shared-memory split changing, which short chunks do not get back.  1999 rows, 28 heads of 128: 192 -> 151 us.
+template <int D>
+cudaError_t launch_prefill(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer,
+                           const int32_t* table_row, uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens) {
+    if ((uint64_t)Hq * ((n + QROWS - 1) / QROWS) > 2 * 148)
+        return launch_prefill_n<D, 3>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
+    return launch_prefill_n<D, 1>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
 }
 
 }  // namespace
@@ -202,7 +220,7 @@ bool attention_prefill_supported(uint32_t Hq, uint32_t Hkv, uint32_t D) {
 }
 
 // out/q: [n][Hq*D] fp32 (q with bias and RoPE applied); rows are positions first..first+n-1 of the sequence whose
-// block-table row is `table_row`
+// block-table row is `table_row`.
 cudaError_t attention_prefill(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
                               uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t D, uint32_t block_tokens) {
     if (n == 0) return cudaSuccess;
