@@ -203,7 +203,7 @@ int32_t vb_trace_read(vb_ctx* ctx, uint64_t* out, uint32_t max_records, uint32_t
  *   "attn_mma"       1: tensor-core attention for the fp16 cache; 0: the scalar fp32 path
  *   "fuse_append"    1: bias + RoPE + KV append inside the attention kernel
  *   "prefill_chunk"  prompt tokens that go through the layers together in vb_prefill (16; 1 = token by token)
- *   "prefill_gemm"   1: prompts longer than "prefill_gemm_min" (16 for int4 group-32 and int8 weights, else 48) tokens go
+ *   "prefill_gemm"   1: prompts longer than "prefill_gemm_min" (16 for int4 group-32, 8 for int8 weights, else 48) tokens go
  *                    through the layers in chunks of up to
  *                    "prefill_rows" (2048) tokens whose products run on the tcgen05 tensor cores; 0: batched kernels
  *   "prefill_split"  how those chunk products treat the 11 significant bits of fp16 operands: 2 (default): x and the
@@ -211,8 +211,7 @@ int32_t vb_trace_read(vb_ctx* ctx, uint64_t* out, uint32_t max_records, uint32_t
  *                    to fp32 products to ~2^-22); 1: only x is split; 0: single fp16 operands (fastest; at 32 layers and 2048
  *                    cached rows the rounding moves the logits by up to 2.8e-2).  Set before the first long prefill.
  *   "prefill_flash"  1: those chunks use the causal tile attention kernel (head_dim 64 or 128); 0: one row per token
- *   "prefill_two_per_sm" 1 (default): 128-row tiles run two blocks per SM with half the ring depth each
- *   "prefill_wide"   1: 256 rows of x per tensor-core tile when a chunk has more than 128 rows (default 0)
+ *   "prefill_two_per_sm", "prefill_wide"   accepted, without effect
  *   "decode_gemm"    1: the products of a decode step (lm_head included) run as tensor-core GEMMs, one row of x per
  *                    slot; default 1 when max_batch >= 16 and the weights are int8 per channel or fp16, else 0
  *   "decode_gemm_i8" 1 (default): those products over int8 per-channel weights (batches of up to 32) run on the integer

@@ -67,9 +67,9 @@ def test_canonical_matvec(vb, oracle, fmt, in_dim, out_dim, batch):
 
 
 @pytest.mark.parametrize("fmt,lean", [("q4g32", False), ("q4g32", True), ("i8", False)])
-@pytest.mark.parametrize("n", [17, 33, 34, 65, 66, 129, 140])
+@pytest.mark.parametrize("n", [9, 17, 33, 34, 65, 66, 129, 140])
 def test_prompt_products_from_tensor_memory(fmt, lean, n):
-    """Prompts whose n - 1 chunk rows are the edges of the row tiles (16, 32, 64, 128) and one more, against the CPU checker.
+    """Prompts whose n - 1 chunk rows are the edges of the row tiles (8 of 16, 16, 32, 64, 128) and one more, against the CPU checker.
     K of 1024 (split over a cluster), 384 and 1408 / 1472, 576 QKV rows (half a tile over).  Steps at shrinking positions
     look at the cached rows again, each with few others to dilute it."""
     w, ffn = (L.FMT_Q4G32, 1408) if fmt == "q4g32" else (L.FMT_I8PC, 1472)

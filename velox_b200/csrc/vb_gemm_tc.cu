@@ -447,10 +447,8 @@ bool g_tc_init = false;
 
 }  // namespace
 
-bool gemm_tc_two_per_sm = true;  // vb_set_option("prefill_two_per_sm", 0): one block of twice the ring depth per SM (measured 4 % slower)
 bool gemm_tc_split_k = true;  // vb_set_option("decode_split_k", 0): one block per tile of 128 weight rows
 int gemm_tc_split = 2;  // vb_set_option("prefill_split", n): prefill chunks multiply 0: fp16(x).fp16(W); 1: x as hi + lo; 2: x and W as hi + lo
-bool gemm_tc_wide = false;  // vb_set_option("prefill_wide", 1): 256 rows of x per tile when a chunk has more than 128 (measured slower at 512 rows: fewer blocks than SMs)
 
 template <bool DUAL, int BN, int PER_SM, int XP, int WP>
 static cudaError_t tc_opt_in() {
