@@ -114,3 +114,26 @@ def test_attention_slices(head_dim, group, splits):
         ora.forward_step(5, pos)
         assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
     eng.close()
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("n", [449, 514])
+def test_long_chunk_attention(head_dim, n):
+    """Causal attention of a chunk with blocks for two and for three per SM (40 heads x 7 tiles of 64 rows: 280 blocks, x 9: 360),
+    the last tile full or one row long, against the CPU checker; steps at shrinking positions see the second layer's rows."""
+    spec = LLAMA3_8B_INT4.scaled(name="chunk", d_model=256, n_layers=2, n_q_heads=40, n_kv_heads=4, head_dim=head_dim, ffn_dim=256, vocab=512,
+                                 weight_fmt=L.FMT_F16, head_fmt=L.FMT_F16)
+    eng = H.build_engine(spec, 61, 520)
+    eng.reserve(0, 520)
+    prompt = H.prompt_tokens(spec, 61, n)
+    eng.prefill(prompt)
+    ora, _ = H.build_oracle(spec, 61, 520)
+    for pos, t in enumerate(prompt):
+        ora.forward_step(int(t), pos)
+    assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL
+    for pos in (n - 1, 65, 64, 5, 1):
+        eng.set_state(0, 5, pos)
+        eng.decode(1)
+        ora.forward_step(5, pos)
+        assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
+    eng.close()
