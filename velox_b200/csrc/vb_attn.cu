@@ -975,6 +975,12 @@ static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka) {
     ka.g_chunks = (ka.G + GM - 1) / GM;
     dim3 grid(ka.a.Hkv * ka.g_chunks, ka.n_splits, ka.a.batch);
     const size_t smem = AttnSmem<KVT, EPL, GM, MMA>::total;
+    static std::atomic<uint64_t> opted{0};
+    const cudaError_t oe = once_per_device(opted, [&]() {
+        cudaError_t e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, MMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, MMA>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    });
+    if (oe != cudaSuccess) return oe;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(ATTN_WARPS * 32);
@@ -1039,42 +1045,6 @@ static cudaError_t dispatch_split(const LaunchCfg& lc, const AttnKArgs& ka) {
     case 512: return launch_split<KVT, 16>(lc, ka);
     default: return cudaErrorInvalidValue;
     }
-}
-
-template <typename KVT, int EPL, int GM>
-static cudaError_t opt_in_one() {
-    cudaError_t e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AttnSmem<KVT, EPL, GM, 0>::total);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if constexpr (sizeof(KVT) == 2 && EPL >= 2 && EPL <= 8) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)AttnSmem<KVT, EPL, GM, 1>::total);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if constexpr (EPL == 4) {
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AttnSmem<KVT, EPL, GM, 2>::total);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_split<KVT, EPL, GM, 2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        }
-    }
-    return e;
-}
-template <typename KVT>
-static cudaError_t opt_in_all() {
-    cudaError_t e;
-#define VB_ATTN_OPT(E, G) if ((e = opt_in_one<KVT, E, G>()) != cudaSuccess) return e
-    VB_ATTN_OPT(1, 1); VB_ATTN_OPT(1, 2); VB_ATTN_OPT(1, 4); VB_ATTN_OPT(1, 8);
-    VB_ATTN_OPT(2, 1); VB_ATTN_OPT(2, 2); VB_ATTN_OPT(2, 4); VB_ATTN_OPT(2, 8);
-    VB_ATTN_OPT(4, 1); VB_ATTN_OPT(4, 2); VB_ATTN_OPT(4, 4); VB_ATTN_OPT(4, 8);
-    VB_ATTN_OPT(8, 1); VB_ATTN_OPT(8, 2); VB_ATTN_OPT(8, 4); VB_ATTN_OPT(8, 8); VB_ATTN_OPT(16, 1);
-#undef VB_ATTN_OPT
-    return cudaSuccess;
-}
-cudaError_t attn_init() {
-    cudaError_t e = opt_in_all<__half>();
-    if (e != cudaSuccess) return e;
-    return opt_in_all<float>();
 }
 
 cudaError_t attention_ex(const LaunchCfg& lc, const AttnArgs& a, float scale, size_t kv_batch_stride) {

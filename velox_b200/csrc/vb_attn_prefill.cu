@@ -189,13 +189,13 @@ template <int D, int PER_SM>
 cudaError_t launch_prefill_n(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
                            uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens) {
     constexpr int SMEM = 2 * 2 * KTILE * (D + 8) * 2;
-    static bool opted = false;
-    if (!opted) {
+    static std::atomic<uint64_t> opted{0};
+    const cudaError_t oe = once_per_device(opted, [&]() {
         cudaError_t e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e == cudaSuccess && PER_SM == 3) e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
-        opted = true;
-    }
+        return e;
+    });
+    if (oe != cudaSuccess) return oe;
     const float scale = 1.0f / sqrtf((float)D);
     uint32_t bt_shift = 32;  // block_tokens as a power of two, 32: it is none
     if ((block_tokens & (block_tokens - 1)) == 0) for (bt_shift = 0; (1u << bt_shift) < block_tokens;) ++bt_shift;

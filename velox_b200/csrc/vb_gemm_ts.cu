@@ -495,12 +495,9 @@ EncodeTiledFn ts_encode_fn() {
 template <int FMT, int NT>
 cudaError_t ts_launch(const LaunchCfg& lc, const CUtensorMap& map, TsParams p, uint32_t token_tiles, uint32_t row_tiles) {
     typedef TsShape<FMT, NT> P;
-    static bool opted = false;
-    if (!opted) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_ts<FMT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, P::smem);
-        if (e != cudaSuccess) return e;
-        opted = true;
-    }
+    static std::atomic<uint64_t> opted{0};
+    const cudaError_t oe = once_per_device(opted, [&]() { return cudaFuncSetAttribute(k_gemm_ts<FMT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, P::smem); });
+    if (oe != cudaSuccess) return oe;
     // Split K over a cluster while that shortens the busiest SM's share (the last wave of whole tiles is mostly empty) and every
     // block keeps eight stages.
     const uint32_t tiles = token_tiles * row_tiles, units = p.K / Ts<FMT>::unit;

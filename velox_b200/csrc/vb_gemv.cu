@@ -15,15 +15,11 @@ cudaError_t gemv_fast_init();  // vb_gemv_fast.cu
 
 cudaError_t gemv_init() {
     cudaError_t e;
-    if ((e = gemv_imma_init()) != cudaSuccess || (e = gemv_mma_init()) != cudaSuccess) return e;
+    if ((e = gemv_imma_init()) != cudaSuccess) return e;
     return gemv_fast_init();
 }
 
-cudaError_t kernels_init() {
-    cudaError_t e = gemv_init();
-    if (e != cudaSuccess) return e;
-    return attn_init();
-}
+cudaError_t kernels_init() { return gemv_init(); }
 
 cudaError_t gemv(const LaunchCfg& lc, const GemvArgs& a, int path) {
     if (a.batch == 0 || a.w.rows == 0) return cudaSuccess;

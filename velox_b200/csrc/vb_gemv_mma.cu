@@ -544,6 +544,9 @@ cudaError_t launch_mma(const LaunchCfg& lc, MmArgs a) {
         cfg.numAttrs = 2;
     }
     cfg.attrs = attr;
+    static std::atomic<uint64_t> opted{0};
+    const cudaError_t oe = once_per_device(opted, [&]() { return cudaFuncSetAttribute(k_gemv_mma<FMT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, P::smem); });
+    if (oe != cudaSuccess) return oe;
     if (lc.counter) ++*lc.counter;
     return cudaLaunchKernelEx(&cfg, k_gemv_mma<FMT, T>, a);
 }
@@ -564,21 +567,6 @@ cudaError_t pass_mma(const LaunchCfg& lc, MmArgs a, XfArgs f, unsigned char* ws)
 }
 
 }  // namespace
-
-template <int FMT>
-static cudaError_t opt_in() {
-    cudaError_t e;
-#define VB_OPT_IN(T) if ((e = cudaFuncSetAttribute(k_gemv_mma<FMT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, MmShape<FMT, T>::smem)) != cudaSuccess) return e
-    VB_OPT_IN(1); VB_OPT_IN(2); VB_OPT_IN(4);
-#undef VB_OPT_IN
-    return cudaSuccess;
-}
-cudaError_t gemv_mma_init() {
-    cudaError_t e = opt_in<VB_FMT_Q4G32>();
-    if (e == cudaSuccess) e = opt_in<VB_FMT_Q4G64REF>();
-    if (e == cudaSuccess) e = opt_in<VB_FMT_F16>();
-    return e != cudaSuccess ? e : opt_in<VB_FMT_BF16>();
-}
 
 // fragments of 4 groups of 8 columns and their sums (18 bytes per element of K and group), the rows' scales
 uint64_t gemv_mma_workspace_bytes(uint32_t max_in_dim) { return (uint64_t)max_in_dim * 4 * (16 + 2) + 4096; }

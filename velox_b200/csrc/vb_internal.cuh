@@ -2,6 +2,8 @@
 // the device-side scalar routines (hashing, int4/int8 unpacking) every kernel file uses.
 #pragma once
 
+#include <atomic>
+
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -131,6 +133,19 @@ inline cudaError_t launch(const LaunchCfg& lc, void (*kernel)(KArgs...), dim3 gr
     }
     if (lc.counter) ++*lc.counter;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Kernel attributes are set when a kernel is first launched on a device, not for all kernels of the library when the first context is
+// made: setting one loads the kernel (~15 ms for the variants that no model of the process uses).  `done`: one bit per device.
+template <typename Set>
+inline cudaError_t once_per_device(std::atomic<uint64_t>& done, Set set) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    if ((e = set()) == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
 }
 
 // ---- device scalar helpers --------------------------------------------------------------------------

@@ -9,7 +9,6 @@ const char* last_error();
 // Opt every kernel into the dynamic shared memory it may ask for (once per device, before any capture).
 cudaError_t kernels_init();
 cudaError_t gemv_init();
-cudaError_t attn_init();
 
 // vb_basic.cu
 cudaError_t fill_normal(const LaunchCfg& lc, float* dst, uint64_t n, uint64_t seed, uint64_t stream_id, float mean, float std);
@@ -97,7 +96,6 @@ cudaError_t gemv(const LaunchCfg& lc, const GemvArgs& a, int path);
 // vb_gemv_canon.cu: every format from its canonical layout, fp32 arithmetic
 cudaError_t gemv_canon(const LaunchCfg& lc, const GemvArgs& a);
 // vb_gemv_mma.cu: a few rows of x on mma.sync (int4 tiles, fp16 / bf16 canonical); needs frag_ws
-cudaError_t gemv_mma_init();
 uint64_t gemv_mma_workspace_bytes(uint32_t max_in_dim);
 cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& a, bool* handled);
 
