@@ -180,3 +180,32 @@ def test_mla_runs_of_tiles_that_cross_sequences(vb, heads, lens):
         p = np.exp(s - s.max(axis=1, keepdims=True))
         want = (p / p.sum(axis=1, keepdims=True)) @ cache[b, :n, :DC]
         assert np.max(np.abs(got[b] - want)) <= 2.0 ** -8 * 5, b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("path", [0, 1])
+@pytest.mark.parametrize("split,max_ctx,lens,seen", [(0, 256, [300], [300]), (64, 128, [300, 5, 400], [128, 5, 128]), (128, 130, [600], [256])])
+def test_mla_context_beyond_max_ctx_ends_at_the_last_slice(vb, path, split, max_ctx, lens, seen):
+    """A device-side ctx_len above max_ctx (a replayed graph whose context has outgrown it): both kernels attend up to the end of
+    max_ctx's last slice of split_tokens rows (0: 1024) and read nothing of scratch that no run has written."""
+    from velox_b200.engine import DeviceBuffer as dev
+    lib = vb.load()
+    rng = np.random.default_rng(max_ctx)
+    B, heads, stride, scale = len(lens), 16, 640, 1.0 / np.sqrt(192.0)
+    q = O.bf16_round(rng.standard_normal((B, heads, DC + DR)).astype(np.float32))
+    cache = O.bf16_round(rng.standard_normal((B, stride, DC + DR)).astype(np.float32))
+    d_q, d_cache, d_len = dev.from_numpy(q), dev.from_numpy(O.to_bf16_bits(cache)), dev.from_numpy(np.array(lens, np.uint32))
+    need = lib.vb_op_mla_decode_scratch_bytes(B, heads, max_ctx, split)
+    d_scratch, d_out = dev.from_numpy(np.zeros(need, np.uint8)), dev(B * heads * DC * 4)
+    vb.check(lib.vb_op_mla_set_path(path))
+    try:
+        vb.check(lib.vb_op_mla_decode(d_out.ptr, d_q.ptr, d_cache.ptr, d_len.ptr, B, heads, max_ctx, stride, scale, split, d_scratch.ptr, need, None))
+        vb.check(lib.vb_dev_sync())
+    finally:
+        vb.check(lib.vb_op_mla_set_path(1))
+    got = d_out.to_numpy(np.float32, (B, heads, DC))
+    for b, n in enumerate(seen):
+        s = (q[b] @ cache[b, :n].T) * scale
+        p = np.exp(s - s.max(axis=1, keepdims=True))
+        want = (p / p.sum(axis=1, keepdims=True)) @ cache[b, :n, :DC]
+        assert np.max(np.abs(got[b] - want)) <= 2.0 ** -8 * 5, b

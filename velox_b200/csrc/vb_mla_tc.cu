@@ -157,6 +157,7 @@ struct MlaTcParams {
     uint2* spans;              // [entries] first and last run of an entry
     uint32_t n_seq, n_heads, hbs, q_rows_per_seq;  // hbs: blocks of 128 heads, q_rows_per_seq = hbs * 128
     uint32_t min_tiles;        // of a run
+    uint32_t max_rows;         // rows a sequence counts with at most: the launch and the scratch area are sized for them
     uint32_t direct;           // out takes 32-byte stores: sequences of one piece go straight there
     uint64_t cache_stride;     // rows between sequences
     float scale;
@@ -164,7 +165,9 @@ struct MlaTcParams {
 
 // The deal: entry e = (sequence e / hbs, head block e % hbs) has ceil(ctx / 64) tiles; all tiles in a row, runs of `run` each.
 // Piece of run p in entry e: number p + e (each next piece raises one of the two by one).
-__device__ __forceinline__ uint32_t mla_tiles(const uint32_t* ctx_len, uint32_t e, uint32_t hbs) { return (ctx_len[e / hbs] + MT_T - 1) / MT_T; }
+// A device-side ctx_len beyond max_rows (a captured step whose context has outgrown its max_ctx) ends at max_rows.
+__device__ __forceinline__ uint32_t mla_ctx(const MlaTcParams& p, uint32_t b) { return min(p.ctx_len[b], p.max_rows); }
+__device__ __forceinline__ uint32_t mla_tiles(const MlaTcParams& p, uint32_t e) { return (mla_ctx(p, e / p.hbs) + MT_T - 1) / MT_T; }
 __device__ __forceinline__ uint32_t mla_run(uint32_t total, uint32_t min_tiles) { return max((total + MT_PAIRS - 1) / MT_PAIRS, min_tiles); }
 // sum over the block of one value per thread (every thread gets it); red: one word per warp
 __device__ __forceinline__ uint32_t block_total(uint32_t v, uint32_t* red) {
@@ -208,11 +211,11 @@ k_mla_decode_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // written ctx_len: only q16 has to be waited for) ---------------------------------------------------------------------------------------
     const uint32_t n_entries = p.n_seq * p.hbs;
     uint32_t mine = 0;
-    for (uint32_t e = threadIdx.x; e < n_entries; e += MT_THREADS) mine += mla_tiles(p.ctx_len, e, p.hbs);
+    for (uint32_t e = threadIdx.x; e < n_entries; e += MT_THREADS) mine += mla_tiles(p, e);
     const uint32_t total = block_total(mine, red), run = mla_run(total, p.min_tiles), lo = pair * run;
     for (uint32_t e0 = 0, before = 0; e0 < n_entries && before <= lo; e0 += MT_THREADS) {
         // where the run begins: exclusive scan of 256 entries at a time
-        const uint32_t e = e0 + threadIdx.x, v = e < n_entries ? mla_tiles(p.ctx_len, e, p.hbs) : 0;
+        const uint32_t e = e0 + threadIdx.x, v = e < n_entries ? mla_tiles(p, e) : 0;
         uint32_t incl = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const uint32_t n = __shfl_up_sync(0xFFFFFFFFu, incl, o); if (lane >= (uint32_t)o) incl += n; }
@@ -236,7 +239,7 @@ k_mla_decode_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     uint32_t n = 0, e = s_entry, off = s_off, left = lo < total ? min(run, total - lo) : 0;
     uint32_t pieces = 0;
     for (; left > 0; ++e, off = 0) {
-        const uint32_t b = e / p.hbs, hb = e % p.hbs, ctx = p.ctx_len[b], tiles_e = (ctx + MT_T - 1) / MT_T;
+        const uint32_t b = e / p.hbs, hb = e % p.hbs, ctx = mla_ctx(p, b), tiles_e = (ctx + MT_T - 1) / MT_T;
         const uint32_t nt = min(left, tiles_e - off);
         if (nt == 0) continue;
         left -= nt;
@@ -546,6 +549,14 @@ bool make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint32_t box_
 }  // namespace
 
 static uint32_t mla_min_tiles(uint32_t split_tokens) { return split_tokens ? (split_tokens + MT_T - 1) / MT_T : 4; }
+// Contexts end where the mma.sync kernel's last slice does: max_ctx in whole slices of split_tokens (0: 1024).
+static uint64_t mla_max_rows(uint32_t max_ctx, uint32_t split_tokens) {
+    const uint64_t slice = split_tokens ? split_tokens : 1024;
+    return (max_ctx + slice - 1) / slice * slice;
+}
+static uint64_t mla_total_tiles(uint32_t batch, uint32_t hbs, uint32_t max_ctx, uint32_t split_tokens) {
+    return (uint64_t)batch * hbs * ((mla_max_rows(max_ctx, split_tokens) + MT_T - 1) / MT_T);
+}
 
 uint64_t mla_tc_extra_scratch_bytes(uint32_t batch, uint32_t n_heads) {
     const uint64_t rows = (uint64_t)((n_heads + MT_M - 1) / MT_M) * MT_M;
@@ -554,8 +565,8 @@ uint64_t mla_tc_extra_scratch_bytes(uint32_t batch, uint32_t n_heads) {
 
 // pieces: one per run of tiles and per (sequence, block of heads) at most
 uint64_t mla_tc_partial_bytes(uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens) {
-    const uint64_t entries = (uint64_t)batch * ((n_heads + MT_M - 1) / MT_M), tiles = entries * ((max_ctx + MT_T - 1) / MT_T), m = mla_min_tiles(split_tokens);
-    const uint64_t runs = (tiles + m - 1) / m, slots = (runs < MT_PAIRS ? runs : MT_PAIRS) + entries;
+    const uint32_t hbs = (n_heads + MT_M - 1) / MT_M;
+    const uint64_t entries = (uint64_t)batch * hbs, m = mla_min_tiles(split_tokens), runs = (mla_total_tiles(batch, hbs, max_ctx, split_tokens) + m - 1) / m, slots = (runs < MT_PAIRS ? runs : MT_PAIRS) + entries;
     return slots * (n_heads < (uint32_t)MT_M ? n_heads : (uint32_t)MT_M) * MT_ROW * 4 + 32;
 }
 
@@ -582,7 +593,8 @@ cudaError_t mla_decode_tc(const LaunchCfg& lc, float* out, const float* q, const
     p.min_tiles = mla_min_tiles(split_tokens);
     p.direct = ((uintptr_t)out & 31) == 0 ? 1u : 0u;
     p.cache_stride = cache_stride; p.scale = fmaxf(fabsf(scale), 1e-30f);  // the sign goes into q; 0 would turn masked scores into NaN
-    const uint64_t tiles = (uint64_t)batch * hbs * ((max_ctx + MT_T - 1) / MT_T), runs = (tiles + p.min_tiles - 1) / p.min_tiles;
+    const uint64_t max_rows = mla_max_rows(max_ctx, split_tokens), runs = (mla_total_tiles(batch, hbs, max_ctx, split_tokens) + p.min_tiles - 1) / p.min_tiles;
+    p.max_rows = max_rows < 0xFFFFFFC0ull ? (uint32_t)max_rows : 0xFFFFFFC0u;
     const uint32_t n8 = batch * rows_per_seq * (MT_LAT / 8);
     LaunchCfg chained = lc;  // each of the three starts its prologue while the one before it runs
     chained.pdl = true;
