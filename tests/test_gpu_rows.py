@@ -137,3 +137,44 @@ def test_long_chunk_attention(head_dim, n):
         ora.forward_step(5, pos)
         assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL, pos
     eng.close()
+
+
+def at_offset(dev, a, nbytes):
+    """A device copy of `a` that starts nbytes into its allocation: (buffer, address)."""
+    buf = dev.from_numpy(np.concatenate([np.zeros(nbytes, np.uint8), np.ascontiguousarray(a).view(np.uint8).reshape(-1)]))
+    return buf, buf.ptr.value + nbytes
+
+
+@pytest.mark.parametrize("fmt", ["f32", "f16", "bf16", "q4g32", "q4g64ref", "i8pc"])
+@pytest.mark.parametrize("offset,batch", [(4, 1), (8, 3), (12, 9)])
+def test_canonical_matvec_of_rows_at_any_float(vb, oracle, fmt, offset, batch):
+    """x and dst may start at any float: same bound as above."""
+    from velox_b200.engine import DeviceBuffer as dev
+    c = {"f32": O.FMT_F32, "f16": O.FMT_F16, "bf16": O.FMT_BF16, "q4g32": O.FMT_Q4G32, "q4g64ref": O.FMT_Q4G64REF, "i8pc": O.FMT_I8PC}[fmt]
+    in_dim, out_dim = 576, 37
+    w = oracle.fill_normal(out_dim * in_dim, 6, 1, 0.02).reshape(out_dim, in_dim)
+    data, scales = oracle.quantize(w, c)
+    x = oracle.fill_normal(batch * in_dim, 6, 2, 1.0).reshape(batch, in_dim)
+    dw, ds = dev.from_numpy(data), dev.from_numpy(scales) if scales is not None else None
+    (bx, px), (by, py) = at_offset(dev, x, offset), at_offset(dev, np.zeros((batch, out_dim), np.float32), offset)
+    vb.check(vb.load().vb_op_matmul(py, px, dw.ptr, ds.ptr if ds else None, c, in_dim, out_dim, batch, None))
+    got = by.to_numpy(np.uint8, (offset + batch * out_dim * 4,))[offset:].copy().view(np.float32).reshape(batch, out_dim)
+    exact = x.astype(np.float64) @ oracle.dequantize(data, scales, c, out_dim, in_dim).astype(np.float64).T
+    assert np.max(np.abs(got - exact)) <= in_dim * 2.0 ** -24 * 5 * 0.02 * np.sqrt(in_dim)
+
+
+def test_norm_weights_at_any_float(vb):
+    """The norm and the rows of a fused instruction from pointers that are 4-byte aligned give what aligned ones give (the same sums)."""
+    from velox_b200.engine import DeviceBuffer as dev
+    lib, d, ffn = vb.load(), 512, 1024
+    rng = np.random.default_rng(3)
+    ws = [dev.from_numpy((0.02 * rng.standard_normal(s)).astype(np.float32)) for s in ((d, d), (ffn, d), (ffn, d), (d, ffn))]
+    desc = [L.C.byref(L.Weight(w.ptr, None, L.FMT_F32)) for w in ws]
+    attn, norm, resid = rng.standard_normal(d).astype(np.float32), (1 + 0.1 * rng.standard_normal(d)).astype(np.float32), rng.standard_normal(d).astype(np.float32)
+    scratch, out = dev(ffn * 4), []
+    for off in (0, 4):
+        (ba, pa), (bn, pn), (bh, ph) = at_offset(dev, attn, off), at_offset(dev, norm, off), at_offset(dev, np.zeros(d, np.float32), off)
+        br = dev.from_numpy(resid)
+        vb.check(lib.vb_op_fused_outproj_res_swiglu_res(ph, pa, br.ptr, desc[0], pn, desc[1], desc[2], desc[3], d, d, ffn, 1e-5, scratch.ptr, ffn * 4, None))
+        out.append(bh.to_numpy(np.uint8, (off + d * 4,))[off:].copy().view(np.float32))
+    assert np.array_equal(out[0], out[1])

@@ -143,8 +143,26 @@ __device__ __forceinline__ float warp_reduce_scatter(float (&v)[V], uint32_t lan
     return r;
 }
 
+// ALIGNED: 16-byte loads; else element by element
+template <bool ALIGNED>
+__device__ __forceinline__ float4 load_x4(const float* x) {
+    if constexpr (ALIGNED) return *reinterpret_cast<const float4*>(x);
+    else return make_float4(x[0], x[1], x[2], x[3]);
+}
+template <bool ALIGNED>
 __device__ __forceinline__ void load_norm8(const void* w, int fmt, uint32_t e0, f32x2 (&f)[4]) {
-    if (fmt == VB_FMT_F32) {
+    if constexpr (!ALIGNED) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const uint32_t at = e0 + 2 * i + e;
+                v[e] = fmt == VB_FMT_F16 ? __half2float(((const __half*)w)[at]) : fmt == VB_FMT_BF16 ? __bfloat162float(((const __nv_bfloat16*)w)[at]) : ((const float*)w)[at];
+            }
+            f[i] = pack2(v[0], v[1]);
+        }
+    } else if (fmt == VB_FMT_F32) {
         const float4 a = __ldg(reinterpret_cast<const float4*>((const float*)w + e0)), b = __ldg(reinterpret_cast<const float4*>((const float*)w + e0) + 1);
         f[0] = pack2(a.x, a.y); f[1] = pack2(a.z, a.w); f[2] = pack2(b.x, b.y); f[3] = pack2(b.z, b.w);
     } else {
@@ -154,8 +172,9 @@ __device__ __forceinline__ void load_norm8(const void* w, int fmt, uint32_t e0, 
     }
 }
 
-// grid (blocks of GC_WARPS / ks row groups, passes of NB rows of x), GC_THREADS threads
-template <int FMT, int NB>
+// grid (blocks of GC_WARPS / ks row groups, passes of NB rows of x), GC_THREADS threads.  ALIGNED: x and the norm weights start on
+// 16-byte boundaries (in a context they do; the per-op entry points take any pointer to whole elements)
+template <int FMT, int NB, bool ALIGNED>
 __global__ void __launch_bounds__(GC_THREADS, 2) k_gemv_canon(const CanonArgs a) {
     constexpr int R = GC_R, W = Canon<FMT>::words, D = NB == 1 ? Canon<FMT>::depth : NB == 8 ? Canon<FMT>::depth_8 : Canon<FMT>::depth_rows, V = R * NB;
     constexpr bool PAIRS = !Canon<FMT>::group_scale && NB <= 4;  // accumulate even and odd elements apart (packed FMA all the way)
@@ -247,13 +266,13 @@ __global__ void __launch_bounds__(GC_THREADS, 2) k_gemv_canon(const CanonArgs a)
         if (!last) request(d, d + D, false);
         else if ((uint32_t)(d + D) < ahead_left) request(d, d + D, true);
         f32x2 nw[4];
-        if (a.norm_w && in) load_norm8(a.norm_w, a.norm_fmt, (c0 + d * 32) * 8, nw);
+        if (a.norm_w && in) load_norm8<ALIGNED>(a.norm_w, a.norm_fmt, (c0 + d * 32) * 8, nw);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             // (keeps the compiler from holding the x of several steps, or of all eight rows, in registers at once)
             if (b % 2 == 0) asm volatile("" ::: "memory");
             float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
-            if (in) { u = *reinterpret_cast<const float4*>(xp[b] + d * 256); v = *reinterpret_cast<const float4*>(xp[b] + d * 256 + 4); }
+            if (in) { u = load_x4<ALIGNED>(xp[b] + d * 256); v = load_x4<ALIGNED>(xp[b] + d * 256 + 4); }
             f32x2 x2[4] = {pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w)};
             if (a.norm_w && in) {
 #pragma unroll
@@ -340,18 +359,19 @@ __global__ void __launch_bounds__(GC_THREADS, 2) k_gemv_canon(const CanonArgs a)
     trace_exit(a.trace);
 }
 
-template <int FMT, int NB>
+template <int FMT, int NB, bool ALIGNED>
 cudaError_t launch_canon(const LaunchCfg& lc, const CanonArgs& a) {
     const uint32_t per = a.epilogue == EPI_SWIGLU ? GC_R / 2 : GC_R, groups = (a.rows + per - 1) / per, per_block = GC_WARPS / a.ks;
-    return launch(lc, k_gemv_canon<FMT, NB>, dim3((groups + per_block - 1) / per_block, (a.batch + NB - 1) / NB), dim3(GC_THREADS), 0, a);
+    return launch(lc, k_gemv_canon<FMT, NB, ALIGNED>, dim3((groups + per_block - 1) / per_block, (a.batch + NB - 1) / NB), dim3(GC_THREADS), 0, a);
 }
 template <int FMT>
 cudaError_t launch_canon_fmt(const LaunchCfg& lc, const CanonArgs& a) {
     // rows of x per pass over the weights: 8 hold 64 accumulator registers a lane beside the weights in flight
-    if (a.batch == 1) return launch_canon<FMT, 1>(lc, a);
-    if (a.batch == 2) return launch_canon<FMT, 2>(lc, a);
-    if (a.batch <= 4) return launch_canon<FMT, 4>(lc, a);
-    return launch_canon<FMT, 8>(lc, a);
+    if ((((uintptr_t)a.x | (uintptr_t)a.norm_w) & 15) != 0) return launch_canon<FMT, 1, false>(lc, a);
+    if (a.batch == 1) return launch_canon<FMT, 1, true>(lc, a);
+    if (a.batch == 2) return launch_canon<FMT, 2, true>(lc, a);
+    if (a.batch <= 4) return launch_canon<FMT, 4, true>(lc, a);
+    return launch_canon<FMT, 8, true>(lc, a);
 }
 
 }  // namespace
