@@ -63,3 +63,18 @@ def test_no_device_fails_loudly(vb):
     x = np.zeros(8, dtype=np.float32)
     p = x.ctypes.data_as(C.c_void_p)
     assert lib.vb_op_matmul(p, p, p, None, vb.FMT_F32, 8, 1, 1, None) in (vb.ERR_CUDA, vb.ERR_OOM)
+
+
+def test_no_kernel_attribute_is_set_once_per_process():
+    """A kernel's shared-memory limit is a property of the kernel on ONE device: every opt-in runs for each device (once_per_device, or
+    kernels_init, which every context and entry point calls), and no plain static flag guards an initialisation that several
+    host threads may reach together."""
+    src = os.path.join(ROOT, "velox_b200", "csrc")
+    for name in sorted(os.listdir(src)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(src, name)).read())
+        assert not re.search(r"\bstatic\s+bool\s+\w+\s*=|^bool\s+g_\w*init", text, re.M), name
+        if "cudaFuncSetAttribute" in text and name not in ("vb_gemv_fast.cu", "vb_gemv_imma.cu"):  # (those two: kernels_init)
+            for m in re.finditer("cudaFuncSetAttribute", text):
+                assert "once_per_device(" in text[max(0, m.start() - 400):m.start()], name

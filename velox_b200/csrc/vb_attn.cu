@@ -1078,18 +1078,7 @@ cudaError_t attention_ex(const LaunchCfg& lc, const AttnArgs& a, float scale, si
 cudaError_t attention(const LaunchCfg& lc, const AttnArgs& a) { return attention_ex(lc, a, 0.0f, 0); }
 
 bool attn_make_kv_map(void* map_out, const void* pool, uint64_t rows, uint32_t D) {
-    typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                      const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                      CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
+    const EncodeTiledFn fn = encode_tiled_fn();
     if (!fn || !map_out || !pool || D % 64 != 0 || rows == 0 || rows > 0x7FFFFFFFull || ((uintptr_t)pool & 15) != 0) return false;
     const cuuint64_t dims[2] = {D, rows};
     const cuuint64_t strides[1] = {(cuuint64_t)D * 2};

@@ -485,24 +485,9 @@ k_tile_i8_umma(uint4* __restrict__ dst, const int8_t* __restrict__ src, uint32_t
     dst[tile * 1024 + r * 8 + (c ^ (r & 7))] = v;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn_i8() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
 // int8 [rows][K] row-major, boxes of [box_rows][128 bytes], 128-byte swizzle, zeros outside the matrix
 bool make_map_i8(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t K, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn_i8();
+    EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {K, rows};
     const cuuint64_t strides[1] = {K};
@@ -512,7 +497,6 @@ bool make_map_i8(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t K, uin
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool g_i8_init = false;
 constexpr uint64_t I8_COUNTER_BYTES = 64 * 1024, I8_PART_BYTES = 4 * 1024 * 1024;
 
 }  // namespace
@@ -521,14 +505,12 @@ bool gemm_i8_half_ring = true;  // vb_set_option("i8_half_ring", 0): every block
 bool gemm_i8_tiles = true;  // vb_set_option("i8_tiles", 0): weight tiles by tiled TMA from the canonical matrices instead of the tile-major copies
 bool gemm_i8_enabled = true;  // vb_set_option("decode_gemm_i8", 0): decode batches over int8 weights go through the fp16 copies again
 
-cudaError_t gemm_i8_init() {
-    if (g_i8_init) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_i8<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_gemm_i8<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM);
-    if (e != cudaSuccess) return e;
-    g_i8_init = true;
-    return cudaSuccess;
+static cudaError_t gemm_i8_init() {
+    static std::atomic<uint64_t> opted{0};
+    return once_per_device(opted, []() {
+        const cudaError_t e = cudaFuncSetAttribute(k_gemm_i8<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_gemm_i8<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM);
+    });
 }
 
 bool gemm_i8_supported(const GemvArgs& a) {

@@ -415,25 +415,10 @@ k_weights_to_f16(uint4* __restrict__ dst, uint4* __restrict__ dst_lo, const void
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
 
 // fp16 [rows][K] row-major, boxes of [128 rows][64 columns], 128-byte swizzle, zeros outside the matrix
 bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t K, uint32_t box_rows = BM) {
-    EncodeTiledFn fn = encode_fn();
+    EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {K, rows};
     const cuuint64_t strides[1] = {K * 2};
@@ -443,32 +428,17 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t K, uint32
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool g_tc_init = false;
-
 }  // namespace
 
 bool gemm_tc_split_k = true;  // vb_set_option("decode_split_k", 0): one block per tile of 128 weight rows
 int gemm_tc_split = 2;  // vb_set_option("prefill_split", n): prefill chunks multiply 0: fp16(x).fp16(W); 1: x as hi + lo; 2: x and W as hi + lo
 
 template <bool DUAL, int BN, int PER_SM, int XP, int WP>
-static cudaError_t tc_opt_in() {
-    return cudaFuncSetAttribute(k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_for(PER_SM));
-}
-template <bool DUAL, int BN, int PER_SM, int XP, int WP>
 static cudaError_t tc_launch(const LaunchCfg& lc, const dim3& grid, const CUtensorMap* m, const GemmParams& p) {
+    static std::atomic<uint64_t> opted{0};
+    const cudaError_t e = once_per_device(opted, []() { return cudaFuncSetAttribute(k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_for(PER_SM)); });
+    if (e != cudaSuccess) return e;
     return launch(lc, k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, grid, dim3(128), smem_bytes_for(PER_SM), m[0], m[1], m[2], m[3], m[4], p);
-}
-
-cudaError_t gemm_tc_init() {
-    if (g_tc_init) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-#define VB_TC(...) if ((e = tc_opt_in<__VA_ARGS__>()) != cudaSuccess) return e
-    VB_TC(false, 32, 1, 1, 1); VB_TC(true, 32, 1, 1, 1);
-    VB_TC(false, 128, 2, 1, 1); VB_TC(false, 128, 2, 2, 1); VB_TC(false, 128, 1, 2, 2);
-    VB_TC(true, 128, 2, 1, 1); VB_TC(true, 128, 1, 2, 1); VB_TC(true, 128, 1, 2, 2);
-#undef VB_TC
-    g_tc_init = true;
-    return cudaSuccess;
 }
 
 // fp16 [rows][cols] copy of a weight matrix (int8 per channel: the integers; the row scale stays with the caller)
@@ -511,8 +481,7 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
     const uint32_t K = a.w.cols, out_dim = a.w.rows, n_rows = a.batch;
     if (n_rows == 0) return cudaSuccess;
     if (gemm_tc_workspace_bytes(out_dim, K, n_rows, dual) > workspace_bytes || ((uintptr_t)workspace & 1023) != 0) return cudaErrorInvalidValue;
-    cudaError_t e = gemm_tc_init();
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     const uint64_t rows_pad = gemm_tc_rows_padded(n_rows);
     const uint64_t xb = (rows_pad * K * 2 + 1023) / 1024 * 1024, wb = ((uint64_t)out_dim * K * 2 + 1023) / 1024 * 1024;
     const bool narrow = n_rows <= 32;  // decode batches: 32 rows of x per tile, no tensor-core work on padding

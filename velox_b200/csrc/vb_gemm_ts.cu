@@ -477,20 +477,6 @@ __global__ void __launch_bounds__(512) k_rows_split(__half* __restrict__ hi, __h
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn ts_encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* q = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &res) == cudaSuccess && res == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(q);
-    }
-    return fn;
-}
 
 template <int FMT, int NT>
 cudaError_t ts_launch(const LaunchCfg& lc, const CUtensorMap& map, TsParams p, uint32_t token_tiles, uint32_t row_tiles) {
@@ -554,7 +540,7 @@ uint64_t gemm_ts_workspace_bytes(uint32_t in_dim, uint32_t n_rows) {
 }
 
 cudaError_t gemm_ts(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uint64_t workspace_bytes) {
-    if (!gemm_ts_supported(a) || !ts_encode_fn()) return cudaErrorInvalidValue;
+    if (!gemm_ts_supported(a) || !encode_tiled_fn()) return cudaErrorInvalidValue;
     const uint32_t K = a.w.cols, n_rows = a.batch;
     if (n_rows == 0) return cudaSuccess;
     if (gemm_ts_workspace_bytes(K, n_rows) > workspace_bytes || ((uintptr_t)workspace & 15) != 0) return cudaErrorInvalidValue;
@@ -573,7 +559,7 @@ cudaError_t gemm_ts(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
     const cuuint64_t dims[2] = {K, 2ull * pad};
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
     const cuuint32_t box[2] = {64, nt}, estr[2] = {1, 1};
-    if (ts_encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, hi, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    if (encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, hi, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorNotSupported;
     TsParams p = {};

@@ -128,7 +128,6 @@ extern bool imma_spread;
 
 // vb_gemm_tc.cu: multi-row products on the tcgen05 tensor cores (prefill chunks); the arguments are those of gemv(),
 // `batch` = rows of x; the workspace holds the fp16 operands
-cudaError_t gemm_tc_init();
 extern bool gemm_tc_split_k;
 uint64_t gemm_tc_operand_bytes(uint32_t out_dim, uint32_t in_dim, uint32_t n_rows, bool dual);
 uint64_t gemm_tc_workspace_zero_bytes();  // leading bytes of the workspace that must be zero before the first call

@@ -398,11 +398,8 @@ int32_t vb_op_mla_decode(float* out, const float* q, const void* latent_cache, c
         return VB_OK;
     }
     if (split_tokens == 0) split_tokens = 1024;
-    static bool opted = false;
-    if (!opted) {
-        VB_CUDA(cudaFuncSetAttribute(k_mla_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ML_SMEM));
-        opted = true;
-    }
+    static std::atomic<uint64_t> opted{0};
+    VB_CUDA(once_per_device(opted, []() { return cudaFuncSetAttribute(k_mla_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ML_SMEM); }));
     MlaArgs a;
     a.q = q; a.cache = (const __nv_bfloat16*)latent_cache; a.ctx_len = ctx_len; a.partial = (float*)scratch;
     a.n_heads = n_heads; a.split_tokens = split_tokens; a.n_splits = (max_ctx + split_tokens - 1) / split_tokens;
@@ -430,12 +427,11 @@ int32_t vb_op_mla_head_product(float* dst, const float* src, const void* w_bf16,
     lc.stream = (cudaStream_t)stream;
     // whole 16s and 16-byte rows: the tensor-core kernel
     if (n_in % 16 == 0 && n_out % 16 == 0 && (((uintptr_t)src | (uintptr_t)w_bf16) & 15) == 0) {
-        static bool opted_hp = false;
-        if (!opted_hp) {
-            VB_CUDA(cudaFuncSetAttribute(k_mla_head_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(true)));
-            VB_CUDA(cudaFuncSetAttribute(k_mla_head_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(false)));
-            opted_hp = true;
-        }
+        static std::atomic<uint64_t> opted_hp{0};
+        VB_CUDA(once_per_device(opted_hp, []() {
+            const cudaError_t e = cudaFuncSetAttribute(k_mla_head_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(true));
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(k_mla_head_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, hp_smem_bytes(false));
+        }));
         const dim3 g3(n_heads, (n_out + HP_O - 1) / HP_O, (batch + HP_B - 1) / HP_B);
         if (w_rows_are_out) VB_CUDA(launch(lc, k_mla_head_mma<true>, g3, dim3(HP_THREADS), hp_smem_bytes(true), dst, src, (const __nv_bfloat16*)w_bf16, n_heads, n_in, n_out, batch));
         else VB_CUDA(launch(lc, k_mla_head_mma<false>, g3, dim3(HP_THREADS), hp_smem_bytes(false), dst, src, (const __nv_bfloat16*)w_bf16, n_heads, n_in, n_out, batch));

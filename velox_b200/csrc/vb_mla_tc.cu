@@ -519,24 +519,9 @@ k_mla_q_bf16(uint4* __restrict__ dst, const float* __restrict__ q, uint32_t n_he
     dst[i] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn_mla() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-    return fn;
-}
 // bf16 [rows][576] row-major, boxes of [box_rows][64 columns], 128-byte swizzle, zeros outside the matrix
 bool make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn_mla();
+    EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {MT_LAT, rows};
     const cuuint64_t strides[1] = {MT_LAT * 2};
@@ -573,12 +558,9 @@ uint64_t mla_tc_partial_bytes(uint32_t batch, uint32_t n_heads, uint32_t max_ctx
 // extra: the area of mla_tc_extra_scratch_bytes (16-byte aligned): a status word, then Q in bf16, then the entries' spans
 cudaError_t mla_decode_tc(const LaunchCfg& lc, float* out, const float* q, const void* cache, const uint32_t* ctx_len, float* partial, void* extra,
                           uint32_t batch, uint32_t n_heads, uint32_t max_ctx, uint32_t split_tokens, uint64_t cache_stride, float scale) {
-    static bool opted = false;
-    cudaError_t e;
-    if (!opted) {
-        if ((e = cudaFuncSetAttribute(k_mla_decode_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM)) != cudaSuccess) return e;
-        opted = true;
-    }
+    static std::atomic<uint64_t> opted{0};
+    cudaError_t e = once_per_device(opted, []() { return cudaFuncSetAttribute(k_mla_decode_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM); });
+    if (e != cudaSuccess) return e;
     const uint32_t hbs = (n_heads + MT_M - 1) / MT_M, rows_per_seq = hbs * MT_M;
     uint32_t* status = reinterpret_cast<uint32_t*>(extra);
     __nv_bfloat16* q16 = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(extra) + 1024);
