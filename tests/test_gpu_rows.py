@@ -178,3 +178,10 @@ def test_norm_weights_at_any_float(vb):
         vb.check(lib.vb_op_fused_outproj_res_swiglu_res(ph, pa, br.ptr, desc[0], pn, desc[1], desc[2], desc[3], d, d, ffn, 1e-5, scratch.ptr, ffn * 4, None))
         out.append(bh.to_numpy(np.uint8, (off + d * 4,))[off:].copy().view(np.float32))
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("fmt", ["f32", "f16", "bf16", "q4g32", "q4g64ref", "i8pc"])
+@pytest.mark.parametrize("in_dim,out_dim,batch", [(64, 9, 20), (576, 37, 7), (1088, 130, 17), (576, 4099, 8), (576, 4099, 9), (576, 4099, 13)])
+def test_canonical_matvec_passes(vb, oracle, fmt, in_dim, out_dim, batch):
+    """Rows of x in passes of two (all of them one wave of warps), four, and for fp32 eight; full and ragged last passes."""
+    test_canonical_matvec(vb, oracle, fmt, in_dim, out_dim, batch)

@@ -6,7 +6,7 @@
 // chain of launches: what every kernel does between the end of its predecessor and its own first store.
 //  * A warp owns four rows of W (two of gate and two of up for SwiGLU) and walks along K, 8 consecutive elements a lane
 //    and step: one x value loaded serves four weights, and x (L1-resident after its first touch) needs no staging
-//    through shared memory and no barrier.  Up to eight rows of x share the pass over the weights.
+//    through shared memory and no barrier.  Several rows of x share the pass over the weights (launch_canon_fmt).
 //  * The loads of the next DEPTH steps are in registers or in flight: 128..192 bytes a thread, 64..98 KB an SM at 16
 //    warps, what HBM's latency at 44 GB/s an SM asks for.  The first DEPTH steps are requested BEFORE the
 //    grid-dependency wait (weights never depend on the kernel before), so at the size of a 135M model the whole
@@ -26,16 +26,17 @@ namespace {
 constexpr int GC_R = 4;        // rows of W per warp
 constexpr int GC_WARPS = 8;    // per block
 constexpr int GC_THREADS = GC_WARPS * 32;
+constexpr uint32_t GC_WAVE = 148 * 16;  // warps the chip holds
 
-// words: 32-bit words of 8 consecutive elements; depth: steps requested ahead (fewer where the accumulators of several
-// rows of x take the registers)
+// words: 32-bit words of 8 consecutive elements; depth: steps requested ahead (depth_rows: where the accumulators of several rows
+// of x take the registers)
 template <int FMT> struct Canon;
-template <> struct Canon<VB_FMT_F32> { static constexpr int words = 8, depth = 1, depth_rows = 1, depth_8 = 1; static constexpr bool group_scale = false; };
-template <> struct Canon<VB_FMT_F16> { static constexpr int words = 4, depth = 3, depth_rows = 1, depth_8 = 1; static constexpr bool group_scale = false; };
-template <> struct Canon<VB_FMT_BF16> { static constexpr int words = 4, depth = 3, depth_rows = 1, depth_8 = 1; static constexpr bool group_scale = false; };
-template <> struct Canon<VB_FMT_I8PC> { static constexpr int words = 2, depth = 4, depth_rows = 2, depth_8 = 2; static constexpr bool group_scale = false; };
-template <> struct Canon<VB_FMT_Q4G32> { static constexpr int words = 1, depth = 4, depth_rows = 2, depth_8 = 1; static constexpr bool group_scale = true; };
-template <> struct Canon<VB_FMT_Q4G64REF> { static constexpr int words = 1, depth = 4, depth_rows = 2, depth_8 = 1; static constexpr bool group_scale = true; };
+template <> struct Canon<VB_FMT_F32> { static constexpr int words = 8, depth = 1, depth_rows = 1; static constexpr bool group_scale = false; };
+template <> struct Canon<VB_FMT_F16> { static constexpr int words = 4, depth = 3, depth_rows = 1; static constexpr bool group_scale = false; };
+template <> struct Canon<VB_FMT_BF16> { static constexpr int words = 4, depth = 3, depth_rows = 1; static constexpr bool group_scale = false; };
+template <> struct Canon<VB_FMT_I8PC> { static constexpr int words = 2, depth = 4, depth_rows = 2; static constexpr bool group_scale = false; };
+template <> struct Canon<VB_FMT_Q4G32> { static constexpr int words = 1, depth = 4, depth_rows = 2; static constexpr bool group_scale = true; };
+template <> struct Canon<VB_FMT_Q4G64REF> { static constexpr int words = 1, depth = 4, depth_rows = 2; static constexpr bool group_scale = true; };
 
 struct CanonArgs {
     const void *w, *scales, *w2, *scales2;  // w2: the up matrix of SwiGLU
@@ -176,7 +177,7 @@ __device__ __forceinline__ void load_norm8(const void* w, int fmt, uint32_t e0, 
 // 16-byte boundaries (in a context they do; the per-op entry points take any pointer to whole elements)
 template <int FMT, int NB, bool ALIGNED>
 __global__ void __launch_bounds__(GC_THREADS, 2) k_gemv_canon(const CanonArgs a) {
-    constexpr int R = GC_R, W = Canon<FMT>::words, D = NB == 1 ? Canon<FMT>::depth : NB == 8 ? Canon<FMT>::depth_8 : Canon<FMT>::depth_rows, V = R * NB;
+    constexpr int R = GC_R, W = Canon<FMT>::words, D = NB == 1 ? Canon<FMT>::depth : Canon<FMT>::depth_rows, V = R * NB;
     constexpr bool PAIRS = !Canon<FMT>::group_scale && NB <= 4;  // accumulate even and odd elements apart (packed FMA all the way)
     constexpr bool GS = Canon<FMT>::group_scale;
     __shared__ float part[GC_WARPS][V];
@@ -364,14 +365,20 @@ cudaError_t launch_canon(const LaunchCfg& lc, const CanonArgs& a) {
     const uint32_t per = a.epilogue == EPI_SWIGLU ? GC_R / 2 : GC_R, groups = (a.rows + per - 1) / per, per_block = GC_WARPS / a.ks;
     return launch(lc, k_gemv_canon<FMT, NB, ALIGNED>, dim3((groups + per_block - 1) / per_block, (a.batch + NB - 1) / NB), dim3(GC_THREADS), 0, a);
 }
+// Rows of x per pass over the weights.  A matrix whose passes all run at once as one wave of warps gives each the fewest rows: what
+// the pass takes is its own latency, and the weights come from L2.  Else four rows to a pass: eight share the weights further but
+// hold 64 accumulator registers and spill (fp16 28672 x 4096, 16 rows: 252 us in eights, 248 in fours), which only fp32 with its
+// eight-byte pairs wins back, where the last pass is more than half full (8 rows 199 / 224 us, 12 rows 363 / 327, 16 rows 370 /
+// 429).  One step of the 135M shape, 5 / 9 / 15 / 32 rows, ms: fp32 1.38 / 1.73 / 1.69 / 2.22 with eights throughout, now
+// 0.91 / 1.14 / 1.36 / 2.11; q4 group-64 1.23 / 1.66 / 2.46 / 3.93, now 0.80 / 0.98 / 1.18 / 2.05.
 template <int FMT>
-cudaError_t launch_canon_fmt(const LaunchCfg& lc, const CanonArgs& a) {
-    // rows of x per pass over the weights: 8 hold 64 accumulator registers a lane beside the weights in flight
+cudaError_t launch_canon_fmt(const LaunchCfg& lc, const CanonArgs& a, uint32_t warps) {
     if ((((uintptr_t)a.x | (uintptr_t)a.norm_w) & 15) != 0) return launch_canon<FMT, 1, false>(lc, a);
     if (a.batch == 1) return launch_canon<FMT, 1, true>(lc, a);
-    if (a.batch == 2) return launch_canon<FMT, 2, true>(lc, a);
-    if (a.batch <= 4) return launch_canon<FMT, 4, true>(lc, a);
-    return launch_canon<FMT, 8, true>(lc, a);
+    if (a.batch == 2 || warps * ((a.batch + 1) / 2) <= GC_WAVE) return launch_canon<FMT, 2, true>(lc, a);
+    if constexpr (FMT == VB_FMT_F32)
+        if ((a.batch - 1) % 8 >= 4 && warps * ((a.batch + 3) / 4) > GC_WAVE) return launch_canon<FMT, 8, true>(lc, a);
+    return launch_canon<FMT, 4, true>(lc, a);
 }
 
 }  // namespace
@@ -384,18 +391,18 @@ cudaError_t gemv_canon(const LaunchCfg& lc, const GemvArgs& g) {
     a.norm_w = g.norm_w; a.norm_fmt = g.norm_fmt; a.eps = g.eps; a.state = g.state;
     a.batch = g.batch; a.dst_stride = g.dst_stride ? g.dst_stride : g.w.rows; a.dst_offset = g.dst_offset;
     a.epilogue = g.epilogue; a.trace = g.trace;
-    // Share K among warps until the row groups make several waves of the ~2400 warps the chip holds (the last wave is
+    // Share K among warps until the row groups make several waves of the warps the chip holds (the last wave is
     // then a small part), as long as every warp keeps four steps; below one wave, down to a single step each.
-    const uint32_t per = g.epilogue == EPI_SWIGLU ? GC_R / 2 : GC_R, groups = (a.rows + per - 1) / per, n8 = a.K / 8, wave = 148 * 16;
+    const uint32_t per = g.epilogue == EPI_SWIGLU ? GC_R / 2 : GC_R, groups = (a.rows + per - 1) / per, n8 = a.K / 8;
     a.ks = 1;
-    while (a.ks < GC_WARPS && ((groups * a.ks < 6 * wave && n8 >= 32 * 4 * 2 * a.ks) || (groups * a.ks < wave && n8 >= 32 * 2 * a.ks))) a.ks *= 2;
+    while (a.ks < GC_WARPS && ((groups * a.ks < 6 * GC_WAVE && n8 >= 32 * 4 * 2 * a.ks) || (groups * a.ks < GC_WAVE && n8 >= 32 * 2 * a.ks))) a.ks *= 2;
     switch (g.w.fmt) {
-    case VB_FMT_F32: return launch_canon_fmt<VB_FMT_F32>(lc, a);
-    case VB_FMT_F16: return launch_canon_fmt<VB_FMT_F16>(lc, a);
-    case VB_FMT_BF16: return launch_canon_fmt<VB_FMT_BF16>(lc, a);
-    case VB_FMT_Q4G32: return launch_canon_fmt<VB_FMT_Q4G32>(lc, a);
-    case VB_FMT_Q4G64REF: return launch_canon_fmt<VB_FMT_Q4G64REF>(lc, a);
-    case VB_FMT_I8PC: return launch_canon_fmt<VB_FMT_I8PC>(lc, a);
+    case VB_FMT_F32: return launch_canon_fmt<VB_FMT_F32>(lc, a, groups * a.ks);
+    case VB_FMT_F16: return launch_canon_fmt<VB_FMT_F16>(lc, a, groups * a.ks);
+    case VB_FMT_BF16: return launch_canon_fmt<VB_FMT_BF16>(lc, a, groups * a.ks);
+    case VB_FMT_Q4G32: return launch_canon_fmt<VB_FMT_Q4G32>(lc, a, groups * a.ks);
+    case VB_FMT_Q4G64REF: return launch_canon_fmt<VB_FMT_Q4G64REF>(lc, a, groups * a.ks);
+    case VB_FMT_I8PC: return launch_canon_fmt<VB_FMT_I8PC>(lc, a, groups * a.ks);
     default: return cudaErrorInvalidValue;
     }
 }

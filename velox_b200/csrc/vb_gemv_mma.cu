@@ -585,10 +585,15 @@ cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& g, bool* handled) {
         const uint32_t tiles = (swiglu ? 2 : 1) * g.w.rows / 16, places = 2 * 148, rounds = (tiles + places - 1) / places;
         if (g.batch <= 4 && K <= 8192 && tiles * 4 >= rounds * places * 3) return cudaSuccess;
     } else {
-        // The fp32 kernel needs one launch and no conversion: ahead on small matrices (135M model, group-64, one row: 2.8 against
-        // 6.4 us) and with one or two rows of 16-bit weights (it streams those at 5..6 TB/s).
+        // The fp32 kernel needs one launch and no conversion, and takes small matrices in one wave: ahead there, and with one or two
+        // rows of 16-bit weights (it streams those at 5..6 TB/s).  Where the line lies (decode steps of models of 768 to 2048
+        // columns, products from the named size on taken here, us; 16-bit / group-64):
+        //   3 rows: 1024 columns from 1M weights 521 / 589, 4M 415 / 420, 10M 457 / 451; 2048 columns 4M 553 / 529, 10M 592 / 560
+        //   8 rows, one pass of 16-bit: 1024 columns 839 / 1142, 592 / 692, 664 / 680; 2048 columns 884 / 1007, 923 / 960
+        //   32 rows: 1024 columns 3062 / 4353, 1760 / 2092, 1814 / 1946; 1536 columns 2165 / 2650 from 4M, 1957 / 2411 from 10M
         if (!q4 && g.batch < 3) return cudaSuccess;
-        if (weights * g.batch < 8000000ull) return cudaSuccess;
+        const uint32_t one_pass = q4 ? 4 : 8;
+        if (weights < (g.batch > 1 && g.batch <= one_pass ? 4000000ull : 8000000ull)) return cudaSuccess;
     }
     MmArgs a;
     if (q4) {
