@@ -579,11 +579,13 @@ cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& g, bool* handled) {
     const uint64_t weights = (uint64_t)g.w.rows * K * (swiglu ? 2 : 1);
     if (g.w.fmt == VB_FMT_Q4G32) {
         // One row: the integer kernel stages x itself and needs one launch.  2..4 rows are one pass of its multi-row flavour too,
-        // faster (8B shape: O 6.2 against 8.2 us, gate/up 17.5 / 22.9, head 55 / 64) unless its tiles fill the last round of
-        // SMs badly (QKV: 384 tiles on 296 places, 14.7 / 10.4) or four rows of x are long to stage (down: 19.7 / 15.8).
+        // faster (8B shape: O 6.2 against 8.2 us, gate/up 17.5 / 22.9, head 55 / 64) unless four rows of x are long to stage
+        // (down: 19.7 / 15.8) or the tiles of a large matrix fill the last of several rounds of SMs badly (QKV: 384 tiles on 296
+        // places, 14.7 / 10.4).  Below 8M weights, or in a single round, its one launch is ahead however the tiles fall (models of
+        // 1024 / 1536 / 2048 columns, a step of 2 rows: 387 / 391 / 297 us, by the fill alone 509 / 426 / 334).
         if (g.batch < 2) return cudaSuccess;
         const uint32_t tiles = (swiglu ? 2 : 1) * g.w.rows / 16, places = 2 * 148, rounds = (tiles + places - 1) / places;
-        if (g.batch <= 4 && K <= 8192 && tiles * 4 >= rounds * places * 3) return cudaSuccess;
+        if (g.batch <= 4 && K <= 8192 && (rounds == 1 || weights < 8000000ull || tiles * 4 >= rounds * places * 3)) return cudaSuccess;
     } else {
         // The fp32 kernel needs one launch and no conversion, and takes small matrices in one wave: ahead there, and with one or two
         // rows of 16-bit weights (it streams those at 5..6 TB/s).  Where the line lies (decode steps of models of 768 to 2048
