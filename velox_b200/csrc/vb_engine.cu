@@ -287,7 +287,8 @@ int32_t ensure_tc_ws(vb_ctx* c, uint32_t rows, bool with_head) {
     need = std::max(need, gemm_tc_workspace_bytes(dm, c->ffn, rows, false));
     if (with_head) need = std::max(need, gemm_tc_workspace_bytes(c->vocab, dm, rows, false));
     if (c->tc_ws_bytes >= need) return VB_OK;
-    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }  // a captured step holds the old address
+    // a step captured with these products holds the old address (a prompt's workspace alone is in no captured step)
+    if (c->graph_exec && c->decode_gemm) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
     if (c->tc_ws) cudaFree(c->tc_ws);
     c->tc_ws = nullptr; c->tc_ws_bytes = 0;
     if (cudaMalloc(&c->tc_ws, need + 1024) != cudaSuccess) {  // + 1024: the swizzled operands start on a 1024-byte boundary
