@@ -1,8 +1,11 @@
 """Device memory around prompts and weights: what is allocated when, and what happens when the card is nearly full."""
+import numpy as np
 import pytest
+import torch
 
 import helpers as H
 from velox_b200 import lib as L
+from velox_b200.engine import Engine
 from velox_b200.modelspec import LLAMA3_8B_INT4
 
 pytestmark = pytest.mark.gpu
@@ -11,6 +14,23 @@ pytestmark = pytest.mark.gpu
 def spec_of(fmt, **kw):
     base = dict(name="ws", d_model=512, n_layers=2, n_q_heads=8, n_kv_heads=2, head_dim=64, ffn_dim=1408, vocab=1024, weight_fmt=fmt, head_fmt=fmt)
     return LLAMA3_8B_INT4.scaled(**{**base, **kw})
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("fmt", [L.FMT_Q4G32, L.FMT_I8PC, L.FMT_F16])
+def test_prompts_of_growing_length_allocate_twice_at_most(fmt):
+    eng = H.build_engine(spec_of(fmt), 71, 2048)
+    eng.reserve(0, 2048)
+    seen = set()
+    for n in (20, 60, 130, 300, 520, 700, 1100, 2000):
+        eng.prefill(H.prompt_tokens(eng.spec, 71, n))
+        seen.add(free_bytes())
+    eng.close()
+    assert len(seen) <= 2
 
 
 def test_long_prompt_keeps_the_captured_step():
@@ -38,3 +58,24 @@ def test_long_prompt_keeps_the_captured_step():
     finally:
         other.set_option("gemv_multirow", 1)
     eng.close(), other.close()
+
+
+def test_prompt_in_a_nearly_full_card():
+    """A lean context whose chunk buffers do not fit takes shorter chunks: the logits of the roomy run up to the rounding of other
+    row tiles (2^-11 of the fp16 cache)."""
+    spec = spec_of(L.FMT_Q4G32, d_model=2048, n_q_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=8192)
+    prompt = H.prompt_tokens(spec, 73, 4000)
+    got = []
+    for left in (None, 300 << 20):  # the buffers of 4096 rows: 34 + 50 + 34 + 34 + 134 MB and 134 MB of parts
+        eng = Engine(spec, max_seq_len=4096, lean_weights=True)
+        eng.load_synthetic(73)
+        eng.set_option("prefill_rows", 4096)
+        eng.reserve(0, 4096)
+        eng.prefill(prompt[:17])
+        hog = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda") if left else None
+        eng.prefill(prompt)
+        got.append(eng.logits())
+        eng.close()
+        del hog
+        torch.cuda.empty_cache()
+    assert np.max(np.abs(got[0] - got[1])) <= 1e-2
