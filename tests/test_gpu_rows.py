@@ -7,7 +7,7 @@ import helpers as H
 from oracle import oracle as O
 from velox_b200 import lib as L
 from velox_b200.engine import Engine
-from velox_b200.modelspec import LLAMA3_8B_INT4
+from velox_b200.modelspec import LLAMA3_8B_INT4, ModelSpec
 
 pytestmark = pytest.mark.gpu
 
@@ -185,3 +185,34 @@ def test_norm_weights_at_any_float(vb):
 def test_canonical_matvec_passes(vb, oracle, fmt, in_dim, out_dim, batch):
     """Rows of x in passes of two (all of them one wave of warps), four, and for fp32 eight; full and ragged last passes."""
     test_canonical_matvec(vb, oracle, fmt, in_dim, out_dim, batch)
+
+
+class LargeOutput(ModelSpec):
+    """The output projections a million times larger: their group scales lie around 1e4, and the last row's logits hang on what the
+    second layer's attention finds in the rows before it."""
+
+    def tensors(self):
+        return [(r, l, rows, cols, mean, std * 1.5e6 if r == L.ROLE_WO else std) for r, l, rows, cols, mean, std in super().tensors()]
+
+
+@pytest.mark.parametrize("lean", [False, True])
+@pytest.mark.parametrize("n", [12, 30, 70])
+def test_prompts_over_int4_scales_beyond_fp16_products(lean, n):
+    """(n - 8) * scale beyond 65504: prompts of every route against the CPU checker; a matrix reloaded within range takes the route
+    of its new values."""
+    base = dict(LLAMA3_8B_INT4.__dict__, name="scales", d_model=512, n_layers=2, n_q_heads=8, n_kv_heads=2, head_dim=64, ffn_dim=1408, vocab=1024)
+    for spec in (LargeOutput(**base), ModelSpec(**base)):
+        if isinstance(spec, LargeOutput):
+            eng = Engine(spec, max_seq_len=96, lean_weights=lean)
+            eng.reserve(0, 96)
+        eng.spec = spec
+        eng.load_synthetic(81)
+        prompt = H.prompt_tokens(spec, 81, n)
+        eng.prefill(prompt)
+        ora, stored = H.build_oracle(spec, 81, 96)
+        scales = stored[(L.ROLE_WO, 0)][1].view(np.float16)
+        assert (float(np.abs(scales).max()) > 8188) == isinstance(spec, LargeOutput)
+        for pos, t in enumerate(prompt):
+            ora.forward_step(int(t), pos)
+        assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL
+    eng.close()

@@ -14,6 +14,7 @@ constexpr uint32_t RING_SLOTS = 1024;  // VELOX_HOST_RING_SLOTS (src/codegen.rs:
 struct Tensor {
     WMat m;
     bool loaded = false;
+    bool beyond_f16 = false;  // int4 group-32: some (n - 8) * scale is none that fp16 holds
 };
 
 }  // namespace vb

@@ -250,6 +250,13 @@ bool tc_products_ok(vb_ctx* c) {
 // the packed weights, so they win while the weights are what takes time, and they are the only ones a lean context can run.
 // Four layers of the 8B int4 shape and a last token, ms: 64 rows 1.23 (fp16 copies: 1.58; sixteen rows at a time: 3.3), 128
 // rows 1.55 (1.69), 160 rows 2.37 (2.00); the 7B int8 shape: 64 rows 1.23 (1.85), 128 1.28 (1.95), 200 2.07 (2.19), 256 2.12 (2.22).
+// Both make fp16 operands of the weights, so int4 matrices with a scale beyond 8188 (8 * 8188 = 65504) stay with the kernels that
+// apply the scales in fp32.
+bool weights_within_f16(const vb_ctx* c) {
+    for (const Tensor& t : c->t)
+        if (t.beyond_f16) return false;
+    return true;
+}
 uint32_t ts_rows_max(const vb_ctx* c) { return c->d.weight_fmt == VB_FMT_I8PC ? 256 : 128; }
 bool ts_products_ok(vb_ctx* c) {
     if (gemm_tc_split != 2) return false;  // fewer parts: the products of vb_gemm_tc.cu
@@ -690,7 +697,7 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
     VB_CREATE_CUDA(cudaMemsetAsync(c->state, 0, d.max_batch * sizeof(SeqState), c->stream));
     VB_CREATE_CUDA(cudaMemsetAsync(c->pf_state, 0, d.max_batch * sizeof(SeqState), c->stream));
     c->state_host.assign(d.max_batch, SeqState{0, 0, 0, 0});
-    VB_CREATE_CUDA(cudaHostAlloc((void**)&c->ring_host, (size_t)d.max_batch * RING_SLOTS * 4, cudaHostAllocMapped));
+    VB_CREATE_CUDA(cudaHostAlloc((void**)&c->ring_host, (size_t)d.max_batch * RING_SLOTS * 4 + 4, cudaHostAllocMapped));  // (+ a word of the loader's)
     memset(c->ring_host, 0xFF, (size_t)d.max_batch * RING_SLOTS * 4);
     VB_CREATE_CUDA(cudaHostGetDevicePointer((void**)&c->ring_dev, c->ring_host, 0));
     const uint64_t B = d.max_batch;
@@ -799,11 +806,21 @@ static int32_t canon_begin(Tensor* t, Canon* cn) {
     return VB_OK;
 }
 
+__global__ void k_flag_big_scales(uint32_t* flag, const uint16_t* __restrict__ scales, uint64_t n) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        if ((scales[i] & 0x7FFFu) > 0x6FFFu) *flag = 1u;  // 0x6FFF: 8188
+}
+
 static int32_t finish_load(vb_ctx* c, Tensor* t, int32_t role, int32_t layer, const Canon& cn) {
     LaunchCfg lc = lcfg(c, false);
     lc.counter = nullptr;
     if (t->m.tiled) VB_CUDA(tile_q4(lc, const_cast<void*>(t->m.tiled), const_cast<void*>(t->m.tiled_scales), cn.data, cn.scales, t->m.rows, t->m.cols));
     const bool q4 = t->m.fmt == VB_FMT_Q4G32 || t->m.fmt == VB_FMT_Q4G64REF;
+    volatile uint32_t* flag = c->ring_host + (size_t)c->d.max_batch * RING_SLOTS;
+    *flag = 0u;
+    if (t->m.fmt == VB_FMT_Q4G32)
+        VB_CUDA(launch(lc, k_flag_big_scales, dim3(148), dim3(256), 0, c->ring_dev + (size_t)c->d.max_batch * RING_SLOTS, (const uint16_t*)cn.scales,
+                       (uint64_t)t->m.rows * (t->m.cols / 32)));
     if (t->m.v3 && q4) VB_CUDA(tile_q4_v3(lc, const_cast<void*>(t->m.v3), cn.data, cn.scales, t->m.fmt, t->m.rows, t->m.cols));
     if (t->m.v3 && t->m.fmt == VB_FMT_I8PC)
         VB_CUDA(tile_i8_v3(lc, const_cast<void*>(t->m.v3), const_cast<void*>(t->m.v3_scales), cn.data, cn.scales, t->m.rows, t->m.cols));
@@ -819,6 +836,7 @@ static int32_t finish_load(vb_ctx* c, Tensor* t, int32_t role, int32_t layer, co
         }
     }
     VB_CUDA(cudaStreamSynchronize(c->stream));
+    t->beyond_f16 = *flag != 0u;
     return VB_OK;
 }
 
@@ -1037,7 +1055,7 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // velox_cuda_runner_k2.cu:1614-1704.)  Sharded contexts and the last token take the per-token path below.
     // Prompts of up to half a chunk go token by token: the same bits as the same tokens fed one step at a time.
     uint32_t done = 0;
-    const bool gemm_ok = c->prefill_gemm && c->d.tp_size <= 1 && c->prefill_rows >= 1;
+    const bool gemm_ok = c->prefill_gemm && c->d.tp_size <= 1 && c->prefill_rows >= 1 && weights_within_f16(c);
     const bool tc_ok = gemm_ok && n_tokens > c->prefill_gemm_min && tc_products_ok(c);
     const uint32_t rows = std::min(c->prefill_rows, n_tokens - 1);
     const bool use_ts = gemm_ok && n_tokens > c->prefill_ts_min && ts_products_ok(c) && (!tc_ok || rows <= ts_rows_max(c));
