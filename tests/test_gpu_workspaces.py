@@ -73,9 +73,36 @@ def test_prompt_in_a_nearly_full_card():
         eng.reserve(0, 4096)
         eng.prefill(prompt[:17])
         hog = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda") if left else None
-        eng.prefill(prompt)
+        try:
+            eng.prefill(prompt)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
         got.append(eng.logits())
         eng.close()
-        del hog
-        torch.cuda.empty_cache()
     assert np.max(np.abs(got[0] - got[1])) <= 1e-2
+
+
+def test_group64_weights_in_a_nearly_full_card():
+    """The tile-major copies of group-64 weights are left out where only the weights themselves fit; gate and up have one copy, not two."""
+    spec = spec_of(L.FMT_Q4G64REF, d_model=2048, n_layers=4, n_q_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=8192, vocab=32000, embed_fmt=L.FMT_Q4G64REF)
+    packed = sum(rows * cols for _, _, rows, cols, _, _ in spec.tensors() if rows > 1) * 9 // 16
+    prompt, got, sizes = H.prompt_tokens(spec, 74, 12), [], []
+    for left in (None, 400 << 20):
+        hog = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda") if left else None
+        try:
+            eng = Engine(spec, max_seq_len=64)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        eng.load_synthetic(74)
+        eng.reserve(0, 64)
+        eng.prefill(prompt)
+        eng.decode(3)
+        got.append(eng.logits())
+        n = L.C.c_uint64()
+        L.check(L.load().vb_weight_bytes(eng.h, L.C.byref(n)))
+        sizes.append(n.value)
+        eng.close()
+    assert packed <= sizes[1] < 1.01 * packed + (1 << 20) and sizes[0] <= 2 * sizes[1]
+    assert np.max(np.abs(got[0] - got[1])) <= 1e-2  # (the rounding of the fp16 cache apart)

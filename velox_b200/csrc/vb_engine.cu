@@ -76,8 +76,8 @@ void set_tied_head(vb_ctx* c) {
 }
 
 // Lay the arena out in execution order.  Wq|Wk|Wv (and their scales) are adjacent so that the fused QKV
-// product sees one [Hq*D + 2*Hkv*D][d] matrix.
-int32_t plan_arena(vb_ctx* c) {
+// product sees one [Hq*D + 2*Hkv*D][d] matrix.  tile_group64: group-64 int4 matrices get their tile-major copies too.
+int32_t plan_arena(vb_ctx* c, bool tile_group64) {
     uint64_t off = 0;
     // pass 1: compute offsets; pass 2 (after allocation) turns them into pointers
     struct Slot { int role, layer; uint64_t data, scales, tiled, tiled_scales, v3; bool has_tiled; uint64_t v3_scales = ~0ULL; };
@@ -86,14 +86,14 @@ int32_t plan_arena(vb_ctx* c) {
     const bool lean = (c->d.flags & VB_FLAG_LEAN_WEIGHTS) != 0;
     auto add_group = [&](std::initializer_list<int> roles, int layer) {
         std::vector<Slot> g;
-        bool tile_all = true, i8_all = true;  // all members int4 (group-64: not in a lean arena) / all int8 per-channel, in tileable shapes
+        bool tile_all = true, i8_all = true;  // all members int4 / all int8 per-channel, in tileable shapes
         for (int role : roles) {
             uint32_t rows, cols; int32_t fmt;
             if (!role_shape(c, role, &rows, &cols, &fmt)) continue;
             Tensor& t = c->tensor(role, layer);
             t.m.fmt = fmt; t.m.rows = rows; t.m.cols = cols;
             g.push_back({role, layer, ~0ULL, ~0ULL, 0, 0, ~0ULL, false});
-            if (!(fmt == VB_FMT_Q4G32 || (fmt == VB_FMT_Q4G64REF && !lean)) || !tile_q4_supported(rows, cols)) tile_all = false;
+            if (!(fmt == VB_FMT_Q4G32 || (fmt == VB_FMT_Q4G64REF && tile_group64)) || !tile_q4_supported(rows, cols)) tile_all = false;
             if (fmt != VB_FMT_I8PC || !tile_q4_supported(rows, cols)) i8_all = false;
             if (role == VB_ROLE_EMBED && !c->d.tied_lm_head) tile_all = i8_all = false;  // rows are looked up, never multiplied
         }
@@ -124,7 +124,7 @@ int32_t plan_arena(vb_ctx* c) {
                 for (Slot& s : g) { s.has_tiled = true; s.tiled = off; s.tiled_scales = off; off += packed_bytes(s); }
                 off = align256(off);
             }
-            const bool swiglu_only = lean_group && (g[0].role == VB_ROLE_WGATE || g[0].role == VB_ROLE_WUP);
+            const bool swiglu_only = (lean_group || c->tensor(g[0].role, layer).m.fmt == VB_FMT_Q4G64REF) && (g[0].role == VB_ROLE_WGATE || g[0].role == VB_ROLE_WUP);
             if (!swiglu_only) {
                 for (Slot& s : g) { s.v3 = off; off += packed_bytes(s); }  // the integer tensor-core layout
                 off = align256(off);
@@ -161,7 +161,7 @@ int32_t plan_arena(vb_ctx* c) {
                 off += 2 * (wmat_data_bytes(tg.m.fmt, tg.m.rows, tg.m.cols) + wmat_scale_bytes(tg.m.fmt, tg.m.rows, tg.m.cols));
                 off = align256(off);
             } else if ((tg.m.fmt == VB_FMT_I8PC && tile_q4_supported(tg.m.rows, tg.m.cols)) ||
-                       (tg.m.fmt == VB_FMT_Q4G64REF && !lean && tg.m.rows % 8 == 0 && tg.m.cols % 128 == 0)) {
+                       (tg.m.fmt == VB_FMT_Q4G64REF && tile_group64 && tile_q4_supported(tg.m.rows, tg.m.cols))) {
                 swiglu_off.push_back(~0ULL);
                 swiglu_v3_off.push_back(off);  // 2*rows x cols of blocks (int8: then 2*rows scales)
                 off += 2 * (wmat_data_bytes(tg.m.fmt, tg.m.rows, tg.m.cols) + wmat_scale_bytes(tg.m.fmt, tg.m.rows, tg.m.cols));
@@ -177,6 +177,13 @@ int32_t plan_arena(vb_ctx* c) {
     if (!c->d.tied_lm_head) add_group({VB_ROLE_LM_HEAD}, 0);
     add_group({VB_ROLE_EMBED}, 0);
     c->arena_bytes = off ? off : 256;
+    if (tile_group64) {
+        // The copies (as much again as the weights) are a matter of speed: they are made where they leave room for the cache and
+        // what prompts and steps allocate later (8 GB: the workspace of a 72B model's chunks, and some).
+        size_t free_b = 0, total_b = 0;
+        const uint64_t kv = (uint64_t)c->n_blocks * 2 * c->hkv * c->d.kv_block_tokens * c->d.head_dim * c->d.n_layers * sizeof(__half);
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < c->arena_bytes + kv + (8ull << 30)) return plan_arena(c, false);
+    }
     cudaError_t e = cudaMalloc(&c->arena, c->arena_bytes);
     if (e != cudaSuccess) { cuda_fail(e, "cudaMalloc(weight arena)", __FILE__, __LINE__); return VB_ERR_OOM; }
     for (const Slot& s : slots) {
@@ -678,7 +685,7 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
     VB_CREATE_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     VB_CREATE_CUDA(cudaEventCreate(&c->ev0));
     VB_CREATE_CUDA(cudaEventCreate(&c->ev1));
-    VB_CREATE_TRY(plan_arena(c));
+    VB_CREATE_TRY(plan_arena(c, (d.weight_fmt == VB_FMT_Q4G64REF || d.head_fmt == VB_FMT_Q4G64REF) && !(d.flags & VB_FLAG_LEAN_WEIGHTS)));
     c->kv_layer_elems = (uint64_t)c->n_blocks * 2 * c->hkv * d.kv_block_tokens * d.head_dim;
     VB_CREATE_TRY(dev_alloc(&c->kv_pool, c->kv_layer_elems * d.n_layers));
     VB_CREATE_CUDA(cudaMemsetAsync(c->kv_pool, 0, c->kv_layer_elems * d.n_layers * sizeof(__half), c->stream));
