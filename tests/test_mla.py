@@ -209,3 +209,21 @@ def test_mla_context_beyond_max_ctx_ends_at_the_last_slice(vb, path, split, max_
         p = np.exp(s - s.max(axis=1, keepdims=True))
         want = (p / p.sum(axis=1, keepdims=True)) @ cache[b, :n, :DC]
         assert np.max(np.abs(got[b] - want)) <= 2.0 ** -8 * 5, b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,n_out,rows_out", [(128, 512, 0), (512, 128, 1)])
+def test_head_product_rounds_like_fp32(vb, n_in, n_out, rows_out):
+    """The sums of the tensor-core kernel are rounded: n_in / 16 additions, each off by 2^-24 of a partial sum at most and in random
+    directions, and truncations as large inside a step, give 2 * 2^-24 * sqrt(n_in / 16).  (A chain of fp32 multiply-adds over 512
+    is off by 4e-7; sums left to the tensor core, which truncates, by 1.7e-6.)"""
+    from velox_b200.engine import DeviceBuffer as dev
+    heads, batch, rng = 4, 16, np.random.default_rng(n_in)
+    w = O.bf16_round((0.02 * rng.standard_normal((heads, n_out, n_in) if rows_out else (heads, n_in, n_out))).astype(np.float32))
+    x = rng.standard_normal((batch, heads, n_in)).astype(np.float32)
+    d_w, d_x, d_y = dev.from_numpy(O.to_bf16_bits(w)), dev.from_numpy(x), dev(batch * heads * n_out * 4)
+    vb.check(vb.load().vb_op_mla_head_product(d_y.ptr, d_x.ptr, d_w.ptr, heads, n_in, n_out, batch, rows_out, None))
+    vb.check(vb.load().vb_dev_sync())
+    want = np.einsum("bhk,hok->bho" if rows_out else "bhk,hko->bho", x.astype(np.float64), w.astype(np.float64))
+    got = d_y.to_numpy(np.float32, (batch, heads, n_out))
+    assert np.linalg.norm(got - want) <= 2 * 2.0 ** -24 * np.sqrt(n_in / 16) * np.linalg.norm(want)

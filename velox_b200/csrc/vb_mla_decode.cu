@@ -251,8 +251,10 @@ __global__ void __launch_bounds__(256) k_mla_head_product(float* __restrict__ ds
 // warps of 16 outputs x 32 rows, K in chunks of 64, W_h through three stages of cp.async, x through registers (converted on the
 // way to shared memory, the next chunk's loads in flight meanwhile).  W_h and x are read once per such tile; mma and ldmatrix
 // take about the same time (12 and 7 per warp and K step).
-// 128 heads, batch 64: 512 -> 128 17 us, 128 -> 512 21 us (the kernel above, which reads W_h element by element and once for
-// every 16 rows: 198 and 84 us; 32 KB of W_h per block and 16 rows at a time, x converted anew by every block: 45 and 25 us).
+// 128 heads, batch 64: 512 -> 128 16.0 us, 128 -> 512 18.7 us (the kernel above, which reads W_h element by element and once for
+// every 16 rows: 195 and 81 us; 32 KB of W_h per block and 16 rows at a time, x converted anew by every block: 45 and 25 us).
+// Error against 64 bits 1.2e-7 and 0.7e-7 (the kernel above 4.1e-7 and 2.0e-7; with the sums left in the tensor core, 0.5 and 0.9 us
+// faster, 17e-7 and 4.6e-7).
 constexpr int HP_O = 128, HP_B = 64, HP_K = 64, HP_THREADS = 512, HP_XROW = HP_K + 8;  // (rows 16 bytes apart modulo 128: no bank conflicts)
 __device__ __forceinline__ void hp_ldsm4(uint32_t (&r)[4], uint32_t addr, bool trans) {
     if (trans) asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -322,19 +324,24 @@ __global__ void __launch_bounds__(HP_THREADS, 2) k_mla_head_mma(float* __restric
                 uint32_t A[4];
                 hp_ldsm4(A, wb + a_at + (W_ROWS_ARE_OUT ? k : k * W_ROW) * 2, !W_ROWS_ARE_OUT);
 #pragma unroll
-                for (int part = 0; part < 3; ++part) {
+                for (uint32_t np = 0; np < 2; ++np) {
+                    if (np < pairs) {
+                        // The tensor core truncates what it accumulates, so a step starts from zero with the smallest part (its
+                        // truncations are as small) and is added to the sum with a rounding of its own.
+                        float e[2][4] = {};
 #pragma unroll
-                    for (uint32_t np = 0; np < 2; ++np) {
-                        if (np < pairs) {
+                        for (int part = 2; part >= 0; --part) {
                             uint32_t B[4];
                             hp_ldsm4(B, xb + part * X_PART + b_at + (np * 16 * HP_XROW + k) * 2, false);
 #pragma unroll
-                            for (int n = 0; n < 2; ++n) {
-                                float* e = d[2 * np + n];
+                            for (int n = 0; n < 2; ++n)
                                 asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                                    : "+f"(e[0]), "+f"(e[1]), "+f"(e[2]), "+f"(e[3]) : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(B[2 * n]), "r"(B[2 * n + 1]));
-                            }
+                                    : "+f"(e[n][0]), "+f"(e[n][1]), "+f"(e[n][2]), "+f"(e[n][3]) : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(B[2 * n]), "r"(B[2 * n + 1]));
                         }
+#pragma unroll
+                        for (int n = 0; n < 2; ++n)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) d[2 * np + n][i] += e[n][i];
                     }
                 }
             }
