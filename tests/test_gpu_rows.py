@@ -216,3 +216,28 @@ def test_prompts_over_int4_scales_beyond_fp16_products(lean, n):
             ora.forward_step(int(t), pos)
         assert float(np.max(np.abs(eng.logits() - ora.logits))) <= TOL
     eng.close()
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "f16", "bf16", "f32"])
+@pytest.mark.parametrize("batch", [1, 3, 8])
+def test_products_of_a_few_rows_round_like_fp32(oracle, fmt, batch):
+    """The head product of a decode step against 64 bits from the same hidden row: x in parts that carry its 24 bits, every 64 of K
+    added with a rounding of 2^-24 of the partial sum at most, in random directions: 2^-24 * sqrt(K / 64)."""
+    w, emb = FMTS[fmt]
+    d = 4096
+    spec = LLAMA3_8B_INT4.scaled(name="round-" + fmt, d_model=d, n_layers=1, n_q_heads=4, n_kv_heads=2, head_dim=64, ffn_dim=256, vocab=2048,
+                                 weight_fmt=w, head_fmt=w, embed_fmt=emb)
+    eng = H.build_engine(spec, 91, 16, max_batch=batch)
+    for slot in range(batch):
+        eng.reserve(slot, 16)
+        eng.prefill(H.prompt_tokens(spec, 91 + slot, 3), slot)
+    eng.decode(1)
+    data, scales = eng.export_tensor(L.ROLE_LM_HEAD, 0, spec.vocab, d)
+    head = O.dequantize(data, scales, w, spec.vocab, d).astype(np.float64)
+    nfmt = spec.storage_fmt(L.ROLE_FINAL_NORM)
+    norm = O.dequantize(*eng.export_tensor(L.ROLE_FINAL_NORM, 0, 1, d), nfmt, 1, d).astype(np.float64).reshape(d)
+    for slot in range(batch):
+        x = eng.hidden(slot).astype(np.float64)
+        want = head @ (x / np.sqrt((x * x).mean() + spec.rms_eps) * norm)
+        assert np.linalg.norm(eng.logits(slot) - want) <= 2.0 ** -24 * np.sqrt(d / 64) * np.linalg.norm(want), slot
+    eng.close()

@@ -8,10 +8,13 @@
 // writes, more than an SM has).  What has to be kept down is instructions: 16 x 128 weights (1152 bytes) arrive every 50
 // clocks, 200 issue slots.
 //
-// Weights.  A = 16 weight rows x 16 of K.  int4: a masked nibble IS an fp16 operand, the subnormal n * 2^-24 (bits 0-3) or
-// n * 2^-20 (bits 4-7, its x is stored divided by 16), exact: one AND per two weights and no conversion.  Groups keep their
+// Weights.  A = 16 weight rows x 16 of K.  int4 group-32: a masked nibble IS an fp16 operand, the subnormal n * 2^-24 (bits 0-3)
+// or n * 2^-20 (bits 4-7, its x is stored divided by 16), exact: one AND per two weights and no conversion.  Groups keep their
 // own accumulator: symmetric group-32 (n - 8) * s: the accumulator starts at -8 * sum(x), then acc += s * d; group-64
-// n * s + m: acc += s * d + m * sum(x).  Block layout: the "v3" tiles of vb_gemv_imma.cu (a lane's 16 bytes are its words of
+// n * s + m = (n - 8) * s + (m + 8 s): acc += s * d + (m + 8 s) * sum(x).  The tensor core aligns a subnormal operand's products
+// by its exponent, not by its leading bit, and drops bits below: 1e-6 of a product's result, which the integer kernel's x (1.7e-5)
+// does not notice, but group-64 weights, whose other kernels compute in fp32 (1.1e-7), do: their nibbles become n - 8 by one
+// addition (1.1..1.9e-7; 5 % of a decode step of the 8B shape).  Block layout: the "v3" tiles of vb_gemv_imma.cu (a lane's 16 bytes are its words of
 // four groups, so that one mma pair stays inside a group).  fp16 / bf16: rows g and g + 8 of the canonical matrix, 16 bytes
 // a lane: the lane's 8 elements of K are its share of two mma (the order of K inside them is free as long as x follows it).
 //
@@ -22,14 +25,18 @@
 // block's share (with its sums) contiguous.  The products stream it through a ring of bulk copies in shared memory: read
 // through L1 instead, every block of K waited a trip to L2 (gate/up of the 8B shape, 4 rows: 23 us).
 //
+// Sums.  The tensor core truncates what it accumulates: 16-bit products left in one accumulator along K were off by 3e-6 (K 4096) to
+// 9e-6 (14336), all to the same side.  Every 64 of K start from zero and are added with a rounding: 1.3..1.8e-7 (fp32 kernel 1.0..1.4e-7),
+// for 4 % of a step of 5 rows and more.
+//
 // Split.  A block is 4 warps on 4 row tiles (8 on 16 for 32 columns) over the same range of K, so that they share the
 // fragments.  Matrices with few tiles split K over a cluster of up to 8 blocks; the partials meet in distributed shared memory
 // and are added in rank order (the same bits every run).  A warp streams its tiles through a ring of its own, filled before the
 // grid-dependency wait.
 //
 // Measured, 8B shape, a product with its k_x_frag in a graph: gate/up with 4 rows 22.9 us, with 8 rows 30.7, with 16 46.5
-// (vb_gemv_imma.cu: 19.3 us for every 4 rows); down 15.8 / 21.4 / 42 (21.6 for every 4); group-64 gate/up with one row 21.5
-// (fp32 kernel: 50); fp16 gate/up with 4 rows 46.6 (235 MB: 5.0 TB/s; fp32 kernel 72).  The steady state is bound by issue
+// (vb_gemv_imma.cu: 19.3 us for every 4 rows); down 15.8 / 21.4 / 42 (21.6 for every 4); fp16 gate/up with 4 rows 46.6 (235 MB:
+// 5.0 TB/s; fp32 kernel 72).  A step of one group-64 row 2.09 ms (fp32 kernel: 3.9).  The steady state is bound by issue
 // and latency (IPC 1.6 of 4, ~115 instructions a block and 8 columns): 5.0 TB/s of int4, 6.0 of fp16.
 #include <cooperative_groups.h>
 
@@ -97,11 +104,26 @@ __device__ __forceinline__ void mma16816_from(float (&d)[4], uint32_t a0, uint32
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
 }
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-// the words of rows g and g + 8 as the A operands of two mma (see the head of the file)
+// the words of rows g and g + 8 as the A operands of two mma, subnormal (see the head of the file)
 __device__ __forceinline__ void nibbles(uint32_t (&A)[8], uint32_t u, uint32_t v) {
     A[0] = u & 0x000F000Fu; A[1] = v & 0x000F000Fu; A[2] = u & 0x00F000F0u; A[3] = v & 0x00F000F0u;
     u >>= 8; v >>= 8;
     A[4] = u & 0x000F000Fu; A[5] = v & 0x000F000Fu; A[6] = u & 0x00F000F0u; A[7] = v & 0x00F000F0u;
+}
+
+__device__ __forceinline__ uint32_t hadd2_bits(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// the same as normal numbers: n - 8 (bits 0-3) and 16 * (n - 8) (bits 4-7)
+__device__ __forceinline__ void nibbles_normal(uint32_t (&A)[8], uint32_t u, uint32_t v) {
+    constexpr uint32_t LOW = 0xE408E408u, HIGH = 0xE480E480u;  // -1032, -1152
+    A[0] = hadd2_bits(lop3_and_or(u, 0x000F000Fu, 0x64006400u), LOW); A[1] = hadd2_bits(lop3_and_or(v, 0x000F000Fu, 0x64006400u), LOW);
+    A[2] = hadd2_bits(lop3_and_or(u, 0x00F000F0u, 0x64006400u), HIGH); A[3] = hadd2_bits(lop3_and_or(v, 0x00F000F0u, 0x64006400u), HIGH);
+    u >>= 8; v >>= 8;
+    A[4] = hadd2_bits(lop3_and_or(u, 0x000F000Fu, 0x64006400u), LOW); A[5] = hadd2_bits(lop3_and_or(v, 0x000F000Fu, 0x64006400u), LOW);
+    A[6] = hadd2_bits(lop3_and_or(u, 0x00F000F0u, 0x64006400u), HIGH); A[7] = hadd2_bits(lop3_and_or(v, 0x00F000F0u, 0x64006400u), HIGH);
 }
 
 // Bounded wait (vb_tma.cuh); one that runs out is reported and the block carries on with what is there.
@@ -269,10 +291,11 @@ __global__ void __launch_bounds__(MmShape<FMT, T>::warps * 32, MmShape<FMT, T>::
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
 #pragma unroll
-                            for (int i = 0; i < 2; ++i) nibbles(A[m][i], word_of(w0[m], 2 * h + i), word_of(w1[m], 2 * h + i));
+                            for (int i = 0; i < 2; ++i) nibbles_normal(A[m][i], word_of(w0[m], 2 * h + i), word_of(w1[m], 2 * h + i));
                             const uint32_t z0 = word_of(w2[m], h), z1 = word_of(w2[m], 2 + h);
                             s0[m] = __half22float2(*reinterpret_cast<const __half2*>(&z0));
                             s1[m] = __half22float2(*reinterpret_cast<const __half2*>(&z1));
+                            s0[m].y = fmaf(8.0f, s0[m].x, s0[m].y); s1[m].y = fmaf(8.0f, s1[m].x, s1[m].y);  // n * s + m = (n - 8) * s + (m + 8 * s)
                         }
 #pragma unroll
                         for (int n = 0; n < T; ++n) {
@@ -292,16 +315,18 @@ __global__ void __launch_bounds__(MmShape<FMT, T>::warps * 32, MmShape<FMT, T>::
                     }
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
+                    for (int n = 0; n < T; ++n) {
+                        const uint4 b0 = xp[n * 32], b1 = xp[(T + n) * 32];
 #pragma unroll
-                        for (int n = 0; n < T; ++n) {
-                            const uint4 bx = xp[(j * T + n) * 32];
+                        for (int m = 0; m < MT; ++m) {
+                            const uint4 &u0 = w[m][0], &v0 = w[m][1], &u1 = w[m][2], &v1 = w[m][3];
+                            float e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                            mma16816<FMT>(e, u0.x, v0.x, u0.y, v0.y, b0.x, b0.y);
+                            mma16816<FMT>(e, u0.z, v0.z, u0.w, v0.w, b0.z, b0.w);
+                            mma16816<FMT>(e, u1.x, v1.x, u1.y, v1.y, b1.x, b1.y);
+                            mma16816<FMT>(e, u1.z, v1.z, u1.w, v1.w, b1.z, b1.w);
 #pragma unroll
-                            for (int m = 0; m < MT; ++m) {
-                                const uint4 &u = w[m][2 * j], &v = w[m][2 * j + 1];
-                                mma16816<FMT>(acc[m][n], u.x, v.x, u.y, v.y, bx.x, bx.y);
-                                mma16816<FMT>(acc[m][n], u.z, v.z, u.w, v.w, bx.z, bx.w);
-                            }
+                            for (int i = 0; i < 4; ++i) acc[m][n][i] += e[i];
                         }
                     }
                 }
@@ -466,7 +491,7 @@ __global__ void __launch_bounds__(XF_THREADS) k_x_frag(const XfArgs a) {
         }
     }
     if (!active) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.unscale[b] = (F::q4 ? 16777216.0f : 1.0f) / up;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.unscale[b] = (FMT == VB_FMT_Q4G32 ? 16777216.0f : 1.0f) / up;
     if (a.norm_w && in) {
         p.x = (p.x * inv) * wp.x; p.y = (p.y * inv) * wp.y; p.z = (p.z * inv) * wp.z; p.w = (p.w * inv) * wp.w;
         q.x = (q.x * inv) * wq.x; q.y = (q.y * inv) * wq.y; q.z = (q.z * inv) * wq.z; q.w = (q.w * inv) * wq.w;
@@ -512,7 +537,7 @@ __global__ void __launch_bounds__(XF_THREADS) k_x_frag(const XfArgs a) {
                     float* f = reinterpret_cast<float*>(sums) + (c >> 1) * 4 + (c & 1);
                     f[0] = f[2] = sum * (-8.0f / 16777216.0f);
                 } else {
-                    reinterpret_cast<float*>(sums)[c] = sum / 16777216.0f;
+                    reinterpret_cast<float*>(sums)[c] = sum;
                 }
             }
         }
