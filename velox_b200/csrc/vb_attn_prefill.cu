@@ -2,8 +2,10 @@
 // first..first+n-1 of ONE sequence, whose K/V (this chunk's included) are already in the cache.  Same arithmetic
 // as the per-token kernel of vb_attn.cu with fp16 caches (the reference: src/runtime.rs:772-831, one query at a
 // time; its batched driver: src/runners/velox_cuda_runner_k2.cu:1614-1704): scores (q.k)/sqrt(D), softmax over
-// positions <= the row's own, weighted sum of V; q and the softmax weights are rounded to fp16 for the two
-// products, maxima, sums and accumulators are fp32.
+// positions <= the row's own, weighted sum of V; maxima, sums and accumulators are fp32.  For the two products q and the softmax
+// weights are fp16, rounded (chunks over fp16 copies of the weights), or with SPLIT two fp16 parts each, as in the per-token
+// kernel: prompts that kernel had served (error of their logits, 8B int4 shape, four layers, 17 to 48 tokens: 1.99e-4 with it,
+// 1.97e-4 with parts, 2.05e-4 with rounded ones; the prompt takes the same time).
 //
 // One block = 64 consecutive rows of one query head (4 warps x 16 rows); the K/V rows of the head's KV group are
 // staged 64 positions at a time with cp.async (double buffered, rows padded by 16 bytes against bank conflicts),
@@ -38,8 +40,13 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// what the fp16 pair `h` dropped of (lo, hi)
+__device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t h) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    return pack_h2(lo - f.x, hi - f.y);
+}
 
-template <int D, int PER_SM>
+template <int D, int PER_SM, bool SPLIT>
 __global__ void __launch_bounds__(128, PER_SM)
 k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __half* __restrict__ kv_layer,
                const int32_t* __restrict__ table_row, uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens,
@@ -83,7 +90,7 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
     stage(0, 0);
 
     // this warp's 16 rows of q as A fragments, pre-scaled by 1/sqrt(D)
-    uint32_t qa[D / 16][4];
+    uint32_t qa[D / 16][4], ql[SPLIT ? D / 16 : 1][4];  // (ql: what the rounding of qa dropped)
     {
         const uint32_t ra = r0 + warp * 16 + g, rb = ra + 8;
         const float* qa_row = q + ((size_t)min(ra, n - 1) * Hq + h) * D;
@@ -94,10 +101,12 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
             const float2 a1 = *reinterpret_cast<const float2*>(qb_row + kt * 16 + 2 * t);
             const float2 a2 = *reinterpret_cast<const float2*>(qa_row + kt * 16 + 8 + 2 * t);
             const float2 a3 = *reinterpret_cast<const float2*>(qb_row + kt * 16 + 8 + 2 * t);
-            qa[kt][0] = pack_h2(a0.x * scale, a0.y * scale);
-            qa[kt][1] = pack_h2(a1.x * scale, a1.y * scale);
-            qa[kt][2] = pack_h2(a2.x * scale, a2.y * scale);
-            qa[kt][3] = pack_h2(a3.x * scale, a3.y * scale);
+            const float2 a[4] = {a0, a1, a2, a3};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                qa[kt][i] = pack_h2(a[i].x * scale, a[i].y * scale);
+                if constexpr (SPLIT) ql[kt][i] = pack_rest(a[i].x * scale, a[i].y * scale, qa[kt][i]);
+            }
         }
     }
     float o[D / 8][4];
@@ -125,6 +134,7 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
                 for (int j = 0; j < KTILE / 8; ++j) {
                     uint32_t b0, b1, b2, b3;
                     ldsm_x4(sK + (8 * j + (lane & 7)) * ROWB + (16 * kt + 8 * (lane >> 3)) * 2, b0, b1, b2, b3);
+                    if constexpr (SPLIT) { mma16816(s[j], ql[kt], b0, b1); mma16816(s[j], ql[kt + 1], b2, b3); }
                     mma16816(s[j], qa[kt], b0, b1);
                     mma16816(s[j], qa[kt + 1], b2, b3);
                 }
@@ -147,7 +157,7 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
             const float ca = exp2f((m_a - mx_a) * LOG2E), cb = exp2f((m_b - mx_b) * LOG2E);
             m_a = mx_a; m_b = mx_b;
             float sum_a = 0.0f, sum_b = 0.0f;
-            uint32_t pa[KTILE / 16][4];
+            uint32_t pa[KTILE / 16][4], pl[SPLIT ? KTILE / 16 : 1][4];
 #pragma unroll
             for (int j = 0; j < KTILE / 8; ++j) {
                 const float p0 = exp2f((s[j][0] - m_a) * LOG2E), p1 = exp2f((s[j][1] - m_a) * LOG2E);
@@ -155,6 +165,10 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
                 sum_a += p0 + p1; sum_b += p2 + p3;
                 pa[j >> 1][(j & 1) * 2 + 0] = pack_h2(p0, p1);
                 pa[j >> 1][(j & 1) * 2 + 1] = pack_h2(p2, p3);
+                if constexpr (SPLIT) {
+                    pl[j >> 1][(j & 1) * 2 + 0] = pack_rest(p0, p1, pa[j >> 1][(j & 1) * 2 + 0]);
+                    pl[j >> 1][(j & 1) * 2 + 1] = pack_rest(p2, p3, pa[j >> 1][(j & 1) * 2 + 1]);
+                }
             }
             l_a = l_a * ca + sum_a; l_b = l_b * cb + sum_b;
 #pragma unroll
@@ -166,6 +180,7 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
                     uint32_t b0, b1, b2, b3;
                     const uint32_t mtx = lane >> 3;
                     ldsm_x4_t(sV + (16 * kk + 8 * (mtx & 1) + (lane & 7)) * ROWB + (8 * (dn + (mtx >> 1))) * 2, b0, b1, b2, b3);
+                    if constexpr (SPLIT) { mma16816(o[dn], pl[kk], b0, b1); mma16816(o[dn + 1], pl[kk], b2, b3); }
                     mma16816(o[dn], pa[kk], b0, b1);
                     mma16816(o[dn + 1], pa[kk], b2, b3);
                 }
@@ -185,21 +200,21 @@ k_attn_prefill(float* __restrict__ out, const float* __restrict__ q, const __hal
     }
 }
 
-template <int D, int PER_SM>
+template <int D, int PER_SM, bool SPLIT>
 cudaError_t launch_prefill_n(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
                            uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens) {
     constexpr int SMEM = 2 * 2 * KTILE * (D + 8) * 2;
     static std::atomic<uint64_t> opted{0};
     const cudaError_t oe = once_per_device(opted, [&]() {
-        cudaError_t e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e == cudaSuccess && PER_SM == 3) e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaError_t e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e == cudaSuccess && PER_SM == 3) e = cudaFuncSetAttribute(k_attn_prefill<D, PER_SM, SPLIT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         return e;
     });
     if (oe != cudaSuccess) return oe;
     const float scale = 1.0f / sqrtf((float)D);
     uint32_t bt_shift = 32;  // block_tokens as a power of two, 32: it is none
     if ((block_tokens & (block_tokens - 1)) == 0) for (bt_shift = 0; (1u << bt_shift) < block_tokens;) ++bt_shift;
-    return launch(lc, k_attn_prefill<D, PER_SM>, dim3(Hq, (n + QROWS - 1) / QROWS), dim3(128), SMEM, out, q, kv_layer, table_row, first, n, Hq,
+    return launch(lc, k_attn_prefill<D, PER_SM, SPLIT>, dim3(Hq, (n + QROWS - 1) / QROWS), dim3(128), SMEM, out, q, kv_layer, table_row, first, n, Hq,
                   Hkv, block_tokens, bt_shift, scale);
 }
 
@@ -207,10 +222,11 @@ cudaError_t launch_prefill_n(const LaunchCfg& lc, float* out, const float* q, co
 // to the other kernels' shared-memory split changing, which short chunks do not get back.  1999 rows, 28 heads of 128: 192 -> 151 us.
 template <int D>
 cudaError_t launch_prefill(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer,
-                           const int32_t* table_row, uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens) {
+                           const int32_t* table_row, uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t block_tokens, bool split) {
+    if (split) return launch_prefill_n<D, 1, true>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
     if ((uint64_t)Hq * ((n + QROWS - 1) / QROWS) > 2 * 148)
-        return launch_prefill_n<D, 3>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
-    return launch_prefill_n<D, 1>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
+        return launch_prefill_n<D, 3, false>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
+    return launch_prefill_n<D, 1, false>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
 }
 
 }  // namespace
@@ -220,13 +236,13 @@ bool attention_prefill_supported(uint32_t Hq, uint32_t Hkv, uint32_t D) {
 }
 
 // out/q: [n][Hq*D] fp32 (q with bias and RoPE applied); rows are positions first..first+n-1 of the sequence whose
-// block-table row is `table_row`.
+// block-table row is `table_row`.  split: q and the softmax weights as two fp16 parts each.
 cudaError_t attention_prefill(const LaunchCfg& lc, float* out, const float* q, const __half* kv_layer, const int32_t* table_row,
-                              uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t D, uint32_t block_tokens) {
+                              uint32_t first, uint32_t n, uint32_t Hq, uint32_t Hkv, uint32_t D, uint32_t block_tokens, bool split) {
     if (n == 0) return cudaSuccess;
     if (!attention_prefill_supported(Hq, Hkv, D)) return cudaErrorInvalidValue;
-    if (D == 64) return launch_prefill<64>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
-    return launch_prefill<128>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens);
+    if (D == 64) return launch_prefill<64>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens, split);
+    return launch_prefill<128>(lc, out, q, kv_layer, table_row, first, n, Hq, Hkv, block_tokens, split);
 }
 
 }  // namespace vb

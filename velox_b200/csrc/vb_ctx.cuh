@@ -153,6 +153,7 @@ struct StepIO {
     uint64_t i8_ws_bytes = 0;
     uint32_t first = 0;     // tensor-core chunks: position of row 0 (row j is position first + j of one sequence)
     bool causal_chunk = false;  // rows are consecutive positions of one sequence (prefill chunk), not one row per slot
+    bool split_attn = false;    // ... whose attention keeps the parts of q and of the softmax weights that one fp16 value drops
 };
 
 template <typename T>

@@ -508,7 +508,7 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
         a.max_splits = c->n_splits; a.tokens_per_split = c->tokens_per_split; a.scratch = c->attn_scratch;
         a.trace = next_trace(); a.err = c->err_word;
         if (io.causal_chunk && c->prefill_flash && attention_prefill_supported(c->hq, c->hkv, d.head_dim))
-            VB_TRY(attention_prefill(lcfg(c, true), io.attn_out, io.q, kv_layer, io.block_table, io.first, B, c->hq, c->hkv, d.head_dim, d.kv_block_tokens));
+            VB_TRY(attention_prefill(lcfg(c, true), io.attn_out, io.q, kv_layer, io.block_table, io.first, B, c->hq, c->hkv, d.head_dim, d.kv_block_tokens, io.split_attn));
         else
             VB_TRY(attention(lcfg(c, true), a));
         // O-projection + residual
@@ -1093,6 +1093,7 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
         if (use_ts) { io.ts_ws = c->ts_ws; io.ts_ws_bytes = c->ts_ws_bytes; }
         else if (use_tc) { io.tc_ws = tc_ws_aligned(c); io.tc_ws_bytes = c->tc_ws_bytes; }
         io.causal_chunk = use_tc;
+        io.split_attn = !tc_ok;
         // the last token always takes the per-token path below (it produces the logits); the last chunk may be ragged (token by
         // token instead, a 120-token prompt of the 72B shape spent 66 ms on its last 8)
         while (done + 1 < n_tokens) {
