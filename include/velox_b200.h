@@ -269,7 +269,8 @@ int32_t vb_op_embed(float* dst, const uint32_t* tokens, const void* table, const
 /* RmsNorm (src/runtime.rs:588-601). `w_fmt` F32 or F16. */
 int32_t vb_op_rmsnorm(float* dst, const float* x, const void* w, int32_t w_fmt, uint32_t dim, uint32_t batch,
                       float eps, void* stream);
-/* Matmul (src/runtime.rs:702-740): dst[b][o] = sum_k x[b][k] * W[o][k], W in canonical layout. */
+/* Matmul (src/runtime.rs:702-740): dst[b][o] = sum_k x[b][k] * W[o][k], W in canonical layout.  Here and below x, dst and the
+ * norm weights may start at any element; W of fp32 / fp16 / bf16 starts on 16 bytes, of int8 on 8, of int4 (and its scales) on 4. */
 int32_t vb_op_matmul(float* dst, const float* x, const void* w, const void* scales, int32_t fmt,
                      uint32_t in_dim, uint32_t out_dim, uint32_t batch, void* stream);
 /* Multi-row Matmul on the tcgen05 tensor cores (the reference's multi-token kernels for prefill chunks and

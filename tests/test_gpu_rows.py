@@ -1,5 +1,7 @@
 """Products of a few rows of x (mma.sync kernel) and single rows of every format: one decode step of a batch against the
 CPU checker, at the sizes where tiles, column groups, weight passes and cluster splits end."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -266,3 +268,64 @@ def test_short_prompts_keep_the_parts_of_q_and_probabilities(head_dim, lean, n):
         got.append(eng.logits().astype(np.float64))
     eng.close()
     assert np.linalg.norm(got[1] - got[0]) <= 4e-5 * np.linalg.norm(got[0])
+
+
+@functools.lru_cache(maxsize=1)
+def checker_of(fmt, wide):
+    """(spec, CPU checker) with rows of 4096: `wide` one layer whose matrices are all large, else two of few heads."""
+    w, emb = {**FMTS, "i8": (L.FMT_I8PC, L.FMT_F16)}[fmt]
+    kw = dict(n_layers=1, n_q_heads=32, n_kv_heads=8, head_dim=128, ffn_dim=1024, vocab=2048) if wide else dict(
+        n_layers=2, n_q_heads=4, n_kv_heads=2, head_dim=64, ffn_dim=1536, vocab=512)
+    spec = LLAMA3_8B_INT4.scaled(name="k4096-" + fmt, d_model=4096, weight_fmt=w, head_fmt=w, embed_fmt=emb, **kw)
+    return spec, H.build_oracle(spec, 31, 144)[0]
+
+
+TOL_4096 = TOL * 8 ** 0.5  # rows eight times as long: logits sqrt(8) times as large
+
+
+@pytest.mark.parametrize("fmt,batch", [("bf16", 3), ("bf16", 4), ("f16", 3), ("f16", 4), ("q4_0", 1), ("q4_0", 3), ("q4_0", 4), ("q4_0", 8),
+                                       ("q4g32", 2), ("q4g32", 4), ("q4g32", 8)])
+def test_large_matrices_match_checker(fmt, batch):
+    """Matrices of 8M weights and more (QKV 6144 x 4096, O 4096 x 4096 onto the residual stream, gate/up 2048 x 4096, head 2048 x 4096):
+    one and two groups of eight columns, K split over clusters of 4 and 8, one row of group-64."""
+    spec, ora = checker_of(fmt, True)
+    eng = H.build_engine(spec, 31, 16, max_batch=batch)
+    rng = np.random.default_rng(batch)
+    toks = rng.integers(0, spec.vocab, size=(batch, 3))
+    for slot in range(batch):
+        eng.reserve(slot, 16)
+        eng.prefill(toks[slot, :2].astype(np.uint32), slot)
+        eng.set_state(slot, int(toks[slot, 2]), 2)
+    eng.decode(1)
+    for slot in sorted({0, batch // 2, batch - 1}):
+        for pos, t in enumerate(toks[slot]):
+            ora.forward_step(int(t), pos)
+        assert float(np.max(np.abs(eng.logits(slot) - ora.logits))) <= TOL_4096, slot
+    eng.close()
+
+
+@pytest.mark.parametrize("fmt,lean", [("i8", False), ("q4g32", False), ("q4g32", True)])
+def test_prompt_products_split_over_large_clusters(fmt, lean):
+    """Prompts over rows of 4096: QKV of 512 rows splits K over clusters of 8, gate/up of 3072 over 4; one to 128 rows a tile.  Steps at
+    shrinking positions look at the cached rows again, with few others to dilute them."""
+    spec, ora = checker_of(fmt, False)
+    ns, later = (17, 33, 65, 129), (16, 2, 1)
+    prompt, want, steps = H.prompt_tokens(spec, 31, ns[-1]), {}, []
+    for pos, t in enumerate(prompt):
+        ora.forward_step(int(t), pos)
+        if pos + 1 in ns:
+            want[pos + 1] = ora.logits.copy()
+    for pos in later:
+        ora.forward_step(7, pos)
+        steps.append(ora.logits.copy())
+    eng = Engine(spec, max_seq_len=144, lean_weights=lean)
+    eng.load_synthetic(31)
+    eng.reserve(0, 144)
+    for n in ns:
+        eng.prefill(prompt[:n])
+        assert float(np.max(np.abs(eng.logits() - want[n]))) <= TOL_4096, n
+        for pos, w in zip(later, steps):
+            eng.set_state(0, 7, pos)
+            eng.decode(1)
+            assert float(np.max(np.abs(eng.logits() - w))) <= TOL_4096, (n, pos)
+    eng.close()

@@ -227,3 +227,31 @@ def test_head_product_rounds_like_fp32(vb, n_in, n_out, rows_out):
     want = np.einsum("bhk,hok->bho" if rows_out else "bhk,hko->bho", x.astype(np.float64), w.astype(np.float64))
     got = d_y.to_numpy(np.float32, (batch, heads, n_out))
     assert np.linalg.norm(got - want) <= 2 * 2.0 ** -24 * np.sqrt(n_in / 16) * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("path", [0, 1])
+@pytest.mark.parametrize("scale", [float("nan"), 0.0, -0.07])
+def test_mla_unusual_scales(vb, path, scale):
+    """A scale that is no number is not taken for zero; zero weighs all rows alike; a negative one turns the scores round."""
+    from velox_b200.engine import DeviceBuffer as dev
+    lib, rng, heads, n = vb.load(), np.random.default_rng(2), 8, 70
+    q = O.bf16_round(rng.standard_normal((1, heads, DC + DR)).astype(np.float32))
+    cache = O.bf16_round(rng.standard_normal((1, 128, DC + DR)).astype(np.float32))
+    d_q, d_cache, d_len = dev.from_numpy(q), dev.from_numpy(O.to_bf16_bits(cache)), dev.from_numpy(np.array([n], np.uint32))
+    need = lib.vb_op_mla_decode_scratch_bytes(1, heads, 128, 0)
+    d_scratch, d_out = dev(need), dev(heads * DC * 4)
+    vb.check(lib.vb_op_mla_set_path(path))
+    try:
+        vb.check(lib.vb_op_mla_decode(d_out.ptr, d_q.ptr, d_cache.ptr, d_len.ptr, 1, heads, 128, 128, scale, 0, d_scratch.ptr, need, None))
+        vb.check(lib.vb_dev_sync())
+    finally:
+        vb.check(lib.vb_op_mla_set_path(1))
+    got = d_out.to_numpy(np.float32, (heads, DC))
+    if scale != scale:
+        assert np.all(np.isnan(got))
+        return
+    s = (q[0] @ cache[0, :n].T) * scale
+    p = np.exp(s - s.max(axis=1, keepdims=True))
+    want = (p / p.sum(axis=1, keepdims=True)) @ cache[0, :n, :DC]
+    assert np.max(np.abs(got - want)) <= 2.0 ** -8 * 5

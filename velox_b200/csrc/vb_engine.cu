@@ -622,7 +622,7 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
                fmt_shape_ok((int32_t)d.embed_fmt, d.d_model) && d.d_model % 8 == 0 && d.ffn_dim % 8 == 0,
                "vb_create: dimensions not divisible by the quantization group of the chosen format");
     VB_REQUIRE(!d.tied_lm_head || d.head_fmt == d.embed_fmt, "vb_create: tied lm_head needs head_fmt == embed_fmt");
-    VB_REQUIRE((uint64_t)d.ffn_dim * 4 <= 200 * 1024 && (uint64_t)d.d_model * 4 <= 200 * 1024, "vb_create: width exceeds the staging limit");
+    VB_REQUIRE((uint64_t)d.ffn_dim * 4 <= 200 * 1024 && (uint64_t)d.d_model * 4 <= 200 * 1024, "vb_create: a width exceeds 51200");
     if (d.attn_kind != VB_ATTN_GQA) { set_error("vb_create: attn_kind %u is served by vb_op_mla_absorbed only", d.attn_kind); return VB_ERR_UNSUPPORTED; }
     VB_REQUIRE((d.flags & ~VB_FLAG_LEAN_WEIGHTS) == 0, "vb_create: unknown flags 0x%x", d.flags);
     VB_REQUIRE(!(d.flags & VB_FLAG_LEAN_WEIGHTS) || d.max_batch == 1, "vb_create: VB_FLAG_LEAN_WEIGHTS serves max_batch == 1 only");

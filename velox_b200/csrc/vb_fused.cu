@@ -115,7 +115,7 @@ int32_t vb_op_fused_norm_qkv_rope_attn(float* dst_attn, const float* input_hidde
     VB_REQUIRE(n_kv > 0 && n_q % n_kv == 0, "vb_op_fused_norm_qkv_rope_attn: n_q=%u not a multiple of n_kv=%u", n_q, n_kv);
     VB_REQUIRE(head_dim == 32 || head_dim == 64 || head_dim == 128 || head_dim == 256, "vb_op_fused_norm_qkv_rope_attn: head_dim=%u", head_dim);
     VB_REQUIRE(max_seq > 0 && (step_dev || step < max_seq), "vb_op_fused_norm_qkv_rope_attn: step %u outside the cache of %u rows", step, max_seq);
-    VB_REQUIRE((size_t)d_model * 4 <= 200 * 1024, "vb_op_fused_norm_qkv_rope_attn: d_model=%u exceeds the staging limit", d_model);
+    VB_REQUIRE((size_t)d_model * 4 <= 200 * 1024, "vb_op_fused_norm_qkv_rope_attn: d_model=%u exceeds 51200", d_model);
     VB_REQUIRE(((uintptr_t)k_layer & 15) == 0 && ((uintptr_t)v_layer & 15) == 0 && ((uintptr_t)scratch & 15) == 0, "vb_op_fused_norm_qkv_rope_attn: caches and scratch must be 16-byte aligned");
     VB_REQUIRE(scratch_bytes >= vb_op_fused_scratch_bytes(d_model, n_q, n_kv, head_dim, 0, max_seq), "vb_op_fused_norm_qkv_rope_attn: scratch of %llu bytes is too small", (unsigned long long)scratch_bytes);
     const uint32_t qdim = n_q * head_dim, kvdim = n_kv * head_dim;
@@ -161,7 +161,7 @@ int32_t vb_op_fused_outproj_res_swiglu_res(float* dst_hidden, const float* attn_
                "vb_op_fused_outproj_res_swiglu_res: bad weight descriptor");
     VB_REQUIRE(w_gate->fmt == w_up->fmt, "vb_op_fused_outproj_res_swiglu_res: gate and up must share a format");
     VB_REQUIRE((size_t)ffn_dim * 4 <= 200 * 1024 && (size_t)d_model * 4 <= 200 * 1024 && (size_t)attn_dim * 4 <= 200 * 1024,
-               "vb_op_fused_outproj_res_swiglu_res: a width exceeds the staging limit");
+               "vb_op_fused_outproj_res_swiglu_res: a width exceeds 51200");
     VB_REQUIRE(scratch_bytes >= align16((uint64_t)ffn_dim * 4) && ((uintptr_t)scratch & 15) == 0, "vb_op_fused_outproj_res_swiglu_res: scratch of %llu bytes is too small or unaligned", (unsigned long long)scratch_bytes);
     float* act = (float*)scratch;
     LaunchCfg lc;
@@ -194,7 +194,7 @@ int32_t vb_op_swiglu(float* dst, const float* input, const vb_weight* w_gate, co
                      uint32_t d_model, uint32_t ffn_dim, void* scratch, uint64_t scratch_bytes, void* stream) {
     VB_REQUIRE(dst && input && scratch, "vb_op_swiglu: null pointer");
     VB_REQUIRE(weight_ok(w_gate, d_model) && weight_ok(w_up, d_model) && weight_ok(w_down, ffn_dim) && w_gate->fmt == w_up->fmt, "vb_op_swiglu: bad weight descriptor");
-    VB_REQUIRE((size_t)ffn_dim * 4 <= 200 * 1024 && (size_t)d_model * 4 <= 200 * 1024, "vb_op_swiglu: a width exceeds the staging limit");
+    VB_REQUIRE((size_t)ffn_dim * 4 <= 200 * 1024 && (size_t)d_model * 4 <= 200 * 1024, "vb_op_swiglu: a width exceeds 51200");
     VB_REQUIRE(scratch_bytes >= align16((uint64_t)ffn_dim * 4) && ((uintptr_t)scratch & 15) == 0, "vb_op_swiglu: scratch too small or unaligned");
     float* act = (float*)scratch;
     LaunchCfg lc;

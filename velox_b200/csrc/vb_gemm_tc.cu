@@ -9,9 +9,9 @@
 //     (q-8)*s rounded once; int8 per channel: the integer, exact, the row scale is applied to the fp32
 //     accumulator in the epilogue), either once into a resident copy the engine keeps or per call into the
 //     workspace; fp16 matrices are used where they lie;
-//   * k_gemm_tc: one block per tile of 128 weight rows (the M of the instruction, = tensor-memory lanes) by 32,
-//     128 or 256 rows of x (N, = tensor-memory columns).  Warp 0 / lane 0 issues the TMA copies of 128-byte-swizzled
-//     [128][64] fp16 boxes into a ring of stages, warp 1 / lane 0 issues tcgen05.mma (four K=16 steps per
+//   * k_gemm_tc: one block per tile of 128 weight rows (the M of the instruction, = tensor-memory lanes) by 32 or
+//     128 rows of x (N, = tensor-memory columns).  An elected lane of warp 0 issues the TMA copies of 128-byte-swizzled
+//     [128][64] fp16 boxes into a ring of stages, one of warp 1 tcgen05.mma (four K=16 steps per
 //     stage) and hands each stage back with tcgen05.commit, all four warps read the accumulator with
 //     tcgen05.ld and write the epilogue (store / residual add / SiLU(gate)*up with the two accumulators of the
 //     gate and up matrices side by side in tensor memory).
@@ -28,7 +28,7 @@ namespace vb {
 namespace {
 
 constexpr int BM = 128;      // weight rows per tile (UMMA M)
-                             // rows of x per tile (UMMA N): 128 or 256, a template parameter of the kernel
+                             // rows of x per tile (UMMA N): 32 or 128, a template parameter of the kernel
 constexpr int BK = 64;       // K extent of a stage: 64 fp16 = one 128-byte swizzle row
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KB: one box of 128 rows
 // the ring of stages fills 192 KB; PER_SM = 2: 96 KB, so that two blocks share an SM and one block's prologue and epilogue
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128, PER_SM)
 k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
           const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wl, const __grid_constant__ CUtensorMap map_wl2,
           const GemmParams p) {
-    constexpr int W_TILES = DUAL ? 2 : 1, X_TILES = BN / 128;  // BN = 32: one box of 32 rows
+    constexpr int W_TILES = DUAL ? 2 : 1;
     constexpr int X_BYTES = BN * BK * 2;                        // one part of the x operand of a stage
     constexpr int STAGE_BYTES = W_TILES * WP * TILE_BYTES + XP * X_BYTES;  // [W hi (,W2 hi)][W lo (,W2 lo)][x hi][x lo]
     constexpr int STAGES = RING_BYTES / PER_SM / STAGE_BYTES;
@@ -172,7 +172,6 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             for (int xp = 0; xp < XP; ++xp) {
                 const int xr = tok0 + xp * (int)p.x_lo_row;
                 tma_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, xr, full);
-                if (X_TILES == 2) tma_load_2d(st + X_OFF + xp * X_BYTES + TILE_BYTES, &map_x, kx, xr + 128, full);  // rows 128..255: the next 16 groups of 8
             }
         }
     } else if (warp == 1) {

@@ -45,7 +45,7 @@ extern "C" int32_t vb_op_matmul(float* dst, const float* x, const void* w, const
     VB_REQUIRE(fmt >= VB_FMT_F32 && fmt <= VB_FMT_I8PC, "vb_op_matmul: unknown format %d", fmt);
     VB_REQUIRE(in_dim % 8 == 0 && fmt_shape_ok(fmt, in_dim), "vb_op_matmul: in_dim=%u not valid for format %d", in_dim, fmt);
     VB_REQUIRE(wmat_scale_bytes(fmt, out_dim, in_dim) == 0 || scales, "vb_op_matmul: format %d needs scales", fmt);
-    VB_REQUIRE((size_t)in_dim * 4 <= 200 * 1024, "vb_op_matmul: in_dim=%u exceeds the shared-memory staging limit", in_dim);
+    VB_REQUIRE((size_t)in_dim * 4 <= 200 * 1024, "vb_op_matmul: in_dim=%u exceeds 51200, the widest row of a context or an operation", in_dim);
     if (batch == 0 || out_dim == 0) return VB_OK;
     GemvArgs a;
     a.dst = dst; a.x = x;

@@ -6,7 +6,8 @@
 namespace vb {
 
 const char* last_error();
-// Opt every kernel into the dynamic shared memory it may ask for (once per device, before any capture).
+// Raises the shared-memory limits of the kernels that vb_gemv_fast.cu and vb_gemv_imma.cu launch (the others raise theirs at their
+// first launch on a device).
 cudaError_t kernels_init();
 cudaError_t gemv_init();
 

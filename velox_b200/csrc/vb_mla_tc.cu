@@ -574,7 +574,7 @@ cudaError_t mla_decode_tc(const LaunchCfg& lc, float* out, const float* q, const
     p.n_seq = batch; p.n_heads = n_heads; p.hbs = hbs; p.q_rows_per_seq = rows_per_seq;
     p.min_tiles = mla_min_tiles(split_tokens);
     p.direct = ((uintptr_t)out & 31) == 0 ? 1u : 0u;
-    p.cache_stride = cache_stride; p.scale = fmaxf(fabsf(scale), 1e-30f);  // the sign goes into q; 0 would turn masked scores into NaN
+    p.cache_stride = cache_stride; p.scale = scale == 0.0f ? 1e-30f : fabsf(scale);  // the sign goes into q; 0 would turn masked scores into NaN
     const uint64_t max_rows = mla_max_rows(max_ctx, split_tokens), runs = (mla_total_tiles(batch, hbs, max_ctx, split_tokens) + p.min_tiles - 1) / p.min_tiles;
     p.max_rows = max_rows < 0xFFFFFFC0ull ? (uint32_t)max_rows : 0xFFFFFFC0u;
     const uint32_t n8 = batch * rows_per_seq * (MT_LAT / 8);
