@@ -183,9 +183,9 @@ def test_norm_weights_at_any_float(vb):
 
 
 @pytest.mark.parametrize("fmt", ["f32", "f16", "bf16", "q4g32", "q4g64ref", "i8pc"])
-@pytest.mark.parametrize("in_dim,out_dim,batch", [(64, 9, 20), (576, 37, 7), (1088, 130, 17), (576, 4099, 8), (576, 4099, 9), (576, 4099, 13)])
+@pytest.mark.parametrize("in_dim,out_dim,batch", [(64, 9, 20), (576, 37, 7), (576, 600, 12), (576, 600, 13), (1088, 130, 17), (576, 4099, 8), (576, 4099, 9), (576, 4099, 13)])
 def test_canonical_matvec_passes(vb, oracle, fmt, in_dim, out_dim, batch):
-    """Rows of x in passes of two (all of them one wave of warps), four, and for fp32 eight; full and ragged last passes."""
+    """Rows of x in passes of one and two (all of them one wave of warps), four, and for fp32 eight; full and ragged last passes."""
     test_canonical_matvec(vb, oracle, fmt, in_dim, out_dim, batch)
 
 

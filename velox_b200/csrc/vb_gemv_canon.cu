@@ -365,16 +365,17 @@ cudaError_t launch_canon(const LaunchCfg& lc, const CanonArgs& a) {
     const uint32_t per = a.epilogue == EPI_SWIGLU ? GC_R / 2 : GC_R, groups = (a.rows + per - 1) / per, per_block = GC_WARPS / a.ks;
     return launch(lc, k_gemv_canon<FMT, NB, ALIGNED>, dim3((groups + per_block - 1) / per_block, (a.batch + NB - 1) / NB), dim3(GC_THREADS), 0, a);
 }
-// Rows of x per pass over the weights.  A matrix whose passes all run at once as one wave of warps gives each the fewest rows: what
-// the pass takes is its own latency, and the weights come from L2.  Else four rows to a pass: eight share the weights further but
+// Rows of x per pass over the weights.  A matrix whose passes all run at once as one wave of warps gives each the fewest rows, one or
+// two: what the pass takes is its own latency, and the weights come from L2 (576 x 576, 3 rows, fp32: 3.1 us in ones, 3.6 in twos, 4.4
+// in fours).  Else four rows to a pass: eight share the weights further but
 // hold 64 accumulator registers and spill (fp16 28672 x 4096, 16 rows: 252 us in eights, 248 in fours), which only fp32 with its
 // eight-byte pairs wins back, where the last pass is more than half full (8 rows 199 / 224 us, 12 rows 363 / 327, 16 rows 370 /
 // 429).  One step of the 135M shape, 5 / 9 / 15 / 32 rows, ms: fp32 1.38 / 1.73 / 1.69 / 2.22 with eights throughout, now
-// 0.91 / 1.14 / 1.36 / 2.11; q4 group-64 1.23 / 1.66 / 2.46 / 3.93, now 0.80 / 0.98 / 1.18 / 2.05.
+// 0.90 / 1.14 / 1.36 / 2.11; q4 group-64 1.23 / 1.66 / 2.46 / 3.93, now 0.79 / 0.98 / 1.18 / 2.05.
 template <int FMT>
 cudaError_t launch_canon_fmt(const LaunchCfg& lc, const CanonArgs& a, uint32_t warps) {
     if ((((uintptr_t)a.x | (uintptr_t)a.norm_w) & 15) != 0) return launch_canon<FMT, 1, false>(lc, a);
-    if (a.batch == 1) return launch_canon<FMT, 1, true>(lc, a);
+    if (a.batch == 1 || (a.batch > 2 && warps * a.batch <= GC_WAVE)) return launch_canon<FMT, 1, true>(lc, a);
     if (a.batch == 2 || warps * ((a.batch + 1) / 2) <= GC_WAVE) return launch_canon<FMT, 2, true>(lc, a);
     if constexpr (FMT == VB_FMT_F32)
         if ((a.batch - 1) % 8 >= 4 && warps * ((a.batch + 3) / 4) > GC_WAVE) return launch_canon<FMT, 8, true>(lc, a);
