@@ -352,7 +352,8 @@ int32_t vb_op_mla_absorbed(float* dst, const float* x, const float* w_norm, cons
  * reference's runtime implements only the single-head block above.  For sequence b and head h:
  *   out[b][h][:512] = sum_t softmax_t(scale * q[b][h][:576] . cache[b][t][:576]) * cache[b][t][:512],  t < ctx_len[b]
  * q fp32 [batch][n_heads][576] = [q_nope . W_uk (512) | q_rope (64)]; latent_cache bf16 [batch][cache_stride_rows][576] =
- * [c_kv | k_rope] per token; ctx_len on the device (a captured graph serves growing contexts).  Products run in bf16 on
+ * [c_kv | k_rope] per token; ctx_len on the device (a captured graph serves growing contexts; one
+ * beyond max_ctx ends with max_ctx's last whole slice).  Products run in bf16 on
  * the tensor cores with fp32 accumulation; the context is cut into slices of split_tokens rows (0 = 1024; the tcgen05 kernel: the shortest run of rows it gives a pair of blocks, 0 = 256) merged by a
  * second kernel.  scratch: vb_op_mla_decode_scratch_bytes, 16-byte aligned.  Default kernel: tcgen05.mma with S and O
  * in tensor memory, the latent tiles brought in by tiled TMA; vb_op_mla_set_path(0) selects the mma.sync kernel (process-wide;
