@@ -1,5 +1,7 @@
 """Engine behaviour at the edges of its contracts: a slot never leaves its KV reservation, reloaded weights
 reach every code path that keeps a derived copy."""
+import time
+
 import numpy as np
 import pytest
 
@@ -81,3 +83,53 @@ def test_reloaded_tensor_reaches_the_tensor_core_copies(spec):
     assert err <= LOGIT_TOL, "logits max-abs %g after a reload" % err
     assert np.array_equal(got, want)
     eng.close()
+
+
+@pytest.mark.parametrize("fmt,batch,prefill_rows", [(L.FMT_Q4G32, 1, 160), (L.FMT_Q4G32, 1, 64), (L.FMT_I8PC, 1, 2048), (L.FMT_F16, 16, 100), (L.FMT_I8PC, 16, 100)])
+def test_a_wait_that_ran_out_ends_what_is_enqueued_behind_it(fmt, batch, prefill_rows):
+    """The stop word that such a wait sets, set by hand: a prompt of one or several chunks (pairs of blocks, operands in tensor memory) and a
+    step of a batch (fp16 and int8 tensor-core products) start nothing and report a time-out at once; the context serves again afterwards."""
+    spec = SPEC.scaled(name="stop", weight_fmt=fmt, head_fmt=fmt, embed_fmt=L.FMT_F16)
+    eng = H.build_engine(spec, 5, 720, max_batch=batch)
+    eng.set_option("prefill_rows", prefill_rows)
+    prompt = H.prompt_tokens(spec, 5, 700)
+    eng.reserve(0, 716)
+    eng.prefill(prompt, 0)
+    want = eng.logits()
+    eng.decode(1)
+    want_step = eng.logits()
+    for what in ("prompt", "step"):
+        if what == "step" and batch == 1:
+            continue  # (nothing of a one-row step looks at the word)
+        eng.set_option("stop_word", 1)
+        t0 = time.monotonic()
+        with pytest.raises(L.VeloxError) as e:
+            if what == "prompt":
+                eng.prefill(prompt, 0)
+            else:
+                eng.set_state(0, int(eng.state(0)[0]), 700)
+                eng.decode(1)
+                eng.sync()
+        assert e.value.code == L.ERR_TIMEOUT and time.monotonic() - t0 < 1.0
+        eng.prefill(prompt, 0)
+        assert np.array_equal(eng.logits(), want)
+        eng.decode(1)
+        assert np.array_equal(eng.logits(), want_step)
+        eng.sync()
+    eng.close()
+
+
+def test_a_time_out_is_reported_to_its_own_context():
+    a, b = H.build_engine(SPEC, 5, 128), H.build_engine(SPEC, 6, 128)
+    prompt = H.prompt_tokens(SPEC, 5, 100)
+    for eng in (a, b):
+        eng.reserve(0, 128)
+    a.set_option("stop_word", 1)
+    b.prefill(prompt, 0)
+    b.sync()
+    with pytest.raises(L.VeloxError) as e:
+        a.prefill(prompt, 0)
+    assert e.value.code == L.ERR_TIMEOUT
+    b.sync()
+    a.close()
+    b.close()

@@ -101,6 +101,12 @@ __device__ __forceinline__ void load_row(const KVT* __restrict__ p, uint32_t lan
     }
 }
 
+// Bounded wait; one that runs out is reported and the block carries on.
+__device__ __forceinline__ bool attn_wait(const AttnArgs& a, uint32_t bar, uint32_t parity, uint32_t code) {
+    const bool there = wait_or_stop(bar, parity, a.stop);
+    if (!there) report_wait(a.err, a.stop, code);
+    return there;
+}
 __device__ __forceinline__ float bias_at(const void* w, int fmt, uint32_t i) {
     return fmt == VB_FMT_F16 ? __half2float(((const __half*)w)[i])
          : fmt == VB_FMT_BF16 ? __bfloat162float(((const __nv_bfloat16*)w)[i]) : ((const float*)w)[i];
@@ -550,7 +556,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
             for (uint32_t c = 0; c < n_ch; ++c) {
                 const uint32_t c0 = t_lo + c * CH, buf = c & 1, t0 = c0 + tok0;
                 if (warp >= CH / 16 || t0 >= t_hi) break;
-                if (!mbar_wait(smem_u32(&kv_bar[buf * ATTN_WARPS + warp]), (c >> 1) & 1) && a.err) atomicOr(a.err, 0x400u);
+                attn_wait(a, smem_u32(&kv_bar[buf * ATTN_WARPS + warp]), (c >> 1) & 1, 0x400u);
                 KVT* kb = kv_s + (size_t)buf * 2 * CH * RS;
                 // the copies moved a whole KV block: rows past the context's end hold whatever the pool held (they are
                 // multiplied with probability 0 and must be numbers), and the new token's row is older than this step
@@ -631,7 +637,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
         } else
         for (uint32_t c = 0; c < n_ch; ++c) {
             const uint32_t c0 = t_lo + c * CH, buf = c & 1;
-            if (!mbar_wait(smem_u32(&kv_bar[buf]), (c >> 1) & 1) && a.err) atomicOr(a.err, 0x400u);
+            attn_wait(a, smem_u32(&kv_bar[buf]), (c >> 1) & 1, 0x400u);
             KVT* kb = kv_s + (size_t)buf * 2 * CH * RS;
             const uint32_t c_hi = min(t_hi, c0 + CH);
             if constexpr (MMA) {
@@ -679,8 +685,8 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
                 if (warp < 4) {
                     // ---- softmax: thread = token row = tensor-memory lane ------------------------------------------------------
                     const uint32_t lane_addr = (warp * 32u) << 16, tok = threadIdx.x;
-                    const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(s_bar, c & 1));
-                    if (!ok && a.err && lane == 0) atomicOr(a.err, 0x800u);
+                    attn_wait(a, s_bar, c & 1, 0x800u);
+                    __syncwarp();
                     at_fence_after();
                     float sv[16];
                     at_ld16(tmem + lane_addr, sv);
@@ -739,7 +745,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
                     at_commit(o_bar);
                 }
                 // the staging buffer, the P operand and S^T are free again once that product is done
-                if (!mbar_wait(o_bar, c & 1) && a.err) atomicOr(a.err, 0x1000u);
+                attn_wait(a, o_bar, c & 1, 0x1000u);
                 at_fence_after();
             } else
             for (uint32_t t0 = c0 + warp * TCH; t0 < c_hi; t0 += ATTN_WARPS * TCH) {
@@ -920,11 +926,11 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) k_attn_split(const __grid_con
     };
     if (per_d % 4 == 0) push(std::integral_constant<int, 4>{});
     else push(std::integral_constant<int, 1>{});
-    // bounded like the copies' waits; the peers' own waits come first, so it gets twice their limit
+    // bounded like the copies' waits; the peers' own waits come first (one second, after that 10 ms each), so it gets twice their limit
     if (threadIdx.x < ((ng * per_d + 31) & ~31u)) {
-        bool here = mbar_wait(bar_a, 0) || mbar_wait(bar_a, 0);
+        const bool here = mbar_wait(bar_a, 0) || mbar_wait(bar_a, 0);
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        if (!here && a.err) atomicOr(a.err, 0x2000u);
+        if (!here) report_wait(a.err, a.stop, 0x2000u);
         for (uint32_t i = threadIdx.x; here && i < ng * per_d; i += blockDim.x) {
             const uint32_t g = i / per_d, dd = i % per_d, d = d_lo + dd;
             if (d < d_hi) {

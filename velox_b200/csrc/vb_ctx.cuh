@@ -50,7 +50,8 @@ struct vb_ctx {
     bool tp_fused_reduce = true;          // ... and gather the peers' copies of their own rows: no exchange kernel at all
     uint32_t ring_role[4] = {0, 0, 0, 0};   // per product (qkv, o, gate/up, down): 0 = gemv_ring
     uint32_t gemv_ring = 4, head_ring = 4;  // weight ring depth of the int4 kernel for the layers / the head (GemvArgs::max_ring)
-    uint32_t* err_word = nullptr;         // device word that bounded waits set when they run out
+    // words that a bounded wait sets when it runs out: one in mapped host memory, read without a copy, one in device memory (LaunchCfg)
+    uint32_t *err_word = nullptr, *err_host = nullptr, *stop_word = nullptr;
     float* partial = nullptr;             // [max_batch][d_model] row-parallel partial sums (all-reduced in place)
     unsigned char* tp_pair = nullptr;     // [max_batch] (value, index) of this rank's best logit
     unsigned char* tp_pairs = nullptr;    // [tp_size][max_batch] gathered
@@ -178,6 +179,7 @@ bool takes_i8(const vb_ctx* c, const StepIO& io, const GemvArgs& a);
 void give_i8_ws(vb_ctx* c, StepIO& io);
 cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepIO& io);
 int32_t check_ready(vb_ctx* c, const char* who);
+int32_t check_device_error(vb_ctx* c);
 // [rows][cols] of this rank's shard of a role, and its storage format (false: the model has no such tensor)
 bool role_shape(const vb_ctx* c, int role, uint32_t* rows, uint32_t* cols, int32_t* fmt);
 // vb_gguf.cu

@@ -208,6 +208,7 @@ LaunchCfg lcfg(vb_ctx* c, bool pdl) {
     lc.stream = c->stream;
     lc.pdl = pdl && c->use_pdl;
     lc.counter = &c->launches;
+    lc.err = c->err_word; lc.stop = c->stop_word;
     return lc;
 }
 
@@ -565,7 +566,7 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
         if (c->kv_map_ok) { a.kv_map = c->kv_map; a.kv_map_row0 = (uint32_t)((uint64_t)l * (c->kv_layer_elems / d.head_dim)); }
         a.state = state; a.Hq = c->hq; a.Hkv = c->hkv; a.D = d.head_dim; a.batch = B;
         a.max_splits = c->n_splits ? c->n_splits : pick_attn_splits(c, B); a.tokens_per_split = c->tokens_per_split; a.scratch = c->attn_scratch;
-        a.trace = next_trace(); a.err = c->err_word;
+        a.trace = next_trace(); a.err = c->err_word; a.stop = c->stop_word;
         if (io.causal_chunk && c->prefill_flash && attention_prefill_supported(c->hq, c->hkv, d.head_dim))
             VB_TRY(attention_prefill(lcfg(c, true), io.attn_out, io.q, kv_layer, io.block_table, io.first, B, c->hq, c->hkv, d.head_dim, d.kv_block_tokens, io.split_attn));
         else
@@ -658,6 +659,26 @@ int32_t check_ready(vb_ctx* c, const char* who) {
         return VB_ERR_STATE;
     }
     return VB_OK;
+}
+
+// Reads (and clears) what bounded device-side waits of this context, and of launches without a context, reported when they ran out.
+// Callers have synchronised the stream: the mapped words are read in place.
+int32_t check_device_error(vb_ctx* c) {
+    uint32_t *own = c->err_host, *process = nullptr;
+    VB_CUDA(fast_error_word_host(&process));
+    uint32_t v = 0;
+    for (uint32_t* w : {own, process}) {
+        const uint32_t seen = *reinterpret_cast<volatile uint32_t*>(w);
+        if (seen) *reinterpret_cast<volatile uint32_t*>(w) = 0;
+        v |= seen;
+    }
+    if (v == 0) return VB_OK;
+    VB_CUDA(cudaMemsetAsync(c->stop_word, 0, 4, c->stream));
+    // a split-K product that gave up leaves its tile counters between 0 and the split count: start them over
+    if (c->tc_ws) VB_CUDA(cudaMemsetAsync(tc_ws_aligned(c), 0, gemm_tc_workspace_zero_bytes(), c->stream));
+    if (c->i8_ws) VB_CUDA(cudaMemsetAsync((void*)(((uintptr_t)c->i8_ws + 1023) & ~(uintptr_t)1023), 0, gemm_i8_workspace_zero_bytes(), c->stream));
+    set_error("a bounded device-side wait expired (code 0x%x): results of the last launches are invalid", v);
+    return VB_ERR_TIMEOUT;
 }
 
 }  // namespace vb
@@ -753,9 +774,14 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
     VB_CREATE_CUDA(cudaMemsetAsync(c->state, 0, d.max_batch * sizeof(SeqState), c->stream));
     VB_CREATE_CUDA(cudaMemsetAsync(c->pf_state, 0, d.max_batch * sizeof(SeqState), c->stream));
     c->state_host.assign(d.max_batch, SeqState{0, 0, 0, 0});
-    VB_CREATE_CUDA(cudaHostAlloc((void**)&c->ring_host, (size_t)d.max_batch * RING_SLOTS * 4 + 4, cudaHostAllocMapped));  // (+ a word of the loader's)
+    VB_CREATE_CUDA(cudaHostAlloc((void**)&c->ring_host, (size_t)d.max_batch * RING_SLOTS * 4 + 8, cudaHostAllocMapped));  // (+ a word of the loader's, the error word)
     memset(c->ring_host, 0xFF, (size_t)d.max_batch * RING_SLOTS * 4);
     VB_CREATE_CUDA(cudaHostGetDevicePointer((void**)&c->ring_dev, c->ring_host, 0));
+    c->err_host = c->ring_host + (size_t)d.max_batch * RING_SLOTS + 1;
+    c->err_word = c->ring_dev + (size_t)d.max_batch * RING_SLOTS + 1;
+    *c->err_host = 0;
+    VB_CREATE_TRY(dev_alloc(&c->stop_word, 1));
+    VB_CREATE_CUDA(cudaMemsetAsync(c->stop_word, 0, 4, c->stream));
     const uint64_t B = d.max_batch;
     VB_CREATE_TRY(dev_alloc(&c->hidden, B * d.d_model));
     VB_CREATE_TRY(dev_alloc(&c->qkv, B * c->qkv_rows));
@@ -783,7 +809,6 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
         VB_CREATE_CUDA(cudaMemcpyAsync(c->rope_inv_freq, f.data(), f.size() * 4, cudaMemcpyHostToDevice, c->stream));
         VB_CREATE_CUDA(cudaStreamSynchronize(c->stream));
     }
-    VB_CREATE_CUDA(fast_error_word(&c->err_word));
     VB_CREATE_CUDA(cudaStreamSynchronize(c->stream));
 #undef VB_CREATE_TRY
 #undef VB_CREATE_CUDA
@@ -804,7 +829,7 @@ int32_t vb_destroy(vb_ctx* c) {
     void* frees[] = {c->arena, c->kv_pool, c->block_table_dev, c->state, c->pf_state, c->pf_tokens, c->hidden, c->qkv, c->q,
                      c->attn_out, c->act, c->logits, c->attn_scratch, c->cand_v, c->cand_i, c->rope_inv_freq, c->trace, c->partial, c->tp_pair, c->tp_pairs,
                      c->pfc_state, c->pfc_table, c->pfc_hidden, c->pfc_qkv, c->pfc_q, c->pfc_attn, c->pfc_act, c->tc_ws, c->f16_pool, c->i8_tiles_pool, c->sample_probs,
-                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws, c->frag_ws, c->ts_ws};
+                     c->spec_logits, c->spec_cand_v, c->spec_cand_i, c->spec_tokens, c->i8_ws, c->frag_ws, c->ts_ws, c->stop_word};
     for (void* p : frees) if (p) cudaFree(p);
     if (c->ring_host) cudaFreeHost(c->ring_host);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -1145,11 +1170,22 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
         io.split_attn = !tc_ok;
         // the last token always takes the per-token path below (it produces the logits); the last chunk may be ragged (token by
         // token instead, a 120-token prompt of the 72B shape spent 66 ms on its last 8)
+        uint32_t chunk = 0;
         while (done + 1 < n_tokens) {
             const uint32_t n = std::min(P, n_tokens - 1 - done);
             io.B = n; io.first = done;
+            // A wait that ran out ends the prompt here: the chunk before the last one is through before another is enqueued.
+            if (chunk >= 2) {
+                VB_CUDA(cudaEventSynchronize(chunk & 1 ? c->ev1 : c->ev0));
+                if (*reinterpret_cast<volatile uint32_t*>(c->err_host)) {
+                    VB_CUDA(cudaStreamSynchronize(c->stream));
+                    return check_device_error(c);
+                }
+            }
             VB_CUDA(launch(lcfg(c, false), k_set_chunk_state, dim3((n + 127) / 128), dim3(128), 0, c->pfc_state, (const uint32_t*)c->pf_tokens, done, n, n));
             VB_CUDA(enqueue_step(c, c->pfc_state, false, io));
+            VB_CUDA(cudaEventRecord(chunk & 1 ? c->ev1 : c->ev0, c->stream));
+            ++chunk;
             done += n;
         }
     }
@@ -1162,6 +1198,10 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // hand the slot over to the decode state: first generated token at position n_tokens
     VB_CUDA(cudaMemcpyAsync(c->state + slot, c->pf_state + slot, sizeof(SeqState), cudaMemcpyDeviceToDevice, c->stream));
     VB_CUDA(cudaStreamSynchronize(c->stream));
+    if (*reinterpret_cast<volatile uint32_t*>(c->err_host)) {
+        vb_seq_set(c, slot, 0, 0, 0);
+        return check_device_error(c);
+    }
     c->pos_hi[slot] = n_tokens;
     c->maybe_active[slot] = 1;  // (a prompt that fills the reservation leaves the slot inactive on the device)
     return VB_OK;
@@ -1251,23 +1291,6 @@ int32_t vb_decode_run(vb_ctx* c, uint32_t n_steps, float* elapsed_ms) {
         VB_CUDA(cudaEventRecord(c->ev1, c->stream));
         VB_CUDA(cudaEventSynchronize(c->ev1));
         VB_CUDA(cudaEventElapsedTime(elapsed_ms, c->ev0, c->ev1));
-    }
-    return VB_OK;
-}
-
-// Reads (and clears) the device error word that bounded device-side waits set when they expire.
-static int32_t check_device_error(vb_ctx* c) {
-    // callers have synchronised the stream: the mapped word is read in place
-    uint32_t* w = nullptr;
-    VB_CUDA(fast_error_word_host(&w));
-    const uint32_t v = *reinterpret_cast<volatile uint32_t*>(w);
-    if (v != 0) {
-        *reinterpret_cast<volatile uint32_t*>(w) = 0;
-        // a split-K product that gave up leaves its tile counters between 0 and the split count: start them over
-        if (c->tc_ws) cudaMemsetAsync(tc_ws_aligned(c), 0, gemm_tc_workspace_zero_bytes(), c->stream);
-        if (c->i8_ws) cudaMemsetAsync((void*)(((uintptr_t)c->i8_ws + 1023) & ~(uintptr_t)1023), 0, gemm_i8_workspace_zero_bytes(), c->stream);
-        set_error("a bounded device-side wait expired (code 0x%x): results of the last launches are invalid", v);
-        return VB_ERR_TIMEOUT;
     }
     return VB_OK;
 }
@@ -1463,6 +1486,13 @@ int32_t vb_set_option(vb_ctx* c, const char* name, int64_t value) {
         }
         c->links_standin = true;
         c->links_open = true;
+        return VB_OK;
+    }
+    if (!strcmp(name, "stop_word")) {
+        // Diagnostic: what a wait that ran out leaves behind (1), without a wait that runs out; 0 takes it back
+        VB_CUDA(cudaSetDevice(c->device));
+        VB_CUDA(cudaMemsetAsync(c->stop_word, value != 0, 4, c->stream));
+        VB_CUDA(cudaStreamSynchronize(c->stream));
         return VB_OK;
     }
     if (!strcmp(name, "gemv_spread")) { imma_spread = value != 0; return VB_OK; }

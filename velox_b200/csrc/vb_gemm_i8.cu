@@ -65,18 +65,6 @@ __device__ __forceinline__ void tmem_ld32i(uint32_t taddr, int r[32]) {
                  : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ bool wait_abort(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 128; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1u; return false; }
-    }
-}
-
 struct I8Params {
     float* dst;                 // [n_rows][dst_stride], column offset applied
     const __half* row_scale;    // [out_dim] weight row scales
@@ -85,7 +73,7 @@ struct I8Params {
     const SeqState* state;
     uint32_t out_dim, n_rows, K, dst_stride;
     int epilogue;
-    uint32_t* err;
+    uint32_t *err, *stop;
     float* part;                // [split][tile][32 cols][128 lanes] fp32 partial tiles
     uint32_t* counters;         // [tile], zero between launches
     uint32_t stages;
@@ -122,7 +110,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(bars + s * 8, 1); mbar_init(bars + (STAGES + s) * 8, 1); }
         mbar_init(bar_accum, 1);
-        *abort_flag = 0u;
+        *abort_flag = stop_set(p.stop) ? 1u : 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -134,8 +122,9 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
+    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
 
-    if (warp == 0) {
+    if (warp == 0 && go) {
       if (elect_one()) {
         // weights do not depend on the kernel before this one: the whole ring of weight tiles is requested before the
         // dependency wait, the planes of x (written by the conversion kernel in front) after it
@@ -159,7 +148,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         for (int kb = pre; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!wait_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag)) break;
+            if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag, p.stop)) break;
             const uint32_t full = bars + s * 8, st = base + s * STAGE_BYTES;
             mbar_expect_tx(full, STAGE_BYTES);
             const int kx = (kb_first + kb) * I8_BK;
@@ -174,12 +163,12 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             tma_2d(st + W_TILES * I8_W_BYTES, &map_x, kx, 0, full);
         }
       }
-    } else if (warp == 1) {
+    } else if (warp == 1 && go) {
         // the warp waits together, an elected lane issues (vb_tma.cuh)
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!__all_sync(0xFFFFFFFFu, wait_abort(bars + s * 8, ph, abort_flag))) break;
+            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
             fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
@@ -209,7 +198,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, live);
         if (lane == 0) s_live_mask = m;
     }
-    const bool ok = wait_abort(bar_accum, 0u, abort_flag);
+    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
     fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     if (good) {
@@ -280,9 +269,9 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             }
         }
     } else {
-        if (threadIdx.x == 0 && p.err) atomicOr(p.err, 0x80u);
+        if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x80u);
         const long long t0 = clock64();
-        while (clock64() - t0 < 20000000LL) { }
+        while (go && clock64() - t0 < 20000000LL) { }
     }
     fence_before();
     __syncthreads();
@@ -595,8 +584,7 @@ static cudaError_t gemm_i8_rows(const LaunchCfg& lc, const GemvArgs& a, void* wo
     p.out_dim = out_dim; p.n_rows = n_rows; p.K = K;
     p.dst_stride = a.dst_stride ? a.dst_stride : out_dim;
     p.epilogue = a.epilogue;
-    p.err = nullptr;
-    fast_error_word(&p.err);
+    error_words(lc, &p.err, &p.stop);
     p.counters = reinterpret_cast<uint32_t*>(ws);
     p.part = reinterpret_cast<float*>(ws + I8_COUNTER_BYTES);
     const uint32_t tiles = (out_dim + I8_BM - 1) / I8_BM, nk = (K + I8_BK - 1) / I8_BK;

@@ -70,19 +70,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t r[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Bounded wait that also gives up as soon as another thread of the block has given up.
-__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 128; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1u; return false; }
-    }
-}
-
 struct GemmParams {
     float* dst;                // [n_rows][dst_stride], column offset already applied
     const __half* row_scale;   // != null: accumulator of weight row o is multiplied by row_scale[o] (int8 per channel)
@@ -90,7 +77,7 @@ struct GemmParams {
     const SeqState* state;     // != null: rows of inactive slots are not written
     uint32_t out_dim, n_rows, K, dst_stride;
     int epilogue;
-    uint32_t* err;
+    uint32_t *err, *stop;
     // split K (gridDim.z > 1): every block stores its fp32 partial tile, the last block to arrive at the tile's
     // counter sums the partials in split order (the same bits whoever is last) and runs the epilogue
     float* part;          // [split][tile][BN / 32][32][128]
@@ -130,7 +117,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(bars + s * 8, 1); mbar_init(bars + (STAGES + s) * 8, 1); }
         mbar_init(bar_accum, 1);
-        *abort_flag = 0u;
+        *abort_flag = stop_set(p.stop) ? 1u : 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -142,17 +129,18 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
 
     pdl_wait();  // x (and converted weights) come from the kernels before this one
     pdl_launch_dependents();
 
-    if (warp == 0) {
+    if (warp == 0 && go) {
         // ---- producer: TMA copies into the ring ----
         if (elect_one())
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag)) break;
+            if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag, p.stop)) break;
             const uint32_t full = bars + s * 8, st = base + s * STAGE_BYTES;
             mbar_expect_tx(full, STAGE_BYTES);
             const int kx = (kb_first + kb) * BK;
@@ -160,12 +148,12 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             if (DUAL) tma_load_2d(st + TILE_BYTES, &map_w2, kx, row0, full);
             tma_load_2d(st + X_OFF, &map_x, kx, tok0, full);
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 && go) {
         // ---- tensor-core issue: the warp waits together, an elected lane issues (see vb_tma.cuh) ----
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag))) break;
+            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
             tc_fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
@@ -185,7 +173,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncwarp();
 
     // ---- epilogue: warp w owns tensor-memory lanes 32w..32w+31 = weight rows row0 + 32w + lane ----
-    const bool ok = wait_or_abort(bar_accum, 0u, abort_flag);
+    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
     tc_fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     if (good) {
@@ -267,10 +255,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         }
         }
     } else {
-        if (threadIdx.x == 0 && p.err) atomicOr(p.err, 0x40u);
+        if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x40u);
         // let copies and products that are still in flight land before the memory they use is given back
         const long long t0 = clock64();
-        while (clock64() - t0 < 20000000LL) { }
+        while (go && clock64() - t0 < 20000000LL) { }
     }
     tc_fence_before();
     __syncthreads();
@@ -338,7 +326,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2 * STAGES; ++s) mbar_init(bars + s * 8, 1);
         mbar_init(bar_accum, 1);
-        *abort_flag = 0u;
+        *abort_flag = stop_set(p.stop) ? 1u : 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -351,18 +339,19 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     cluster_sync_all();  // both blocks' barriers and tensor memory are there
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
 
     pdl_wait();  // x (and converted weights) come from the kernels before this one
     pdl_launch_dependents();
 
-    if (warp == 0) {
+    if (warp == 0 && go) {
         // ---- producer: this block's copies, counted by the first block ----
         if (elect_one()) {
             const uint32_t full0 = pair_addr(bars, 0);
             for (int kb = 0; kb < nk; ++kb) {
                 const int s = kb % STAGES;
                 const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-                if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag)) break;
+                if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag, p.stop)) break;
                 const uint32_t full = full0 + s * 8, st = base + s * STAGE_BYTES;
                 if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * STAGE_BYTES);
                 const int kx = kb * BK;
@@ -376,12 +365,12 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
                 for (int xp = 0; xp < XP; ++xp) pair_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, tok0 + (int)rank * (BN / 2) + xp * (int)p.x_lo_row, full);
             }
         }
-    } else if (warp == 1 && rank == 0) {
+    } else if (warp == 1 && rank == 0 && go) {
         // ---- tensor-core issue for both blocks ----
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag))) break;
+            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
             tc_fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
@@ -408,7 +397,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     __syncwarp();
 
     // ---- epilogue: warps w and w + 4 own tensor-memory lanes 32 (w % 4) .. + 31 = weight rows, half of the columns each ----
-    const bool ok = wait_or_abort(bar_accum, 0u, abort_flag);
+    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
     tc_fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     if (good) {
@@ -451,10 +440,10 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
             }
         }
     } else {
-        if (threadIdx.x == 0 && p.err) atomicOr(p.err, 0x40u);
+        if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x40u);
         // let copies and products that are still in flight land before the memory they use is given back
         const long long t0 = clock64();
-        while (clock64() - t0 < 20000000LL) { }
+        while (go && clock64() - t0 < 20000000LL) { }
     }
     tc_fence_before();
     __syncthreads();
@@ -732,8 +721,7 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
     p.out_dim = out_dim; p.n_rows = n_rows; p.K = K;
     p.dst_stride = a.dst_stride ? a.dst_stride : out_dim;
     p.epilogue = a.epilogue;
-    p.err = nullptr;
-    fast_error_word(&p.err);
+    error_words(lc, &p.err, &p.stop);
     p.counters = reinterpret_cast<uint32_t*>(workspace);
     p.part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(workspace) + WS_COUNTER_BYTES);
     p.x_lo_row = (uint32_t)rows_pad;

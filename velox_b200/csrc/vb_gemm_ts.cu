@@ -70,7 +70,7 @@ struct TsParams {
     const SeqState* state;
     uint32_t rows, K, n_rows, dst_stride, x_lo_row, splits;  // rows of dst; x_lo_row: first row of the lo parts in the x map
     int epilogue;
-    uint32_t* err;
+    uint32_t *err, *stop;
     unsigned long long* trace;
 };
 
@@ -99,19 +99,8 @@ __device__ __forceinline__ void ts_ld16(uint32_t taddr, float (&r)[16]) {
                    "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]) : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ bool ts_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 128; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1u; return false; }
-    }
-}
-__device__ __forceinline__ bool ts_warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    return __all_sync(0xFFFFFFFFu, ts_wait(bar, parity, abort_flag));
+__device__ __forceinline__ bool ts_warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, const uint32_t* stop) {
+    return __all_sync(0xFFFFFFFFu, wait_or_abort(bar, parity, abort_flag, stop));
 }
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
@@ -185,7 +174,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     trace_mark(p.trace, 0);
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_AFULL && i < B_AEMPTY ? 4 : 1);
-        *abort_flag = 0u;
+        *abort_flag = stop_set(p.stop) ? 1u : 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -196,7 +185,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     // this block's part of K, in units
     const uint32_t n_units_all = p.K / F::unit, u0 = (uint32_t)((uint64_t)n_units_all * split / S), n_units = (uint32_t)((uint64_t)n_units_all * (split + 1) / S) - u0;
     constexpr int SPU = F::unit / 64;  // A stages per unit
-    const uint32_t n_st = n_units * SPU;
+    uint32_t n_st = n_units * SPU;
 
     // ---- dequantising warps: where this thread's weight row lies; the first units are requested before the dependency wait ----
     const uint32_t lg = warp & 3, row = lg * 32 + lane;  // tensor-memory lanes 32 * (warp % 4) .. + 31
@@ -233,6 +222,8 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     __syncthreads();
     ts_fence_after();
     const uint32_t tmem = *tmem_slot, tm_a = tmem + P::d_cols;
+    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
+    if (!go) n_st = 0;
     pdl_wait();
     pdl_launch_dependents();
     trace_mark(p.trace, 1);
@@ -242,7 +233,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         if (elect_one()) {
             for (uint32_t i = 0; i < n_st; ++i) {
                 const uint32_t s = i % XS;
-                if (i >= XS && !ts_wait(bar(B_XEMPTY + s), (i / XS + 1) & 1, abort_flag)) break;
+                if (i >= XS && !wait_or_abort(bar(B_XEMPTY + s), (i / XS + 1) & 1, abort_flag, p.stop)) break;
                 mbar_expect_tx(bar(B_XFULL + s), P::x_stage);
                 const int kx = (int)(u0 * F::unit + i * 64), y = (int)(blockIdx.x * NT);
                 const uint32_t st = base + s * P::x_stage;
@@ -257,7 +248,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         // ---- tensor-core issue ----
         for (uint32_t i = 0; i < n_st; ++i) {
             const uint32_t xs = i % XS, as = i % AS;
-            if (!ts_warp_wait(bar(B_XFULL + xs), (i / XS) & 1, abort_flag) || !ts_warp_wait(bar(B_AFULL + as), (i / AS) & 1, abort_flag)) break;
+            if (!ts_warp_wait(bar(B_XFULL + xs), (i / XS) & 1, abort_flag, p.stop) || !ts_warp_wait(bar(B_AFULL + as), (i / AS) & 1, abort_flag, p.stop)) break;
             ts_fence_after();
             if (elect_one()) {
                 const uint64_t bh = ts_desc(base + xs * P::x_stage), bl = ts_desc(base + xs * P::x_stage + NT * 128);
@@ -278,7 +269,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         // ---- weights -> tensor memory ----
         const uint32_t lane_addr = (lg * 32u) << 16;
         uint32_t i = 0;
-        bool ok = true;
+        bool ok = go;
         for (uint32_t ub = 0; ub < n_units && ok; ub += F::depth) {
 #pragma unroll
             for (int d = 0; d < F::depth; ++d) {
@@ -287,7 +278,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
 #pragma unroll
                     for (int half = 0; half < SPU; ++half) {
                         const uint32_t as = i % AS;
-                        if (i >= AS) ok = ts_warp_wait(bar(B_AEMPTY + as), (i / AS + 1) & 1, abort_flag);
+                        if (i >= AS) ok = ts_warp_wait(bar(B_AEMPTY + as), (i / AS + 1) & 1, abort_flag, p.stop);
                         if (!ok) break;
                         ts_fence_after();
                         ts_expand<FMT>(raw[d], half, (row & 8) != 0, hi[half], lo);
@@ -306,7 +297,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     }
 
     // ---- epilogue: lane = weight row ----
-    const bool ok = n_st == 0 || ts_wait(bar(B_ACC), 0u, abort_flag);
+    const bool ok = n_st == 0 || wait_or_abort(bar(B_ACC), 0u, abort_flag, p.stop);
     ts_fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     const uint32_t o = swiglu ? tile * 64 + (row >> 4) * 8 + (row & 7) : tile * 128 + row;
@@ -384,10 +375,10 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         }
     }
     if (!good) {
-        if (threadIdx.x == 0 && p.err) atomicOr(p.err, 0x100u);
+        if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x100u);
         // let copies and products that are still in flight land before the memory they use is given back
         const long long c0 = clock64();
-        while (clock64() - c0 < 20000000LL) { }
+        while (go && clock64() - c0 < 20000000LL) { }
     }
     ts_fence_before();
     __syncthreads();
@@ -572,7 +563,7 @@ cudaError_t gemm_ts(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
     p.rows = a.w.rows; p.K = K; p.n_rows = n_rows; p.dst_stride = a.dst_stride ? a.dst_stride : a.w.rows; p.x_lo_row = pad;
     p.epilogue = a.epilogue;
     p.trace = a.trace;
-    fast_error_word(&p.err);
+    error_words(lc, &p.err, &p.stop);
     const uint32_t row_tiles = (a.w.rows * (dual ? 2 : 1) + 127) / 128;
     return q4 ? ts_launch_nt<VB_FMT_Q4G32>(lc, map, p, nt, row_tiles) : ts_launch_nt<VB_FMT_I8PC>(lc, map, p, nt, row_tiles);
 }

@@ -665,8 +665,8 @@ cudaError_t gemv_fast(const LaunchCfg& lc, const GemvArgs& a, bool* handled) {
             size_t ns = ((size_t)TMA_MAX_SMEM - fixed) / TMA_STAGE_BYTES;
             if (ns > TMA_MAX_STAGES) ns = TMA_MAX_STAGES;
             f.n_stages = (uint32_t)ns;
-            cudaError_t e = err_word(&f.err, nullptr);
-            if (e != cudaSuccess) return e;
+            f.err = lc.err;
+            if (const cudaError_t e = lc.err ? cudaSuccess : err_word(&f.err, nullptr)) return e;
             *handled = true;
             const size_t tsmem = fixed + ns * TMA_STAGE_BYTES;
             const dim3 tgrid(n_tiles < 2u * n_sm ? n_tiles : 2u * n_sm);

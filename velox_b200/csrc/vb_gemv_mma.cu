@@ -87,7 +87,7 @@ struct MmArgs {
     const float* x;               // rows of x and the norm's weights, where a product converts them itself
     const void* norm_w; int norm_fmt; float eps;
     const unsigned char* xf;      // [weight blocks of K] x { [frags][T][32 lanes] uint4, q4: [sums][T][8] floats }
-    uint32_t* err;
+    uint32_t *err, *stop;
     const float* unscale;         // [rows of x]
     float* dst;
     const SeqState* state;
@@ -135,11 +135,8 @@ __device__ __forceinline__ void nibbles_normal(uint32_t (&A)[8], uint32_t u, uin
 }
 
 // Bounded wait (vb_tma.cuh); one that runs out is reported and the block carries on with what is there.
-__device__ __forceinline__ void mm_wait(uint32_t bar, uint32_t parity, uint32_t* err) {
-    if (mbar_try_wait(bar, parity)) return;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 2000000000LL) { atomicOr(err, 0x80u); return; }
+__device__ __forceinline__ void mm_wait(uint32_t bar, uint32_t parity, uint32_t* err, uint32_t* stop) {
+    if (!wait_or_stop(bar, parity, stop)) report_wait(err, stop, 0x200u);
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
@@ -294,11 +291,11 @@ __global__ void __launch_bounds__(MmShape<FMT, T>::warps * 32, MmShape<FMT, T>::
         // thread 0 refills the slot before this one once every warp has left it
         const uint32_t gone = phase * MM_SLOTS + at;  // slots finished so far
         if (threadIdx.x == 0 && gone > 0 && gone - 1 + MM_SLOTS < n_slots) {
-            mm_wait(empty + 8 * ((gone - 1) % MM_SLOTS), ((gone - 1) / MM_SLOTS) & 1u, a.err);
+            mm_wait(empty + 8 * ((gone - 1) % MM_SLOTS), ((gone - 1) / MM_SLOTS) & 1u, a.err, a.stop);
             fill(gone - 1 + MM_SLOTS);
         }
         __syncwarp();
-        mm_wait(full + 8 * at, phase & 1u, a.err);
+        mm_wait(full + 8 * at, phase & 1u, a.err, a.stop);
 #pragma unroll
         for (int q = 0; q < MM_SLOT_BLKS; ++q) {
             if (blk + q < n_kb) {
@@ -620,15 +617,15 @@ __global__ void __launch_bounds__(MrShape<FMT, T>::threads, 1) k_gemv_mma_res(co
 #pragma unroll 1
         for (uint32_t ch = 0; ch < (RES ? left : n_ch); ++ch) {
             if constexpr (RES) {
-                if (X == MR_RES && r == 0) mm_wait(full + 8 * ch, 0, a.err);
+                if (X == MR_RES && r == 0) mm_wait(full + 8 * ch, 0, a.err, a.stop);
             } else {
                 const uint32_t slot = q % P::slots;
                 if (q > 0 && q - 1 + P::slots < n_fill && wid == q % (P::groups * P::warps) && lane == 0) {
-                    mm_wait(empty + 8 * ((q - 1) % P::slots), ((q - 1) / P::slots) & 1u, a.err);
+                    mm_wait(empty + 8 * ((q - 1) % P::slots), ((q - 1) / P::slots) & 1u, a.err, a.stop);
                     fill(q - 1 + P::slots);
                 }
                 __syncwarp();
-                mm_wait(full + 8 * slot, (q / P::slots) & 1u, a.err);
+                mm_wait(full + 8 * slot, (q / P::slots) & 1u, a.err, a.stop);
                 x_at = slot * P::slot;
             }
             if (RES || ch < left) {
@@ -866,8 +863,7 @@ cudaError_t gemv_mma(const LaunchCfg& lc, const GemvArgs& g, bool* handled) {
     } else {
         return cudaSuccess;
     }
-    a.err = nullptr;
-    fast_error_word(&a.err);
+    error_words(lc, &a.err, &a.stop);
     a.rows = g.w.rows; a.K = K; a.epilogue = g.epilogue; a.trace = g.trace;
     a.dst_stride = g.dst_stride ? g.dst_stride : g.w.rows; a.dst_offset = g.dst_offset;
     XfArgs f;

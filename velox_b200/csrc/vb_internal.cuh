@@ -114,6 +114,9 @@ struct LaunchCfg {
     cudaStream_t stream = nullptr;
     bool pdl = false;          // launch with programmatic stream serialization
     uint64_t* counter = nullptr;
+    // where a bounded wait that ran out is reported (mapped host memory; null: the process's word, fast_error_word) and the context's
+    // stop word (device memory; may be null), set at the same time: kernels that see it start nothing and wait for nothing
+    uint32_t *err = nullptr, *stop = nullptr;
 };
 
 template <typename... KArgs, typename... Args>

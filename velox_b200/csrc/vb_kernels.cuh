@@ -109,6 +109,12 @@ extern bool attn_use_mma;
 extern bool attn_use_tcgen05;
 cudaError_t fast_error_word(uint32_t** out);
 cudaError_t fast_error_word_host(uint32_t** out);
+// where a launch's bounded waits report (LaunchCfg)
+inline void error_words(const LaunchCfg& lc, uint32_t** err, uint32_t** stop) {
+    *err = lc.err;
+    *stop = lc.stop;
+    if (!lc.err) fast_error_word(err);
+}
 cudaError_t tile_q4(const LaunchCfg& lc, void* tiled, void* tiled_scales, const void* canon, const void* canon_scales,
                     uint32_t rows, uint32_t K);
 
@@ -186,7 +192,7 @@ struct AttnArgs {
     uint32_t max_splits = 1;       // grid size along the context (fixed per context so that graphs replay)
     uint32_t tokens_per_split = 32; // multiple of block_tokens
     unsigned long long* trace = nullptr;
-    uint32_t* err = nullptr;       // device word that a bounded wait sets when it runs out
+    uint32_t *err = nullptr, *stop = nullptr;  // words that a bounded wait sets when it runs out (LaunchCfg)
     float* scratch = nullptr;      // attn_scratch_floats(): partials, then the split counters (zero before the first launch)
     // paged fp16 pool as a tiled-TMA tensor map (attn_make_kv_map; a CUtensorMap on the host) and the row of that map
     // where this layer's part of the pool begins; without it the tensor-core path is not taken

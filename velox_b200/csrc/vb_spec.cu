@@ -126,7 +126,7 @@ int32_t verify_pass(vb_ctx* c, int32_t slot, const uint32_t* cand, uint32_t B, u
     VB_CUDA(argmax(lcfg(c, true), d_win, c->spec_logits, c->vocab, B, c->spec_cand_v, c->spec_cand_i, nullptr, nullptr, 0));
     VB_CUDA(cudaMemcpyAsync(winners, d_win, B * 4, cudaMemcpyDeviceToHost, c->stream));
     VB_CUDA(cudaStreamSynchronize(c->stream));
-    return VB_OK;
+    return check_device_error(c);
 }
 
 }  // namespace

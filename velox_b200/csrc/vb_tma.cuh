@@ -47,6 +47,36 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (clock64() - t0 > 2000000000LL) return false;
     }
 }
+// The context's stop word (LaunchCfg::stop): a wait that runs out sets it, so that what was enqueued behind it does not wait its own second.
+__device__ __forceinline__ bool stop_set(const uint32_t* stop) { return stop && *reinterpret_cast<const volatile uint32_t*>(stop) != 0u; }
+__device__ __forceinline__ void report_wait(uint32_t* err, uint32_t* stop, uint32_t code) {
+    if (err) atomicOr(err, code);
+    if (stop) *reinterpret_cast<volatile uint32_t*>(stop) = code;
+}
+// Bounded wait of a block that goes on, and may leave, when it gives up: a second, or 10 ms where the stop word is set, which is ample for
+// copies that are under way at all.
+__device__ __forceinline__ bool wait_or_stop(uint32_t bar, uint32_t parity, const uint32_t* stop) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 128; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (clock64() - t0 > (stop_set(stop) ? 20000000LL : 2000000000LL)) return false;
+    }
+}
+// Bounded wait that also gives up as soon as another thread of the block has given up, or the stop word is set.
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, const uint32_t* stop) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 128; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (*abort_flag) return false;
+        if (stop_set(stop) || clock64() - t0 > 2000000000LL) { *abort_flag = 1u; return false; }
+    }
+}
 // One lane of the (converged) warp, always the same one.  Tensor-core and TMA instructions take their operands from uniform
 // registers: under `lane == 0` the compiler has to make them uniform instruction by instruction (the latent attention's 36
 // products of a tile came 183 clocks apart instead of ~55), after elect.sync it knows that one lane runs.
