@@ -348,7 +348,8 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
         // ---- producer: this block's copies, counted by the first block ----
         if (elect_one()) {
             const uint32_t full0 = pair_addr(bars, 0);
-            for (int kb = 0; kb < nk; ++kb) {
+            int kb = 0;
+            for (; kb < nk; ++kb) {
                 const int s = kb % STAGES;
                 const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
                 if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag, p.stop)) break;
@@ -364,6 +365,11 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 #pragma unroll
                 for (int xp = 0; xp < XP; ++xp) pair_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, tok0 + (int)rank * (BN / 2) + xp * (int)p.x_lo_row, full);
             }
+            // The last stages come back too before this block leaves: nothing orders their arrivals, sent from the other SM, before the
+            // accumulator's, and one that came later would count at a barrier of the block that has this shared memory next.
+            if (kb == nk)
+                for (kb = nk > STAGES ? nk - STAGES : 0; kb < nk; ++kb)
+                    if (!wait_or_abort(bars + (STAGES + kb % STAGES) * 8, (uint32_t)(kb / STAGES) & 1u, abort_flag, p.stop)) break;
         }
     } else if (warp == 1 && rank == 0 && go) {
         // ---- tensor-core issue for both blocks ----
