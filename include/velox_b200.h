@@ -214,6 +214,9 @@ int32_t vb_trace_read(vb_ctx* ctx, uint64_t* out, uint32_t max_records, uint32_t
  *   "prefill_two_per_sm", "prefill_wide"   accepted, without effect
  *   "decode_gemm"    1: the products of a decode step (lm_head included) run as tensor-core GEMMs, one row of x per
  *                    slot; default 1 when max_batch >= 16 and the weights are int8 per channel or fp16, else 0
+ *   "few_i8"         1 (default): steps of 3 to 16 sequences and speculative verify passes of 3 to 8 rows over int8 per-channel weights
+ *                    run on the integer tensor cores without "decode_gemm" and its copies, from 2 M weights a matrix on (3 and 4
+ *                    rows: 32 M); 0: on the integer matrix-vector kernel, four rows a pass
  *   "decode_gemm_i8" 1 (default): those products over int8 per-channel weights (batches of up to 32) run on the integer
  *                    tensor cores straight from the stored bytes (exact arithmetic, one byte per weight from HBM); 0: through
  *                    resident fp16 copies

@@ -389,6 +389,7 @@ def test_few_int8_rows_on_the_integer_tensor_cores(d_model, ffn, batch):
     eng = H.build_engine(spec, 91, 32, max_batch=batch)
     if d_model < 2048:
         eng.set_option("decode_gemm", 1)
+    eng.build_graph()  # (makes the workspaces of the step's products, as a prompt does; without them it takes others)
     toks = np.random.default_rng(batch).integers(0, spec.vocab, size=(batch, 2))
     for slot in range(batch):
         eng.reserve(slot, 32)
@@ -403,4 +404,37 @@ def test_few_int8_rows_on_the_integer_tensor_cores(d_model, ffn, batch):
             ora.forward_step(int(t), pos)
         # rows of 2048: logits up to twice those of 512
         assert float(np.max(np.abs(eng.logits(slot) - ora.logits))) <= (2 if d_model == 2048 else 1) * TOL, (slot,)
+    eng.close()
+
+
+@pytest.mark.parametrize("d_model,ffn,batch", [(2048, 4224, 5), (2048, 16384, 3), (2048, 16384, 4)])
+def test_few_int8_rows_and_the_options_around_them(d_model, ffn, batch):
+    """Steps that take the integer tensor cores by themselves: "decode_gemm" 0, the default of such a context, leaves them there (the same
+    bits), "few_i8" 0 does not (its matrix-vector products take 16 bits of every 32 values), 1 brings them back."""
+    spec = LLAMA3_8B_INT4.scaled(name="few", d_model=d_model, n_layers=1, n_q_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=ffn, vocab=1040,
+                                 weight_fmt=L.FMT_I8PC, head_fmt=L.FMT_I8PC)
+    eng = H.build_engine(spec, 92, 16, max_batch=batch)
+    for slot in range(batch):
+        eng.reserve(slot, 16)
+
+    def step():
+        eng.build_graph()  # (makes the workspaces of the step's products, as a prompt does)
+        for slot in range(batch):
+            eng.set_state(slot, 7 * slot + 3, 0)
+        before = eng.launch_count()
+        eng.decode(1)
+        return eng.launch_count() - before, np.stack([eng.logits(slot) for slot in range(batch)])
+
+    launches, want = step()
+    eng.set_option("decode_gemm", 0)
+    again = step()
+    assert again[0] == launches and np.array_equal(again[1], want)
+    eng.set_option("few_i8", 0)
+    other = step()[1]
+    assert not np.array_equal(other, want) and float(np.max(np.abs(other - want))) <= TOL
+    eng.set_option("few_i8", 1)
+    assert np.array_equal(step()[1], want)
+    ora, _ = H.build_oracle(spec, 92, 16)
+    ora.forward_step(7 * (batch - 1) + 3, 0)
+    assert float(np.max(np.abs(want[-1] - ora.logits))) <= 2 * TOL  # rows of 2048: logits up to twice those of 512
     eng.close()

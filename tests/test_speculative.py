@@ -41,8 +41,13 @@ def test_checker_speculative_loop_equals_greedy():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("spec,draft", [(SPEC, 3), (SPEC, 7), (QWEN25_7B_INT8.scaled(name="qwen-int8-tiled", d_model=512, n_layers=2, n_q_heads=8,
-                                                                                     n_kv_heads=2, head_dim=64, ffn_dim=1408, vocab=4096), 4)],
-                         ids=["int4-k3", "int4-k7", "int8-bias-k4"])
+                                                                                     n_kv_heads=2, head_dim=64, ffn_dim=1408, vocab=4096), 4),
+                                        # verify passes on the integer tensor cores: of 5 and more rows, and of 3 and 4 (32 M weights a matrix)
+                                        (QWEN25_7B_INT8.scaled(name="qwen-int8-2m", d_model=1024, n_layers=2, n_q_heads=8, n_kv_heads=2, head_dim=128,
+                                                               ffn_dim=2048, vocab=4096), 5),
+                                        (QWEN25_7B_INT8.scaled(name="qwen-int8-32m", d_model=2048, n_layers=1, n_q_heads=16, n_kv_heads=2, head_dim=128,
+                                                               ffn_dim=16384, vocab=4096), 3)],
+                         ids=["int4-k3", "int4-k7", "int8-bias-k4", "int8-2m-k5", "int8-32m-k3"])
 def test_engine_speculative_matches_checker(spec, draft):
     n_new = 64
     base = H.prompt_tokens(spec, 8, 12)

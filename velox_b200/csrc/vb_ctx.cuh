@@ -95,7 +95,7 @@ struct vb_ctx {
     // from `prefill_ts_min` on (vb_gemm_ts.cu: x in parts as fine as those of the kernels for few rows; equal time at 16 rows)
     bool prefill_gemm = true;
     bool decode_gemm = false;   // decode steps of wide batches through the same tensor-core GEMMs (one row per slot)
-    bool few_i8 = false;        // steps of a few rows over int8 weights through the integer tensor-core products alone (few_i8_rows)
+    bool few_i8 = false;        // steps and verify passes of a few rows over int8 weights through the integer tensor-core products alone (few_i8_rows)
     bool decode_gemm_auto = false;  // switched on by vb_create, not by the caller: falls back silently when unsupported
     bool prefill_flash = true;  // causal tile attention for those chunks (vb_attn_prefill.cu) instead of one launch row per token
     uint32_t prefill_rows = 2048, prefill_gemm_min = 48, prefill_ts_min = 16;

@@ -1417,9 +1417,10 @@ int32_t vb_set_option(vb_ctx* c, const char* name, int64_t value) {
     if (!strcmp(name, "decode_gemm")) {  // the workspace is allocated by the next vb_decode_step / vb_decode_graph_build
         VB_REQUIRE(!value || c->d.tp_size <= 1, "vb_set_option: decode_gemm is not available on a sharded context");
         c->decode_gemm = value != 0;
-        c->decode_gemm_auto = c->few_i8 = false;
+        c->decode_gemm_auto = false;
         return VB_OK;
     }
+    if (!strcmp(name, "few_i8")) { c->few_i8 = value != 0 && c->d.tp_size <= 1 && c->d.weight_fmt == VB_FMT_I8PC; return VB_OK; }
     if (!strcmp(name, "decode_gemm_i8")) { gemm_i8_enabled = value != 0; return VB_OK; }
     if (!strcmp(name, "i8_tiles")) { gemm_i8_tiles = value != 0; return VB_OK; }
     if (!strcmp(name, "i8_half_ring")) { gemm_i8_half_ring = value != 0; return VB_OK; }
