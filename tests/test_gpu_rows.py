@@ -438,3 +438,85 @@ def test_few_int8_rows_and_the_options_around_them(d_model, ffn, batch):
     ora.forward_step(7 * (batch - 1) + 3, 0)
     assert float(np.max(np.abs(want[-1] - ora.logits))) <= 2 * TOL  # rows of 2048: logits up to twice those of 512
     eng.close()
+
+
+def bare_int8_engine(d_model, ffn, batch, rows):
+    """One int8 layer whose attention adds nothing (Wo = 0), over fp32 embedding rows: (engine, its weights dequantised in 64 bits)."""
+    spec = LLAMA3_8B_INT4.scaled(name="bare", d_model=d_model, n_layers=1, n_q_heads=d_model // 64, n_kv_heads=1 if d_model == 448 else 2, head_dim=64,
+                                 ffn_dim=ffn, vocab=1040, weight_fmt=L.FMT_I8PC, head_fmt=L.FMT_I8PC, embed_fmt=L.FMT_F32)
+    eng = H.build_engine(spec, 93, 16, max_batch=batch)
+    eng.load_tensor(L.ROLE_WO, 0, np.zeros((d_model, d_model), np.float32))
+    table = np.zeros((spec.vocab, d_model), np.float32)
+    table[:len(rows)] = rows
+    eng.load_tensor(L.ROLE_EMBED, 0, table)
+    eng.set_option("decode_gemm", 1)
+    for slot in range(batch):
+        eng.reserve(slot, 16)
+    w = {}
+    for role, n, k in ((L.ROLE_MLP_NORM, 1, d_model), (L.ROLE_FINAL_NORM, 1, d_model), (L.ROLE_WGATE, ffn, d_model), (L.ROLE_WUP, ffn, d_model),
+                       (L.ROLE_WDOWN, d_model, ffn), (L.ROLE_LM_HEAD, spec.vocab, d_model)):
+        data, scales = eng.export_tensor(role, 0, n, k)
+        if spec.storage_fmt(role) == L.FMT_I8PC:
+            w[role] = data.astype(np.float64) * scales.view(np.float16).astype(np.float64)[:, None]
+        else:
+            w[role] = data.view(np.float16).astype(np.float64).reshape(k)
+    return spec, eng, w
+
+
+def bare_step(eng, batch):
+    eng.build_graph()
+    for slot in range(batch):
+        eng.set_state(slot, slot, 0)
+    eng.decode(1)
+    return np.stack([eng.hidden(slot) for slot in range(batch)]), np.stack([eng.logits(slot) for slot in range(batch)])
+
+
+@pytest.mark.parametrize("batch", [1, 3, 15, 16, 17, 32])
+@pytest.mark.parametrize("d_model,ffn", [(448, 1184), (512, 20608), (1024, 1408)])
+def test_int8_products_of_a_batch_against_64_bits(d_model, ffn, batch):
+    """SiLU, residual (K split over blocks) and plain products, K that is no multiple of 128 and rows beyond a block's registers; rows with an
+    outlier of 1000 and of 100000.  x has 24 bits of its row's largest magnitude m up to 16 rows, 16 bits beyond: rounded to steps of m / P, each
+    value is off by m / (P sqrt(12)) rms, a product by that times the norm of the matrix (a plane too few: 256 times as much)."""
+    rng = np.random.default_rng(batch)
+    rows = rng.standard_normal((batch, d_model)).astype(np.float32)
+    for row, outlier in ((batch - 1, 1.0e3), (batch // 2, 1.0e5)):
+        if batch > 1:
+            rows[row, 5 + row] = outlier
+    spec, eng, w = bare_int8_engine(d_model, ffn, batch, rows)
+    hidden, logits = bare_step(eng, batch)
+    eng.close()
+    levels = (8.3e6 if batch <= 16 else 32000.0) * np.sqrt(12.0)
+    norm = lambda v, g: v / np.sqrt((v * v).mean() + spec.rms_eps) * g
+    gate, up, down, head = w[L.ROLE_WGATE], w[L.ROLE_WUP], w[L.ROLE_WDOWN], w[L.ROLE_LM_HEAD]
+    for slot in range(batch):
+        e = rows[slot].astype(np.float64)
+        x = norm(e, w[L.ROLE_MLP_NORM])
+        g, u = gate @ x, up @ x
+        sig = 1.0 / (1.0 + np.exp(-g))
+        act = g * sig * u
+        step = np.abs(x).max() / levels
+        off = np.sqrt(((sig * (1 + g * (1 - sig)) * u) ** 2 * (gate ** 2).sum(1) + (g * sig) ** 2 * (up ** 2).sum(1)).sum()) * step  # of act
+        fro = np.linalg.norm(down)
+        bound = 1.5 * (np.abs(act).max() / levels * fro + (off + 2.0 ** -22 * np.linalg.norm(act)) * fro / np.sqrt(ffn))
+        want = e + down @ act
+        assert np.linalg.norm(hidden[slot] - want) <= bound + 2.0 ** -24 * np.linalg.norm(want), slot
+        x = norm(hidden[slot].astype(np.float64), w[L.ROLE_FINAL_NORM])
+        want = head @ x
+        assert np.linalg.norm(logits[slot] - want) <= 1.5 * np.abs(x).max() / levels * np.linalg.norm(head) + 2.0 ** -22 * np.linalg.norm(want), slot
+
+
+@pytest.mark.parametrize("batch", [3, 16, 17, 32])
+@pytest.mark.parametrize("d_model,ffn", [(512, 1408), (512, 20608)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_an_int8_row_that_is_not_finite_gives_no_numbers(d_model, ffn, batch, bad):
+    rows = np.random.default_rng(7).standard_normal((batch, d_model)).astype(np.float32)
+    _, eng, _ = bare_int8_engine(d_model, ffn, batch, rows)
+    want = bare_step(eng, batch)
+    eng.close()
+    rows[1, 77] = bad
+    _, eng, _ = bare_int8_engine(d_model, ffn, batch, rows)
+    got = bare_step(eng, batch)
+    eng.close()
+    others = np.arange(batch) != 1
+    for a, b in zip(got, want):
+        assert np.all(np.isnan(a[1])) and np.array_equal(a[others], b[others])

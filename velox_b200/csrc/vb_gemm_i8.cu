@@ -279,37 +279,25 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     trace_exit(p.trace);
 }
 
-// What brings a row's largest magnitude to the top of its planes (m): 1 for an all-zero or non-finite row.
+// What brings a row's largest magnitude (m, below) to the top of its planes; 1 for an all-zero or non-finite row.
 template <int ROWS>
 __device__ __forceinline__ float row_scale_i8(float m) {
+    if (!(m > 0.0f && m <= 3.4028235e38f)) return 1.0f;
     if constexpr (I8Shape<ROWS>::planes == 2) {
-        float pw = 1.0f;
-        if (m > 0.0f && m < 3.0e38f) pw = __fdividef(32000.0f, m);
+        const float pw = m < 8.0e37f ? __fdividef(32000.0f, m) : 32000.0f / m;  // (the fast quotient is 0 from 2^126 on)
         return pw < 3.0e38f ? pw : 1.0f;
     } else {
-        return m > 0.0f && m <= 3.4028235e38f ? fminf(8300000.0f / m, 5.0e37f) : 1.0f;
+        return fminf(8300000.0f / m, 5.0e37f);
     }
 }
-// what takes it back; three planes: a row with a value that is not finite must not give numbers
-template <int ROWS>
-__device__ __forceinline__ float inv_scale_i8(float m, float pw) {
-    return I8Shape<ROWS>::planes == 2 || m <= 3.4028235e38f ? 1.0f / pw : __int_as_float(0x7FC00000);
-}
-// the largest |x|; three planes: in the order of the bits, NaN on top
-template <int ROWS>
+// What takes it back.  A row with a value that is not finite must not give numbers, however many rows share the step.
+__device__ __forceinline__ float inv_scale_i8(float m, float pw) { return m <= 3.4028235e38f ? 1.0f / pw : __int_as_float(0x7FC00000); }
+// the largest |x| in the order of the bits, NaN on top
 __device__ __forceinline__ float row_max_i8(float m, const float4& v) {
-    if constexpr (I8Shape<ROWS>::planes == 2) {
-        return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    } else {
-        const uint32_t s = 0x7FFFFFFFu;
-        return __uint_as_float(max(__float_as_uint(m), max(max(__float_as_uint(v.x) & s, __float_as_uint(v.y) & s), max(__float_as_uint(v.z) & s, __float_as_uint(v.w) & s))));
-    }
+    const uint32_t s = 0x7FFFFFFFu;
+    return __uint_as_float(max(__float_as_uint(m), max(max(__float_as_uint(v.x) & s, __float_as_uint(v.y) & s), max(__float_as_uint(v.z) & s, __float_as_uint(v.w) & s))));
 }
-template <int ROWS>
-__device__ __forceinline__ float warp_max_i8(float m) {
-    if constexpr (I8Shape<ROWS>::planes == 2) return warp_max(m);
-    else return __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
-}
+__device__ __forceinline__ float warp_max_i8(float m) { return __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m))); }
 // four values as bytes of the planes, `K` apart
 template <int ROWS>
 __device__ __forceinline__ void store_planes(int8_t* row, size_t plane, uint32_t k, const float4& v, float pw) {
@@ -385,16 +373,16 @@ k_rows_to_i8(int8_t* __restrict__ planes, float* __restrict__ inv_scale, const f
     };
     float mx = 0.0f;
     for (uint32_t k = threadIdx.x; k < K4; k += blockDim.x) {
-        mx = row_max_i8<ROWS>(mx, normed(k));
+        mx = row_max_i8(mx, normed(k));
     }
-    mx = warp_max_i8<ROWS>(mx);
+    mx = warp_max_i8(mx);
     if ((threadIdx.x & 31) == 0) part_mx[threadIdx.x >> 5] = mx;
     __syncthreads();
     float gmax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) gmax = row_max_i8<ROWS>(gmax, make_float4(part_mx[i], 0.f, 0.f, 0.f));
+    for (int i = 0; i < 8; ++i) gmax = row_max_i8(gmax, make_float4(part_mx[i], 0.f, 0.f, 0.f));
     const float pw = row_scale_i8<ROWS>(gmax);
-    if (threadIdx.x == 0) inv_scale[r] = inv_scale_i8<ROWS>(gmax, pw);
+    if (threadIdx.x == 0) inv_scale[r] = inv_scale_i8(gmax, pw);
     for (uint32_t k = threadIdx.x; k < K4; k += blockDim.x) store_planes<ROWS>(row, plane, k, normed(k), pw);
 }
 
@@ -465,18 +453,18 @@ k_rows_to_i8_regs(int8_t* __restrict__ planes, float* __restrict__ inv_scale, co
     }
     float mx = 0.0f;
 #pragma unroll
-    for (int i = 0; i < XR; ++i) mx = row_max_i8<ROWS>(mx, v[i]);
-    mx = warp_max_i8<ROWS>(mx);
+    for (int i = 0; i < XR; ++i) mx = row_max_i8(mx, v[i]);
+    mx = warp_max_i8(mx);
     __syncthreads();  // red[] is read no more
     if (lane == 0) red[warp] = mx;
     __syncthreads();
     if (warp == 0) {
-        const float g = warp_max_i8<ROWS>(red[lane]);
+        const float g = warp_max_i8(red[lane]);
         if (lane == 0) bc[1] = g;
     }
     __syncthreads();
     const float gmax = bc[1], pw = row_scale_i8<ROWS>(gmax);
-    if (threadIdx.x == 0) inv_scale[r] = inv_scale_i8<ROWS>(gmax, pw);
+    if (threadIdx.x == 0) inv_scale[r] = inv_scale_i8(gmax, pw);
 #pragma unroll
     for (int i = 0; i < XR; ++i) {
         const uint32_t k = threadIdx.x + i * 1024;
