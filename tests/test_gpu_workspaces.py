@@ -106,3 +106,33 @@ def test_group64_weights_in_a_nearly_full_card():
         eng.close()
     assert packed <= sizes[1] < 1.01 * packed + (1 << 20) and sizes[0] <= 2 * sizes[1]
     assert np.max(np.abs(got[0] - got[1])) <= 1e-2  # (the rounding of the fp16 cache apart)
+
+
+def test_int8_prompts_without_room_for_copies():
+    """Prompts of 129 to 256 rows of an int8 model that may not, or cannot, hold fp16 copies of its weights read the packed ones: no copies
+    and no room for converted weights (70 MB a matrix); longer ones take that way too where the card has no such room."""
+    spec = spec_of(L.FMT_I8PC, n_layers=2, d_model=2048, n_q_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=17408)
+    ora, _ = H.build_oracle(spec, 75, 320)
+    prompt = H.prompt_tokens(spec, 75, 300)
+    want = {}
+    for pos, t in enumerate(prompt):
+        ora.forward_step(int(t), pos)
+        want[pos + 1] = ora.logits.copy()
+    for n in (130, 200, 257, 300):
+        for resident_gb, left in ((40, None), (0, None), (40, 120 << 20)):
+            eng = H.build_engine(spec, 75, 320)
+            eng.set_option("tc_resident_gb", resident_gb)
+            eng.reserve(0, 320)
+            eng.prefill(prompt[:20])
+            hog = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda") if left else None
+            before = free_bytes()
+            try:
+                eng.prefill(prompt[:n])
+            finally:
+                used = before - free_bytes()
+                del hog
+                torch.cuda.empty_cache()
+            assert np.max(np.abs(eng.logits() - want[n])) <= 1e-2, (n, resident_gb, left)
+            if n <= 257 and (resident_gb, left) != (40, None):
+                assert used <= 110 << 20, (n, used)  # buffers of 320 rows: 3 + 4 + 3 + 3 + 22 MB and 22 MB of parts
+            eng.close()

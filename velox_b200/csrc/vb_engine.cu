@@ -266,6 +266,9 @@ bool weights_within_f16(const vb_ctx* c) {
     return true;
 }
 constexpr uint32_t TS_ROWS_MAX = 128;
+// int8 prompts stay with them up to 256 rows where no fp16 copies of the weights are there nor can be made: converting 13 GB of weights for
+// one prompt of the 7B shape takes longer than the difference above.
+constexpr uint32_t TS_I8_ROWS_WITHOUT_COPIES = 256;
 bool ts_products_ok(vb_ctx* c) {
     if (gemm_tc_split != 2) return false;  // fewer parts: the products of vb_gemm_tc.cu
     const int roles[] = {VB_ROLE_WQ, VB_ROLE_WO, VB_ROLE_WGATE, VB_ROLE_WDOWN};
@@ -1139,8 +1142,13 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     const bool gemm_ok = c->prefill_gemm && c->d.tp_size <= 1 && c->prefill_rows >= 1 && weights_within_f16(c);
     const bool tc_ok = gemm_ok && n_tokens > c->prefill_gemm_min && tc_products_ok(c);
     const uint32_t rows = std::min(c->prefill_rows, n_tokens - 1);
-    const bool use_ts = gemm_ok && n_tokens > c->prefill_ts_min && ts_products_ok(c) && (!tc_ok || rows <= TS_ROWS_MAX);
+    const bool ts_ok = gemm_ok && n_tokens > c->prefill_ts_min && ts_products_ok(c);
+    bool use_ts = ts_ok && (!tc_ok || rows <= TS_ROWS_MAX);
     const bool use_tc = use_ts || tc_ok;
+    if (tc_ok && ts_ok && !use_ts && c->d.weight_fmt == VB_FMT_I8PC && rows <= TS_I8_ROWS_WITHOUT_COPIES) {
+        if ((rc = ensure_f16_copies(c)) != VB_OK) return rc;
+        use_ts = !c->f16_pool;
+    }
     uint32_t P = use_tc ? rows : c->prefill_chunk;
     if (use_tc || (P >= 2 && P <= 32 && c->d.tp_size <= 1 && 2 * n_tokens > P)) {
         // Rows the chunk buffers hold: two sizes, short prompts and the longest chunk of this context, so that prompts of growing
@@ -1148,18 +1156,20 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
         // 4 to 7 ms of an 11 ms prompt).
         uint32_t cap = P;
         if (use_tc) cap = use_ts && rows <= TS_ROWS_MAX ? TS_ROWS_MAX : std::max(rows, std::min(c->prefill_rows, c->d.max_seq_len));
-        rc = ensure_chunk_buffers(c, cap);
-        if (use_ts) {
-            if (rc == VB_OK) rc = ensure_ts_ws(c, cap);
-            // a context that has filled the card takes its prompts in shorter chunks, as far down as the sixteen rows that always fit
-            while (rc == VB_ERR_OOM && cap > 16) {
-                cap /= 2;
-                P = std::min(P, cap);
-                if ((rc = ensure_chunk_buffers(c, cap)) == VB_OK) rc = ensure_ts_ws(c, cap);
-            }
-        } else if (rc == VB_OK && use_tc && (rc = ensure_f16_copies(c)) == VB_OK) {
-            rc = ensure_tc_ws(c, cap, false);
+        auto buffers = [&]() {
+            const int32_t r = ensure_chunk_buffers(c, cap);
+            return r != VB_OK || !use_tc ? r : use_ts ? ensure_ts_ws(c, cap) : ensure_tc_ws(c, cap, false);
+        };
+        rc = buffers();
+        // A context that has filled the card takes its prompts in shorter chunks, as far down as the sixteen rows that always fit; over
+        // fp16 copies it needs room for converted weights too, whatever the rows, so it leaves them where the packed weights will do.
+        while (use_tc && rc == VB_ERR_OOM && cap > 16) {
+            if (!use_ts && ts_ok) use_ts = true;
+            else cap /= 2;
+            P = std::min(P, cap);
+            rc = buffers();
         }
+        if (rc == VB_OK && use_tc && !use_ts) rc = ensure_f16_copies(c);
         if (rc != VB_OK) return rc;
         VB_CUDA(launch(lcfg(c, false), k_fill_chunk_table, dim3(P), dim3(128), 0, c->pfc_table,
                        (const int32_t*)(c->block_table_dev + (size_t)slot * c->max_blocks), c->max_blocks));
