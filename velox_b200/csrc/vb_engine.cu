@@ -1138,7 +1138,7 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // j attends positions 0..first+j, so the result is the causal one.  (The reference's batched prefill driver:
     // velox_cuda_runner_k2.cu:1614-1704.)  Sharded contexts and the last token take the per-token path below.
     // Prompts of up to half a chunk go token by token: the same bits as the same tokens fed one step at a time.
-    uint32_t done = 0;
+    uint32_t done = 0, chunk = 0;
     const bool gemm_ok = c->prefill_gemm && c->d.tp_size <= 1 && c->prefill_rows >= 1 && weights_within_f16(c);
     const bool tc_ok = gemm_ok && n_tokens > c->prefill_gemm_min && tc_products_ok(c);
     const uint32_t rows = std::min(c->prefill_rows, n_tokens - 1);
@@ -1180,7 +1180,6 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
         io.split_attn = !tc_ok;
         // the last token always takes the per-token path below (it produces the logits); the last chunk may be ragged (token by
         // token instead, a 120-token prompt of the 72B shape spent 66 ms on its last 8)
-        uint32_t chunk = 0;
         while (done + 1 < n_tokens) {
             const uint32_t n = std::min(P, n_tokens - 1 - done);
             io.B = n; io.first = done;
@@ -1208,7 +1207,8 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     // hand the slot over to the decode state: first generated token at position n_tokens
     VB_CUDA(cudaMemcpyAsync(c->state + slot, c->pf_state + slot, sizeof(SeqState), cudaMemcpyDeviceToDevice, c->stream));
     VB_CUDA(cudaStreamSynchronize(c->stream));
-    if (*reinterpret_cast<volatile uint32_t*>(c->err_host)) {
+    // (a prompt that went token by token leaves the report to the next call that reads)
+    if (chunk && *reinterpret_cast<volatile uint32_t*>(c->err_host)) {
         vb_seq_set(c, slot, 0, 0, 0);
         return check_device_error(c);
     }
