@@ -231,13 +231,16 @@ int32_t vb_trace_read(vb_ctx* ctx, uint64_t* out, uint32_t max_records, uint32_t
  *   "pdl"            1: programmatic dependent launch between the kernels of a step
  *   "attn_tcgen05"   1: the decode attention of head_dim-128 models runs its two products as tcgen05.mma (tokens as the M dimension,
  *                    S^T and O^T in tensor memory); same results, measured slower than the mma.sync form (default 0)
- *   "attn_splits"    slices of the context per (sequence, KV head) in the decode attention (1..16; default: one per 32 tokens
- *                    of max_seq_len up to 8, fewer when the batch alone fills the GPU, 16 for long contexts of few KV heads)
+ *   "attn_splits"    slices of the context per (sequence, KV head) in the decode attention, 1..16 (more than 8 where a launch has four
+ *                    such pairs at most); 0 (default): by max_seq_len, the KV heads and the sequences of a launch: 8 while those
+ *                    are few, 4, 3, 2, 1 as they grow, 16 for long contexts of four pairs
  *   "trace"          1: device time stamps per kernel (vb_trace_read)
  *   "tp_p2p"         1: NVLink push exchange when peer regions are open, 0: NCCL
  *   "tp_fused_push"  1: the row-parallel products send their rows to the peers from their own epilogue;
  *   "tp_fused_reduce" 1: ... and gather the peers' copies of their own rows, so the exchange needs no kernel of its own
  *   "tp_poll_ms"     limit of one exchange poll (default ~10000)
+ *   "stop_word"      diagnostic: 1 sets what a device-side wait that ran out leaves behind (the products that look at it start nothing, the
+ *                    call that waits for them returns VB_ERR_TIMEOUT and clears it), 0 clears it
  *   "tp_p2p_standin" diagnostic: private stand-in regions instead of peers (every exchange then runs into its
  *                    poll limit; used by the time-out test) */
 int32_t vb_set_option(vb_ctx* ctx, const char* name, int64_t value);

@@ -520,3 +520,45 @@ def test_an_int8_row_that_is_not_finite_gives_no_numbers(d_model, ffn, batch, ba
     others = np.arange(batch) != 1
     for a, b in zip(got, want):
         assert np.all(np.isnan(a[1])) and np.array_equal(a[others], b[others])
+
+
+SLICES = LLAMA3_8B_INT4.scaled(name="slices8", d_model=256, n_layers=1, n_q_heads=32, n_kv_heads=8, head_dim=128, ffn_dim=256, vocab=512,
+                               weight_fmt=L.FMT_F16, head_fmt=L.FMT_F16)
+SLICE_PROMPTS = (600, 333)
+
+
+@functools.lru_cache(maxsize=None)
+def slices_want(slot):
+    n = SLICE_PROMPTS[slot]
+    ora, _ = H.build_oracle(SLICES, 52, 640)
+    for pos, t in enumerate(H.prompt_tokens(SLICES, 52 + slot, n)):
+        ora.forward_step(int(t), pos)
+    want = {}
+    for pos in (n - 1, 300, 257, 256, 130, 16, 15, 0):
+        ora.forward_step(5, pos)
+        want[pos] = ora.logits.copy()
+    return want
+
+
+@pytest.mark.parametrize("max_seq", [640, 4500])
+@pytest.mark.parametrize("batch", [1, 2])
+@pytest.mark.parametrize("splits", [0, 2, 4, 6, 8, 16])
+def test_attention_slices_of_many_clusters(splits, batch, max_seq):
+    """Eight and sixteen (sequence, KV head) pairs, whose clusters may not all run at once, and block tables on both sides of the 256 entries
+    that are fetched whole; 0: the number of slices that the rule takes, more than eight ask for no more than eight here."""
+    eng = H.build_engine(SLICES, 52, max_seq, max_batch=batch)
+    eng.set_option("attn_splits", splits)
+    for slot in range(batch):
+        eng.reserve(slot, 640)
+        eng.prefill(H.prompt_tokens(SLICES, 52 + slot, SLICE_PROMPTS[slot]), slot)
+    for step in range(8):
+        at = [list(slices_want(slot))[step] for slot in range(batch)]
+        for slot in range(batch):
+            eng.set_state(slot, 5, at[slot])
+        eng.decode(1)
+        for slot in range(batch):
+            assert float(np.max(np.abs(eng.logits(slot) - slices_want(slot)[at[slot]]))) <= TOL, (slot, at[slot])
+    for bad in (-1, 17):
+        with pytest.raises(L.VeloxError):
+            eng.set_option("attn_splits", bad)
+    eng.close()

@@ -976,9 +976,8 @@ uint32_t attn_pick_splits(uint32_t max_seq) {
 bool attn_use_tcgen05 = false;
 bool attn_use_mma = true;  // fp16 caches with head_dim <= 256: QK^T and PV on the tensor cores (option "attn_mma")
 
-// resident != null: nothing is launched; how many of the launch's clusters the device holds at once
 template <typename KVT, int EPL, int GM, int MMA>
-static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka, int* resident) {
+static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka) {
     ka.g_chunks = (ka.G + GM - 1) / GM;
     dim3 grid(ka.a.Hkv * ka.g_chunks, ka.n_splits, ka.a.batch);
     const size_t smem = AttnSmem<KVT, EPL, GM, MMA>::total;
@@ -1009,53 +1008,60 @@ static cudaError_t launch_split_g(const LaunchCfg& lc, AttnKArgs ka, int* reside
         attr[cfg.numAttrs++].val.sharedMemCarveout = 72;
     }
     cfg.attrs = attr;
-    if (resident) return cudaOccupancyMaxActiveClusters(resident, k_attn_split<KVT, EPL, GM, MMA>, &cfg);
     if (lc.counter) ++*lc.counter;
     return cudaLaunchKernelEx(&cfg, k_attn_split<KVT, EPL, GM, MMA>, ka);
 }
 
+// the tensor-core path reads the paged pool of 16-token blocks through its tensor map
+static bool attn_takes_mma(const AttnArgs& a) {
+    return a.kv_fp16 && (a.D == 64 || a.D == 128 || a.D == 256) && attn_use_mma && a.kv_map && a.block_table && a.block_tokens == 16;
+}
+uint32_t attention_clusters(const AttnArgs& a) {
+    const uint32_t g = a.Hq / a.Hkv, at_once = a.D >= 256 && !attn_takes_mma(a) ? 1 : 8;  // query heads of a block, as launch_split has them
+    return a.Hkv * ((g + at_once - 1) / at_once);
+}
+
 template <typename KVT, int EPL>
-static cudaError_t launch_split(const LaunchCfg& lc, const AttnKArgs& ka, int* resident) {
+static cudaError_t launch_split(const LaunchCfg& lc, const AttnKArgs& ka) {
     if constexpr (sizeof(KVT) == 2 && EPL >= 2 && EPL <= 8) {
-        // tensor-core path: paged pool of 16-token blocks reachable through its tensor map
-        if (attn_use_mma && ka.a.kv_map && ka.a.block_table && ka.a.block_tokens == 16) {
+        if (attn_takes_mma(ka.a)) {
             if constexpr (EPL == 4) {
                 if (attn_use_tcgen05) {  // head_dim 128: both products as tcgen05.mma with the tokens as the M dimension
-                    if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 2>(lc, ka, resident);
-                    if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 2>(lc, ka, resident);
-                    if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 2>(lc, ka, resident);
-                    return launch_split_g<KVT, EPL, 8, 2>(lc, ka, resident);
+                    if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 2>(lc, ka);
+                    if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 2>(lc, ka);
+                    if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 2>(lc, ka);
+                    return launch_split_g<KVT, EPL, 8, 2>(lc, ka);
                 }
             }
-            if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 1>(lc, ka, resident);
-            if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 1>(lc, ka, resident);
-            if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 1>(lc, ka, resident);
-            return launch_split_g<KVT, EPL, 8, 1>(lc, ka, resident);
+            if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 1>(lc, ka);
+            if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 1>(lc, ka);
+            if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 1>(lc, ka);
+            return launch_split_g<KVT, EPL, 8, 1>(lc, ka);
         }
     }
     if constexpr (EPL >= 8) {
-        return launch_split_g<KVT, EPL, 1, 0>(lc, ka, resident);  // wide heads: one query head per block keeps registers in bounds
+        return launch_split_g<KVT, EPL, 1, 0>(lc, ka);  // wide heads: one query head per block keeps registers in bounds
     } else {
-        if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 0>(lc, ka, resident);
-        if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 0>(lc, ka, resident);
-        if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 0>(lc, ka, resident);
-        return launch_split_g<KVT, EPL, 8, 0>(lc, ka, resident);
+        if (ka.G == 1) return launch_split_g<KVT, EPL, 1, 0>(lc, ka);
+        if (ka.G == 2) return launch_split_g<KVT, EPL, 2, 0>(lc, ka);
+        if (ka.G <= 4) return launch_split_g<KVT, EPL, 4, 0>(lc, ka);
+        return launch_split_g<KVT, EPL, 8, 0>(lc, ka);
     }
 }
 
 template <typename KVT>
-static cudaError_t dispatch_split(const LaunchCfg& lc, const AttnKArgs& ka, int* resident) {
+static cudaError_t dispatch_split(const LaunchCfg& lc, const AttnKArgs& ka) {
     switch (ka.a.D) {
-    case 32: return launch_split<KVT, 1>(lc, ka, resident);
-    case 64: return launch_split<KVT, 2>(lc, ka, resident);
-    case 128: return launch_split<KVT, 4>(lc, ka, resident);
-    case 256: return launch_split<KVT, 8>(lc, ka, resident);
-    case 512: return launch_split<KVT, 16>(lc, ka, resident);
+    case 32: return launch_split<KVT, 1>(lc, ka);
+    case 64: return launch_split<KVT, 2>(lc, ka);
+    case 128: return launch_split<KVT, 4>(lc, ka);
+    case 256: return launch_split<KVT, 8>(lc, ka);
+    case 512: return launch_split<KVT, 16>(lc, ka);
     default: return cudaErrorInvalidValue;
     }
 }
 
-static cudaError_t attention_any(const LaunchCfg& lc, const AttnArgs& a, float scale, size_t kv_batch_stride, int* resident) {
+cudaError_t attention_ex(const LaunchCfg& lc, const AttnArgs& a, float scale, size_t kv_batch_stride) {
     if (a.batch == 0 || a.Hq == 0) return cudaSuccess;
     if (a.Hkv == 0 || a.Hq % a.Hkv != 0 || a.max_splits == 0 || a.tokens_per_split == 0) return cudaErrorInvalidValue;
     // bulk copies move 16-byte aligned pieces; a paged chunk holds whole KV blocks
@@ -1080,14 +1086,10 @@ static cudaError_t attention_any(const LaunchCfg& lc, const AttnArgs& a, float s
         ka.inv_freq_n = a.D / 2;
         for (uint32_t j = 0; j < a.D / 2; ++j) ka.inv_freq[j] = a.rope_inv_freq_host[j];
     }
-    return a.kv_fp16 ? dispatch_split<__half>(lc, ka, resident) : dispatch_split<float>(lc, ka, resident);
+    return a.kv_fp16 ? dispatch_split<__half>(lc, ka) : dispatch_split<float>(lc, ka);
 }
 
-cudaError_t attention_ex(const LaunchCfg& lc, const AttnArgs& a, float scale, size_t kv_batch_stride) { return attention_any(lc, a, scale, kv_batch_stride, nullptr); }
-
 cudaError_t attention(const LaunchCfg& lc, const AttnArgs& a) { return attention_ex(lc, a, 0.0f, 0); }
-
-cudaError_t attention_resident(const AttnArgs& a, int* clusters) { return attention_any(LaunchCfg(), a, 0.0f, 0, clusters); }
 
 bool attn_make_kv_map(void* map_out, const void* pool, uint64_t rows, uint32_t D) {
     const EncodeTiledFn fn = encode_tiled_fn();

@@ -9,8 +9,6 @@
 
 namespace vb {
 
-constexpr int ATTN_SPLIT_SIZES = 6;
-constexpr uint32_t attn_split_sizes[ATTN_SPLIT_SIZES] = {16, 8, 6, 4, 3, 2};
 constexpr uint32_t RING_SLOTS = 1024;  // VELOX_HOST_RING_SLOTS (src/codegen.rs:1022)
 
 struct Tensor {
@@ -39,7 +37,6 @@ struct vb_ctx {
     // derived
     uint32_t qdim = 0, kvdim = 0, qkv_rows = 0, max_blocks = 0, n_blocks = 0, tokens_per_split = 32;
     uint32_t n_splits = 0;                        // slices of a context in the decode attention (option "attn_splits"); 0: by the rows of a launch
-    uint32_t attn_fit[ATTN_SPLIT_SIZES] = {};     // clusters of attn_split_sizes[i] blocks that the device holds at once
     // this rank's shard (tensor parallel; equal to the whole model when tp_size == 1):
     // query/KV heads, FFN columns [ffn_off, ffn_off + ffn) in whole 128-column blocks, vocabulary rows
     uint32_t hq = 0, hkv = 0, ffn = 0, ffn_off = 0, vocab = 0, vocab_off = 0;

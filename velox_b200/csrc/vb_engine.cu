@@ -462,36 +462,23 @@ StepIO decode_io(vb_ctx* c) {
     return io;
 }
 
-// Slices of a context in the decode attention: the most whose clusters (a slice's blocks of one sequence and KV head) all run at once,
-// one for 128 rows of the longest context at most, but two; `rows`: sequences, or rows of a chunk of one.  A cluster that has to wait for
-// another to end costs a whole attention: 8B int4, step in ms with 2 / 4 / 6 / 8 slices, 2 sequences of 500 rows (16 clusters, of which
-// 15 of eight blocks fit) 1.87 / 1.83 / 1.84 / 2.02, of 3000 rows 2.20 / 2.01 / 1.97 / 2.16; 3 sequences 1.89 / 1.87 / 2.08 / 2.09.  Short contexts
-// gain nothing from more (135M q4, 4 sequences of 250 rows 623 / 649 / 659 / 659 us; one of 130 528 / 526 / 532 / 531).  Counts that cut
-// the head dimension into whole groups of four merge with wider stores: five and seven slices are no faster than four and six, and
-// heads of 64 take neither three nor six (4 sequences: 642 and 657 us).  Sixteen where contexts are long: 3000 rows, 8 / 16
-// slices, 7B int8 1.76 / 1.72, 135M 0.59 / 0.56 ms; 500 rows 1.69 / 1.70, 0.525 / 0.539.
-uint32_t pick_attn_splits(const vb_ctx* c, uint32_t rows) {
-    const uint32_t g = c->hq / c->hkv, pairs = rows * c->hkv * ((g + 7) / 8), most = std::max(2u, (c->d.max_seq_len + 127) / 128);
-    for (int i = 0; i < ATTN_SPLIT_SIZES; ++i) {
-        const uint32_t n = attn_split_sizes[i];
-        if (n == 16 ? c->d.max_seq_len < 2048 : n > most) continue;
-        if (n % 3 == 0 && c->d.head_dim < 128) continue;
-        if (c->attn_fit[i] >= pairs) return n;
-    }
+// Slices of a context in the decode attention (the blocks of a cluster), by the model, the rows of the launch and the longest context alone:
+// the order of the merge, and with it the last bits, does not depend on the chip.  As many as run all their clusters at once on a chip
+// whose GPCs are of uneven size (one measured: 15 clusters of 8 blocks, 33 of 4, 45 of 3, 74 of 2; heads of up to 64: two blocks an SM): a
+// cluster that waits for another to end costs a whole attention.  One for 32 tokens of the longest context, for several rows 96.
+// 8 layers and the head, us with 2 / 3 / 4 / 6 / 8 slices: 8B int4, contexts of 500, 1 sequence (8 clusters) 369 / 370 / 358 / 360 / 360, 2
+// 498 / 498 / 486 / 492 / 538, 4 526 / 527 / 518 / 570 / 608, 5 696 / 697 / 735 / 742 / 785, 8 701 / 763 / 743 / 800 / 886; of 3000, 1 447 / 421 / 400 /
+// 388 / 378, 2 576 / 549 / 529 / 521 / 578, 5 777 / 752 / 824 / 808 / 856; 7B int8, 3 sequences (12 clusters) of 500 703 / 716 / 701 / 710 / 704, of 3000
+// 778 / 764 / 741 / 736 / 722.  The 135M model, 8 sequences (24 clusters), 2 / 4 / 8: 250 rows 933 / 937 / 957, 3000 1230 / 1081 / 1034; three
+// slices of a head of 64 are slower than two.  Sixteen for four clusters at most (each takes most of a GPC, and how many GPCs have so many SMs
+// differs from chip to chip): 3000 rows, 8 / 16, 7B int8 572 / 564, 135M 595 / 587; 1000 rows 548 / 559.
+uint32_t pick_attn_splits(const vb_model_desc& d, uint32_t rows, uint32_t clusters) {
+    static constexpr struct { uint32_t slices, clusters; } rule[] = {{8, 14}, {4, 32}, {3, 42}, {2, 74}};
+    if (d.max_seq_len >= 2048 && clusters <= 4) return 16;
+    const uint32_t per_sm = d.head_dim <= 64 ? 2 : 1, most = rows == 1 ? (d.max_seq_len + 31) / 32 : std::max(2u, (d.max_seq_len + 95) / 96);
+    for (const auto& r : rule)
+        if (clusters <= r.clusters * per_sm && (rows == 1 || r.slices <= most) && !(r.slices == 3 && d.head_dim <= 64)) return std::min(r.slices, most);
     return 1;
-}
-// how many clusters of each size the device holds at once (none where it does not say)
-void ask_attn_fit(vb_ctx* c) {
-    AttnArgs a;
-    a.kv_fp16 = 1; a.block_table = c->block_table_dev; a.max_blocks = c->max_blocks; a.block_tokens = c->d.kv_block_tokens;
-    if (c->kv_map_ok) a.kv_map = c->kv_map;
-    a.Hq = c->hq; a.Hkv = c->hkv; a.D = c->d.head_dim; a.batch = 1; a.tokens_per_split = c->tokens_per_split;
-    for (int i = 0; i < ATTN_SPLIT_SIZES; ++i) {
-        int n = 0;
-        a.max_splits = attn_split_sizes[i];
-        if (attention_resident(a, &n) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        c->attn_fit[i] = n > 0 ? (uint32_t)n : 0;
-    }
 }
 
 // Steps of a few rows (few_i8) leave to the fp32 kernels what the integer GEMV leaves to them: there 24 bits of a row are no gain (a product's
@@ -568,7 +555,12 @@ cudaError_t enqueue_step(vb_ctx* c, SeqState* state, bool with_head, const StepI
         a.block_table = io.block_table; a.max_blocks = c->max_blocks; a.block_tokens = d.kv_block_tokens;
         if (c->kv_map_ok) { a.kv_map = c->kv_map; a.kv_map_row0 = (uint32_t)((uint64_t)l * (c->kv_layer_elems / d.head_dim)); }
         a.state = state; a.Hq = c->hq; a.Hkv = c->hkv; a.D = d.head_dim; a.batch = B;
-        a.max_splits = c->n_splits ? c->n_splits : pick_attn_splits(c, B); a.tokens_per_split = c->tokens_per_split; a.scratch = c->attn_scratch;
+        {
+            // (asked for more than eight: only where the rule would take them too)
+            const uint32_t clusters = B * attention_clusters(a);
+            a.max_splits = c->n_splits ? std::min(c->n_splits, clusters <= 4 ? 16u : 8u) : pick_attn_splits(d, B, clusters);
+        }
+        a.tokens_per_split = c->tokens_per_split; a.scratch = c->attn_scratch;
         a.trace = next_trace(); a.err = c->err_word; a.stop = c->stop_word;
         if (io.causal_chunk && c->prefill_flash && attention_prefill_supported(c->hq, c->hkv, d.head_dim))
             VB_TRY(attention_prefill(lcfg(c, true), io.attn_out, io.q, kv_layer, io.block_table, io.first, B, c->hq, c->hkv, d.head_dim, d.kv_block_tokens, io.split_attn));
@@ -764,7 +756,6 @@ int32_t vb_create(const vb_model_desc* desc, int32_t device, vb_ctx** out) {
     // the decode attention's tensor-core path stages whole KV blocks with tiled TMA copies
     c->kv_map_ok = d.kv_block_tokens == 16 && attn_make_kv_map(c->kv_map, c->kv_pool, c->kv_layer_elems * d.n_layers / d.head_dim, d.head_dim);
     VB_CREATE_TRY(dev_alloc(&c->block_table_dev, (uint64_t)d.max_batch * c->max_blocks));
-    ask_attn_fit(c);
     c->block_table_host.assign((size_t)d.max_batch * c->max_blocks, 0);
     VB_CREATE_CUDA(cudaMemsetAsync(c->block_table_dev, 0, (size_t)d.max_batch * c->max_blocks * 4, c->stream));
     c->free_blocks.reserve(c->n_blocks);
@@ -1462,7 +1453,7 @@ int32_t vb_set_option(vb_ctx* c, const char* name, int64_t value) {
         return VB_OK;
     }
     if (!strcmp(name, "attn_splits")) {
-        VB_REQUIRE(value >= 1 && value <= 16, "vb_set_option: attn_splits is 1..16 (a thread-block cluster)");
+        VB_REQUIRE(value >= 0 && value <= 16, "vb_set_option: attn_splits is 1..16 (a thread-block cluster), or 0: by the rows of a launch");
         c->n_splits = (uint32_t)value;
         return VB_OK;
     }

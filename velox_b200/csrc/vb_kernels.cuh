@@ -206,8 +206,8 @@ uint64_t attn_scratch_floats(uint32_t Hq, uint32_t D, uint32_t batch, uint32_t m
 uint32_t attn_pick_splits(uint32_t max_seq);
 uint32_t attn_tokens_per_split(uint32_t max_seq);
 cudaError_t attention(const LaunchCfg& lc, const AttnArgs& a);
-// how many clusters (of max_splits blocks, one for each sequence and head group) of this attention the device holds at once
-cudaError_t attention_resident(const AttnArgs& a, int* clusters);
+// clusters (of max_splits blocks each) of a sequence: KV heads times the groups their query heads are taken in
+uint32_t attention_clusters(const AttnArgs& a);
 cudaError_t attention_ex(const LaunchCfg& lc, const AttnArgs& a, float scale, size_t kv_batch_stride);
 
 // vb_attn_prefill.cu: causal attention of a prefill chunk (rows = consecutive positions of one sequence)
