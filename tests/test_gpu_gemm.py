@@ -68,10 +68,10 @@ def test_matmul_rows_parity(vb, oracle, dev, fmt, shape):
         assert np.max(np.abs(got[r] - want)) <= 3e-3 * scale
 
 
-# pairs of blocks: tiles of 256 weight rows by 128 rows of x, or 256 where the short ones take a second wave (10 weight tiles x 8)
+# ragged tiles in both directions, one wave of blocks and several
 @pytest.mark.parametrize("fmt", ["f16", "q4g32", "i8pc"])
 @pytest.mark.parametrize("in_dim,out_dim,n_rows", [(64, 5, 33), (128, 255, 128), (192, 257, 129), (96, 513, 255), (64, 2560, 1000), (128, 2305, 1025),
-                                                   (128, 3584, 2047), (64, 6144, 1755)])  # a second wave of long tiles, five of short ones
+                                                   (128, 3584, 2047), (64, 6144, 1755)])
 def test_matmul_rows_by_pairs_of_blocks(vb, oracle, dev, fmt, in_dim, out_dim, n_rows):
     c = code(oracle, fmt)
     w = oracle.fill_normal(out_dim * in_dim, 17, 1, 0.02).reshape(out_dim, in_dim)

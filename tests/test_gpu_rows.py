@@ -360,7 +360,7 @@ def test_few_rows_of_long_and_short_matrices(fmt, batch, ffn):
 @pytest.mark.parametrize("fmt", ["f16", "q4_0", "i8"])
 @pytest.mark.parametrize("n", [131, 1001])
 def test_gate_and_up_of_a_chunk_by_pairs_of_blocks(fmt, n):
-    """SwiGLU tiles of 128 and of 256 rows of x (10 pairs of gate and up rows, 8 tiles of 128: a second wave), both ragged."""
+    """SwiGLU tiles of a prompt of two and of eight tiles of 128 rows, all directions ragged."""
     w = L.FMT_I8PC if fmt == "i8" else FMTS[fmt][0]
     spec = LLAMA3_8B_INT4.scaled(name="pairs-" + fmt, d_model=256, n_layers=2, n_q_heads=4, n_kv_heads=2, head_dim=64, ffn_dim=2496, vocab=512,
                                  weight_fmt=w, head_fmt=L.FMT_F16, embed_fmt=L.FMT_F16)

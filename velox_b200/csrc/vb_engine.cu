@@ -256,8 +256,8 @@ bool tc_products_ok(vb_ctx* c) {
 
 // The same for the products that dequantise into tensor memory (vb_gemm_ts.cu), with the default operand parts.  They read only
 // the packed weights, so they win while the weights are what takes time, and they are the only ones a lean context can run.
-// Whole prompts, ms, here / on pairs of blocks over fp16 copies: 8B int4 64 rows 8.9 / 10.8, 128 rows 11.5 / 11.0 (not worth 28 GB of
-// copies in contexts that never see a longer prompt), 511 rows with them 19.2; 7B int8 64 rows 7.7 / 7.8, 128 rows 8.0 / 8.0, 199 rows 13.5 / 9.3.
+// Four layers of the 8B int4 shape and a last token, ms: 64 rows 1.23 (fp16 copies: 1.58; sixteen rows at a time: 3.3), 128
+// rows 1.55 (1.69), 160 rows 2.37 (2.00); the 7B int8 shape: 64 rows 1.23 (1.85), 128 1.28 (1.95), 200 2.07 (2.19), 256 2.12 (2.22).
 // Both make fp16 operands of the weights, so int4 matrices with a scale beyond 8188 (8 * 8188 = 65504) stay with the kernels that
 // apply the scales in fp32.
 bool weights_within_f16(const vb_ctx* c) {
@@ -265,10 +265,7 @@ bool weights_within_f16(const vb_ctx* c) {
         if (t.beyond_f16) return false;
     return true;
 }
-constexpr uint32_t TS_ROWS_MAX = 128;
-// int8 prompts stay with them up to 256 rows where no fp16 copies of the weights are there nor can be made: converting 13 GB of weights for
-// one prompt of the 7B shape takes longer than the difference above.
-constexpr uint32_t TS_I8_ROWS_WITHOUT_COPIES = 256;
+uint32_t ts_rows_max(const vb_ctx* c) { return c->d.weight_fmt == VB_FMT_I8PC ? 256 : 128; }
 bool ts_products_ok(vb_ctx* c) {
     if (gemm_tc_split != 2) return false;  // fewer parts: the products of vb_gemm_tc.cu
     const int roles[] = {VB_ROLE_WQ, VB_ROLE_WO, VB_ROLE_WGATE, VB_ROLE_WDOWN};
@@ -1134,19 +1131,15 @@ int32_t vb_prefill(vb_ctx* c, int32_t slot, const uint32_t* tokens, uint32_t n_t
     const bool tc_ok = gemm_ok && n_tokens > c->prefill_gemm_min && tc_products_ok(c);
     const uint32_t rows = std::min(c->prefill_rows, n_tokens - 1);
     const bool ts_ok = gemm_ok && n_tokens > c->prefill_ts_min && ts_products_ok(c);
-    bool use_ts = ts_ok && (!tc_ok || rows <= TS_ROWS_MAX);
+    bool use_ts = ts_ok && (!tc_ok || rows <= ts_rows_max(c));
     const bool use_tc = use_ts || tc_ok;
-    if (tc_ok && ts_ok && !use_ts && c->d.weight_fmt == VB_FMT_I8PC && rows <= TS_I8_ROWS_WITHOUT_COPIES) {
-        if ((rc = ensure_f16_copies(c)) != VB_OK) return rc;
-        use_ts = !c->f16_pool;
-    }
     uint32_t P = use_tc ? rows : c->prefill_chunk;
     if (use_tc || (P >= 2 && P <= 32 && c->d.tp_size <= 1 && 2 * n_tokens > P)) {
         // Rows the chunk buffers hold: two sizes, short prompts and the longest chunk of this context, so that prompts of growing
         // length meet one allocation of each and no more (buffers that doubled cost every length that crossed a power of two
         // 4 to 7 ms of an 11 ms prompt).
         uint32_t cap = P;
-        if (use_tc) cap = use_ts && rows <= TS_ROWS_MAX ? TS_ROWS_MAX : std::max(rows, std::min(c->prefill_rows, c->d.max_seq_len));
+        if (use_tc) cap = use_ts && rows <= ts_rows_max(c) ? ts_rows_max(c) : std::max(rows, std::min(c->prefill_rows, c->d.max_seq_len));
         auto buffers = [&]() {
             const int32_t r = ensure_chunk_buffers(c, cap);
             return r != VB_OK || !use_tc ? r : use_ts ? ensure_ts_ws(c, cap) : ensure_tc_ws(c, cap, false);

@@ -9,13 +9,12 @@
 //     (q-8)*s rounded once; int8 per channel: the integer, exact, the row scale is applied to the fp32
 //     accumulator in the epilogue), either once into a resident copy the engine keeps or per call into the
 //     workspace; fp16 matrices are used where they lie;
-//   * k_gemm_pair (more than 32 rows): pairs of SMs, a tile of 256 weight rows by 128 or 256 rows of x (cta_group::2; see there);
-//   * k_gemm_tc (decode batches of up to 32 rows): one block per tile of 128 weight rows (the M of the instruction, = tensor-memory
-//     lanes) by 32 rows of x (N, = tensor-memory columns).
-// In both an elected lane of warp 0 issues the TMA copies of 128-byte-swizzled [rows][64] fp16 boxes into a ring of stages, one of
-// warp 1 tcgen05.mma (K = 16 steps of a stage) and hands each stage back with tcgen05.commit, all warps read the accumulator with
-// tcgen05.ld and write the epilogue (store / residual add / SiLU(gate)*up with the two accumulators of the gate and up matrices side
-// by side in tensor memory).
+//   * k_gemm_tc: one block per tile of 128 weight rows (the M of the instruction, = tensor-memory lanes) by 32 or
+//     128 rows of x (N, = tensor-memory columns).  An elected lane of warp 0 issues the TMA copies of 128-byte-swizzled
+//     [128][64] fp16 boxes into a ring of stages, one of warp 1 tcgen05.mma (four K=16 steps per
+//     stage) and hands each stage back with tcgen05.commit, all four warps read the accumulator with
+//     tcgen05.ld and write the epilogue (store / residual add / SiLU(gate)*up with the two accumulators of the
+//     gate and up matrices side by side in tensor memory).
 // Every wait is bounded; a wait that runs out sets a block-wide abort flag and the library's error word, the
 // block still frees its tensor memory and returns.
 #include <cuda.h>
@@ -28,16 +27,18 @@
 namespace vb {
 namespace {
 
-constexpr int BM = 128;      // weight rows of a block
-constexpr int BN32 = 32;     // rows of x of k_gemm_tc's tiles
+constexpr int BM = 128;      // weight rows per tile (UMMA M)
+                             // rows of x per tile (UMMA N): 32 or 128, a template parameter of the kernel
 constexpr int BK = 64;       // K extent of a stage: 64 fp16 = one 128-byte swizzle row
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KB: one box of 128 rows
-constexpr int RING_BYTES = 192 * 1024;   // the ring of stages
-constexpr int SMEM_BYTES = RING_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+// the ring of stages fills 192 KB; PER_SM = 2: 96 KB, so that two blocks share an SM and one block's prologue and epilogue
+// overlap the other's main loop
+constexpr int RING_BYTES = 192 * 1024;
+__host__ __device__ constexpr int smem_bytes_for(int per_sm) { return RING_BYTES / per_sm + 1024 /* alignment slack */ + 256 /* barriers */; }
 
 // instruction descriptor of tcgen05.mma kind::f16: fp32 accumulate (bits 4-5 = 1), A and B fp16 (formats 0),
 // both K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24
-__host__ __device__ constexpr uint32_t idesc_for(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+__host__ __device__ constexpr uint32_t idesc_for(int bn) { return (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
 
 // shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: start address >> 4 in bits 0-13,
 // leading byte offset (unused with a swizzle; 1) in bits 16-29, stride between groups of 8 rows = 1024 bytes
@@ -82,7 +83,7 @@ struct GemmParams {
     // counter sums the partials in split order (the same bits whoever is last) and runs the epilogue
     float* part;          // [split][tile][BN / 32][32][128]
     uint32_t* counters;   // [tile], zero between launches (the last block puts the zero back)
-    // Operand splitting (k_gemm_pair, template parameters XP and WP): fp16 holds 11 significant bits, and over 32 layers and thousands of cached
+    // Operand splitting (prefill chunks, template parameters XP and WP): fp16 holds 11 significant bits, and over 32 layers and thousands of cached
     // positions that rounding reaches the logits (2.8e-2 at 2048 rows of the 8B shape).  x_parts = 2: x = x_hi + x_lo,
     // both fp16, x_lo rows lie `x_lo_row` rows below x_hi in the same tensor map; w_parts = 2: W = W_hi + W_lo likewise
     // (second tensor maps).  The products W_hi.x_hi + W_hi.x_lo + W_lo.x_hi accumulate into the same tensor-memory
@@ -90,15 +91,19 @@ struct GemmParams {
     uint32_t x_lo_row;
 };
 
-template <bool DUAL>
-__global__ void __launch_bounds__(128, 1)
-k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-    constexpr int BN = BN32, W_TILES = DUAL ? 2 : 1;
-    constexpr int X_BYTES = BN * BK * 2;
-    constexpr int STAGE_BYTES = W_TILES * TILE_BYTES + X_BYTES;  // [W (,W2)][x]
-    constexpr int STAGES = RING_BYTES / STAGE_BYTES;
-    constexpr int X_OFF = W_TILES * TILE_BYTES;
-    constexpr uint32_t IDESC = idesc_for(BM, BN);
+// XP, WP: parts of x and of the weights (1 or 2); compile-time, so that every descriptor is a base plus a constant
+template <bool DUAL, int BN, int PER_SM, int XP, int WP>
+__global__ void __launch_bounds__(128, PER_SM)
+k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
+          const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wl, const __grid_constant__ CUtensorMap map_wl2,
+          const GemmParams p) {
+    constexpr int W_TILES = DUAL ? 2 : 1;
+    constexpr int X_BYTES = BN * BK * 2;                        // one part of the x operand of a stage
+    constexpr int STAGE_BYTES = W_TILES * WP * TILE_BYTES + XP * X_BYTES;  // [W hi (,W2 hi)][W lo (,W2 lo)][x hi][x lo]
+    constexpr int STAGES = RING_BYTES / PER_SM / STAGE_BYTES;
+    static_assert(STAGES >= 2, "ring depth");
+    constexpr int X_OFF = W_TILES * WP * TILE_BYTES;
+    constexpr uint32_t IDESC = idesc_for(BN);
     constexpr uint32_t TMEM_COLS = DUAL ? 2 * BN : BN;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzled tiles want 1024-byte alignment
@@ -109,6 +114,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    // the tiles of x are the fastest block index: the blocks that share a weight tile run together and it comes
+    // from DRAM once
     const int row0 = blockIdx.y * BM, tok0 = blockIdx.x * BN;
     const int nk_all = (int)((p.K + BK - 1) / BK);
     const int kb_first = (int)(((long long)nk_all * blockIdx.z) / gridDim.z), kb_last = (int)(((long long)nk_all * (blockIdx.z + 1)) / gridDim.z);
@@ -146,7 +153,14 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             const int kx = (kb_first + kb) * BK;
             tma_load_2d(st, &map_w, kx, row0, full);
             if (DUAL) tma_load_2d(st + TILE_BYTES, &map_w2, kx, row0, full);
-            tma_load_2d(st + X_OFF, &map_x, kx, tok0, full);
+            if (WP == 2) {
+                tma_load_2d(st + W_TILES * TILE_BYTES, &map_wl, kx, row0, full);
+                if (DUAL) tma_load_2d(st + (W_TILES + 1) * TILE_BYTES, &map_wl2, kx, row0, full);
+            }
+            for (int xp = 0; xp < XP; ++xp) {
+                const int xr = tok0 + xp * (int)p.x_lo_row;
+                tma_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, xr, full);
+            }
         }
     } else if (warp == 1 && go) {
         // ---- tensor-core issue: the warp waits together, an elected lane issues (see vb_tma.cuh) ----
@@ -158,11 +172,18 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
                 const uint64_t da = smem_desc(st), da2 = smem_desc(st + TILE_BYTES), db = smem_desc(st + X_OFF);
+                const uint64_t dal = smem_desc(st + W_TILES * TILE_BYTES), dal2 = smem_desc(st + (W_TILES + 1) * TILE_BYTES), dbl = smem_desc(st + X_OFF + X_BYTES);
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k) {  // 16 fp16 = 32 bytes further along the swizzled row: +2 in the address field
                     const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
                     mma_f16(tmem, da + 2u * k, db + 2u * k, IDESC, acc);
-                    if (DUAL) mma_f16(tmem + BN, da2 + 2u * k, db + 2u * k, IDESC, acc);
+                    if (XP == 2) mma_f16(tmem, da + 2u * k, dbl + 2u * k, IDESC, 1u);
+                    if (WP == 2) mma_f16(tmem, dal + 2u * k, db + 2u * k, IDESC, 1u);
+                    if (DUAL) {
+                        mma_f16(tmem + BN, da2 + 2u * k, db + 2u * k, IDESC, acc);
+                        if (XP == 2) mma_f16(tmem + BN, da2 + 2u * k, dbl + 2u * k, IDESC, 1u);
+                        if (WP == 2) mma_f16(tmem + BN, dal2 + 2u * k, db + 2u * k, IDESC, 1u);
+                    }
                 }
                 mma_commit(bars + (STAGES + s) * 8);  // the stage is free again once these products have read it
                 if (kb == nk - 1) mma_commit(bar_accum);
@@ -263,199 +284,6 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     tc_fence_before();
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-}
-
-// ---- the same products by pairs of SMs -----------------------------------------------------------------------------
-// cta_group::2: the two blocks of a cluster multiply one tile of 256 weight rows (128 in each block's tensor memory; gate and up two such
-// sets of columns) by BN rows of x, each block's shared memory holding its own weight rows and HALF of the rows of x.  One elected thread
-// of the first block issues for both; its barriers count both blocks' copies, and a commit arrives in both.
-// What bounds it: L2 delivers about 37 bytes a clock to every SM at once.  128 x 128 tiles of single blocks ask for 96 KB per 1536 tensor
-// clocks (gate and up, x and W in two parts) or 64 KB per 768, so they waited for it 40 % of their time; a pair with BN = 256 asks
-// for 96 KB per 3072 and 64 KB per 1536, and the tensor cores (under the power cap of a long chunk: 1.3 PFLOP/s of the part products) are
-// what is left, with the last wave of tiles.  Prompts, single blocks -> pairs, ms: 8B int4 128 rows 14.2 -> 11.6 (group-64), 512 23.2 -> 20.2,
-// 3000 133.8 -> 115.9; 8B fp16 100 rows 15.2 -> 10.6; 7B int8 300 rows 16.0 -> 10.9, 1999 55.9 -> 48.8; 135M fp32 300 rows 3.38 -> 2.91.
-constexpr int PAIR_THREADS = 256;
-__device__ __forceinline__ uint32_t pair_addr(uint32_t local, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-    return r;
-}
-// into this block's shared memory, counted off at a barrier of either block
-__device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ void pair_mma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
-                 ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void pair_commit(uint32_t bar) {  // arrives at this offset in both blocks
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// XP, WP: parts of x and of the weights (1 or 2); compile-time, so that every descriptor is a base plus a constant
-template <bool DUAL, int BN, int XP, int WP>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-k_gemm_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
-            const __grid_constant__ CUtensorMap map_wl, const __grid_constant__ CUtensorMap map_wl2, const GemmParams p) {
-    constexpr int W_TILES = DUAL ? 2 : 1;
-    constexpr int X_BYTES = BN / 2 * BK * 2;                               // this block's half of one part of x
-    constexpr int X_OFF = W_TILES * WP * TILE_BYTES;
-    constexpr int STAGE_BYTES = X_OFF + XP * X_BYTES;                      // [W hi (,W2 hi)][W lo (,W2 lo)][x hi][x lo]
-    constexpr int STAGES = RING_BYTES / STAGE_BYTES;
-    static_assert(STAGES >= 2, "ring depth");
-    constexpr uint32_t IDESC = idesc_for(2 * BM, BN);
-    constexpr uint32_t TMEM_COLS = DUAL ? 2 * BN : BN;
-    extern __shared__ unsigned char smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bars = base + STAGES * STAGE_BYTES;                     // full[STAGES] (the first block's count), empty[STAGES], accum
-    const uint32_t bar_accum = bars + 2 * STAGES * 8;
-    unsigned char* gen = smem_raw + (base - smem_u32(smem_raw));
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + STAGES * STAGE_BYTES + (2 * STAGES + 1) * 8);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-
-    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, rank = blockIdx.x & 1;
-    // rows of x fastest: the pairs that share a weight tile run together and it comes from DRAM once
-    const uint32_t tok_tiles = (p.n_rows + BN - 1) / BN, tile = blockIdx.x >> 1;
-    const int row0 = (int)((tile / tok_tiles) * 2 + rank) * BM, tok0 = (int)(tile % tok_tiles) * BN;
-    const int nk = (int)((p.K + BK - 1) / BK);
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < 2 * STAGES; ++s) mbar_init(bars + s * 8, 1);
-        mbar_init(bar_accum, 1);
-        *abort_flag = stop_set(p.stop) ? 1u : 0u;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();  // both blocks' barriers and tensor memory are there
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
-
-    pdl_wait();  // x (and converted weights) come from the kernels before this one
-    pdl_launch_dependents();
-
-    if (warp == 0 && go) {
-        // ---- producer: this block's copies, counted by the first block ----
-        if (elect_one()) {
-            const uint32_t full0 = pair_addr(bars, 0);
-            int kb = 0;
-            for (; kb < nk; ++kb) {
-                const int s = kb % STAGES;
-                const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-                if (!wait_or_abort(bars + (STAGES + s) * 8, ph ^ 1u, abort_flag, p.stop)) break;
-                const uint32_t full = full0 + s * 8, st = base + s * STAGE_BYTES;
-                if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * STAGE_BYTES);
-                const int kx = kb * BK;
-                pair_load_2d(st, &map_w, kx, row0, full);
-                if (DUAL) pair_load_2d(st + TILE_BYTES, &map_w2, kx, row0, full);
-                if (WP == 2) {
-                    pair_load_2d(st + W_TILES * TILE_BYTES, &map_wl, kx, row0, full);
-                    if (DUAL) pair_load_2d(st + (W_TILES + 1) * TILE_BYTES, &map_wl2, kx, row0, full);
-                }
-#pragma unroll
-                for (int xp = 0; xp < XP; ++xp) pair_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, tok0 + (int)rank * (BN / 2) + xp * (int)p.x_lo_row, full);
-            }
-            // The last stages come back too before this block leaves: nothing orders their arrivals, sent from the other SM, before the
-            // accumulator's, and one that came later would count at a barrier of the block that has this shared memory next.
-            if (kb == nk)
-                for (kb = nk > STAGES ? nk - STAGES : 0; kb < nk; ++kb)
-                    if (!wait_or_abort(bars + (STAGES + kb % STAGES) * 8, (uint32_t)(kb / STAGES) & 1u, abort_flag, p.stop)) break;
-        }
-    } else if (warp == 1 && rank == 0 && go) {
-        // ---- tensor-core issue for both blocks ----
-        for (int kb = 0; kb < nk; ++kb) {
-            const int s = kb % STAGES;
-            const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
-            if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
-            tc_fence_after();
-            const uint32_t st = base + s * STAGE_BYTES;
-            if (elect_one()) {
-                const uint64_t da = smem_desc(st), da2 = smem_desc(st + TILE_BYTES), db = smem_desc(st + X_OFF);
-                const uint64_t dal = smem_desc(st + W_TILES * TILE_BYTES), dal2 = smem_desc(st + (W_TILES + 1) * TILE_BYTES), dbl = smem_desc(st + X_OFF + X_BYTES);
-#pragma unroll
-                for (int k = 0; k < BK / 16; ++k) {
-                    const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
-                    pair_mma_f16(tmem, da + 2u * k, db + 2u * k, IDESC, acc);
-                    if (XP == 2) pair_mma_f16(tmem, da + 2u * k, dbl + 2u * k, IDESC, 1u);
-                    if (WP == 2) pair_mma_f16(tmem, dal + 2u * k, db + 2u * k, IDESC, 1u);
-                    if (DUAL) {
-                        pair_mma_f16(tmem + BN, da2 + 2u * k, db + 2u * k, IDESC, acc);
-                        if (XP == 2) pair_mma_f16(tmem + BN, da2 + 2u * k, dbl + 2u * k, IDESC, 1u);
-                        if (WP == 2) pair_mma_f16(tmem + BN, dal2 + 2u * k, db + 2u * k, IDESC, 1u);
-                    }
-                }
-                pair_commit(bars + (STAGES + s) * 8);  // the stage is free again, in both blocks, once these products have read it
-                if (kb == nk - 1) pair_commit(bar_accum);
-            }
-            __syncwarp();
-        }
-    }
-    __syncwarp();
-
-    // ---- epilogue: warps w and w + 4 own tensor-memory lanes 32 (w % 4) .. + 31 = weight rows, half of the columns each ----
-    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
-    tc_fence_after();
-    const bool good = __syncthreads_and(ok && !*abort_flag);
-    if (good) {
-        const uint32_t o = (uint32_t)row0 + (warp & 3) * 32 + lane;
-        const bool o_ok = o < p.out_dim;
-        const float sc = (p.row_scale && o_ok) ? __half2float(p.row_scale[o]) : 1.0f;
-        const float sc2 = (DUAL && p.row_scale2 && o_ok) ? __half2float(p.row_scale2[o]) : 1.0f;
-        const uint32_t lane_addr = tmem + (((warp & 3) * 32u) << 16);
-#pragma unroll 1
-        for (int c0 = (int)(warp >> 2) * (BN / 2); c0 < (int)((warp >> 2) + 1) * (BN / 2); c0 += 32) {
-            if ((uint32_t)(tok0 + c0) >= p.n_rows) break;  // uniform over the warp
-            const uint32_t tl = (uint32_t)(tok0 + c0) + lane;
-            const bool live = tl < p.n_rows && (!p.state || p.state[tl].active);
-            const uint32_t live_mask = __ballot_sync(0xFFFFFFFFu, live);
-            uint32_t v[32], u[DUAL ? 32 : 1];
-            tmem_ld32(lane_addr + c0, v);
-            if constexpr (DUAL) tmem_ld32(lane_addr + BN + c0, u);
-            if (!o_ok) continue;
-            float* d0 = p.dst + (size_t)(tok0 + c0) * p.dst_stride + o;
-            if (!DUAL && p.epilogue == EPI_RESIDUAL) {
-                // all 32 residual values first (independent loads), then the sums: one memory round trip, not 32
-                float res[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) res[j] = ((live_mask >> j) & 1u) ? __ldcg(d0 + (size_t)j * p.dst_stride) : 0.0f;
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if ((live_mask >> j) & 1u) d0[(size_t)j * p.dst_stride] = res[j] + __uint_as_float(v[j]) * sc;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if (!((live_mask >> j) & 1u)) continue;
-                    const float a = __uint_as_float(v[j]) * sc;
-                    if constexpr (DUAL) {
-                        const float up = __uint_as_float(u[j]) * sc2;
-                        d0[(size_t)j * p.dst_stride] = (a / (1.0f + expf(-a))) * up;
-                    } else {
-                        d0[(size_t)j * p.dst_stride] = a;
-                    }
-                }
-            }
-        }
-    } else {
-        if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x40u);
-        // let copies and products that are still in flight land before the memory they use is given back
-        const long long t0 = clock64();
-        while (go && clock64() - t0 < 20000000LL) { }
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();  // neither block's memory goes while the other one's products may still use it
-    tc_fence_after();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
 // ---- operand conversion -------------------------------------------------------------------------------------
@@ -592,41 +420,12 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t K, uint32
 bool gemm_tc_split_k = true;  // vb_set_option("decode_split_k", 0): one block per tile of 128 weight rows
 int gemm_tc_split = 2;  // vb_set_option("prefill_split", n): prefill chunks multiply 0: fp16(x).fp16(W); 1: x as hi + lo; 2: x and W as hi + lo
 
-template <bool DUAL>
+template <bool DUAL, int BN, int PER_SM, int XP, int WP>
 static cudaError_t tc_launch(const LaunchCfg& lc, const dim3& grid, const CUtensorMap* m, const GemmParams& p) {
     static std::atomic<uint64_t> opted{0};
-    const cudaError_t e = once_per_device(opted, []() { return cudaFuncSetAttribute(k_gemm_tc<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+    const cudaError_t e = once_per_device(opted, []() { return cudaFuncSetAttribute(k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_for(PER_SM)); });
     if (e != cudaSuccess) return e;
-    return launch(lc, k_gemm_tc<DUAL>, grid, dim3(128), SMEM_BYTES, m[0], m[1], m[2], p);
-}
-
-template <bool DUAL, int BN, int XP, int WP>
-static cudaError_t pair_launch(const LaunchCfg& lc, const CUtensorMap* m, const GemmParams& p) {
-    static std::atomic<uint64_t> opted{0};
-    const cudaError_t e = once_per_device(opted, []() { return cudaFuncSetAttribute(k_gemm_pair<DUAL, BN, XP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * ((p.n_rows + BN - 1) / BN) * ((p.out_dim + 2 * BM - 1) / (2 * BM)));
-    cfg.blockDim = dim3(PAIR_THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = lc.stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
-    if (lc.pdl) {
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.numAttrs = 2;
-    }
-    cfg.attrs = attr;
-    if (lc.counter) ++*lc.counter;
-    return cudaLaunchKernelEx(&cfg, k_gemm_pair<DUAL, BN, XP, WP>, m[0], m[1], m[2], m[3], m[4], p);
-}
-template <bool DUAL, int BN>
-static cudaError_t pair_parts(const LaunchCfg& lc, const CUtensorMap* m, const GemmParams& p, uint32_t x_parts, uint32_t w_parts) {
-    if (x_parts == 1) return pair_launch<DUAL, BN, 1, 1>(lc, m, p);
-    return w_parts == 1 ? pair_launch<DUAL, BN, 2, 1>(lc, m, p) : pair_launch<DUAL, BN, 2, 2>(lc, m, p);
+    return launch(lc, k_gemm_tc<DUAL, BN, PER_SM, XP, WP>, grid, dim3(128), smem_bytes_for(PER_SM), m[0], m[1], m[2], m[3], m[4], p);
 }
 
 // fp16 [rows][cols] copy of a weight matrix (int8 per channel: the integers; the row scale stays with the caller)
@@ -705,13 +504,8 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
         wh[i] = hi;
         wl[i] = lo;
     }
-    // Rows of x in a pair's tile: 256, or 128 where those take fewer waves of the 74 pairs by more than the seventh that a row costs more
-    // in the short tiles (8B int4, 3000 rows: gate and up in 19 waves of short tiles 122.0 ms, in 10 of long ones 115.9; 512 rows:
-    // O and down in one wave of short tiles 20.2, everything in long ones 23.5).
-    auto waves = [&](uint32_t bn) { return (((n_rows + bn - 1) / bn) * ((out_dim + 2 * BM - 1) / (2 * BM)) + 73) / 74; };
-    const uint32_t pair_bn = waves(128) * 8 < waves(256) * 14 ? 128 : 256;
     CUtensorMap maps[5];  // W, W2, x, W lo, W2 lo
-    if (!make_map(&maps[0], wh[0], out_dim, K) || !make_map(&maps[2], xh, rows_pad * x_parts, K, narrow ? BN32 : pair_bn / 2)) return cudaErrorNotSupported;
+    if (!make_map(&maps[0], wh[0], out_dim, K) || !make_map(&maps[2], xh, rows_pad * x_parts, K, narrow ? 32 : BM)) return cudaErrorNotSupported;
     maps[1] = maps[0];
     if (dual && !make_map(&maps[1], wh[1], out_dim, K)) return cudaErrorNotSupported;
     maps[3] = maps[0]; maps[4] = maps[1];
@@ -740,10 +534,13 @@ cudaError_t gemm_tc(const LaunchCfg& lc, const GemvArgs& a, void* workspace, uin
             if ((uint64_t)splits * tiles * 128 * 32 * 4 > WS_PART_BYTES || tiles * 4 > WS_COUNTER_BYTES) splits = 1;
         }
         const dim3 grid(1, tiles, splits);
-        return dual ? tc_launch<true>(lc, grid, maps, p) : tc_launch<false>(lc, grid, maps, p);
+        return dual ? tc_launch<true, 32, 1, 1, 1>(lc, grid, maps, p) : tc_launch<false, 32, 1, 1, 1>(lc, grid, maps, p);
     }
-    if (pair_bn == 256) return dual ? pair_parts<true, 256>(lc, maps, p, x_parts, w_parts) : pair_parts<false, 256>(lc, maps, p, x_parts, w_parts);
-    return dual ? pair_parts<true, 128>(lc, maps, p, x_parts, w_parts) : pair_parts<false, 128>(lc, maps, p, x_parts, w_parts);
+    const dim3 grid((unsigned)(rows_pad / 128), (out_dim + BM - 1) / BM);
+    // two blocks per SM where half a ring still holds two stages
+    if (x_parts == 1) return dual ? tc_launch<true, 128, 2, 1, 1>(lc, grid, maps, p) : tc_launch<false, 128, 2, 1, 1>(lc, grid, maps, p);
+    if (w_parts == 1) return dual ? tc_launch<true, 128, 1, 2, 1>(lc, grid, maps, p) : tc_launch<false, 128, 2, 2, 1>(lc, grid, maps, p);
+    return dual ? tc_launch<true, 128, 1, 2, 2>(lc, grid, maps, p) : tc_launch<false, 128, 1, 2, 2>(lc, grid, maps, p);
 }
 
 }  // namespace vb

@@ -1,5 +1,5 @@
 // Products of many rows of x on the 5th-generation tensor cores with the WEIGHTS DEQUANTISED INTO TENSOR MEMORY: prompts of
-// int4 group-32 and int8 per-channel models, where the weights are what takes time (17 to 128 rows) or where there is
+// int4 group-32 and int8 per-channel models, where the weights are what takes time (17 to 128 or 256 rows) or where there is
 // no canonical copy to convert (lean contexts, any number of rows).
 //     dst[t][o] = sum_k x[t][k] * W[o][k]
 //
@@ -26,7 +26,7 @@
 // 92 / 127 / 167, down 34 / 51 / 63.  With four rows at a time on vb_gemv_mma.cu a 119-row prompt of the 72B shape took 30 passes
 // over 36 GB of weights (0.36 s), now it takes 45 ms.  128 rows and more are bound by the issue: a stage of 12 products (64 of K,
 // 128 columns) takes ~1400 clocks where the products alone take 770, which two resident blocks overlap only in part.  There
-// the pairs of blocks of vb_gemm_tc.cu are faster (a prompt, ms: 8B int4, 128 rows 11.0, here 11.5; 7B int8, 199 rows 9.3, here 13.5).
+// the kernel of vb_gemm_tc.cu, whose operands are both in shared memory, is faster (gate/up of 512 rows 342 us, here 570).
 // Every wait is bounded; one that runs out sets a block-wide abort flag and the library's error word.
 #include <cooperative_groups.h>
 #include <cuda.h>
