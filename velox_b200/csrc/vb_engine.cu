@@ -461,20 +461,22 @@ StepIO decode_io(vb_ctx* c) {
 
 // Slices of a context in the decode attention (the blocks of a cluster), by the model, the rows of the launch and the longest context alone:
 // the order of the merge, and with it the last bits, does not depend on the chip.  As many as run all their clusters at once on a chip
-// whose GPCs are of uneven size (one measured: 15 clusters of 8 blocks, 33 of 4, 45 of 3, 74 of 2; heads of up to 64: two blocks an SM): a
+// whose GPCs are of uneven size (one measured: 15 clusters of 8 blocks, 22 of 6, 33 of 4, 45 of 3, 74 of 2; heads of up to 64: two blocks an SM): a
 // cluster that waits for another to end costs a whole attention.  One for 32 tokens of the longest context, for several rows 96.
 // 8 layers and the head, us with 2 / 3 / 4 / 6 / 8 slices: 8B int4, contexts of 500, 1 sequence (8 clusters) 369 / 370 / 358 / 360 / 360, 2
 // 498 / 498 / 486 / 492 / 538, 4 526 / 527 / 518 / 570 / 608, 5 696 / 697 / 735 / 742 / 785, 8 701 / 763 / 743 / 800 / 886; of 3000, 1 447 / 421 / 400 /
 // 388 / 378, 2 576 / 549 / 529 / 521 / 578, 5 777 / 752 / 824 / 808 / 856; 7B int8, 3 sequences (12 clusters) of 500 703 / 716 / 701 / 710 / 704, of 3000
 // 778 / 764 / 741 / 736 / 722.  The 135M model, 8 sequences (24 clusters), 2 / 4 / 8: 250 rows 933 / 937 / 957, 3000 1230 / 1081 / 1034; three
-// slices of a head of 64 are slower than two.  Sixteen for four clusters at most (each takes most of a GPC, and how many GPCs have so many SMs
+// and six slices of a head of 64 are slower than two and four.  Sixteen for four clusters at most (each takes most of a GPC, and how many GPCs have so many SMs
 // differs from chip to chip): 3000 rows, 8 / 16, 7B int8 572 / 564, 135M 595 / 587; 1000 rows 548 / 559.
 uint32_t pick_attn_splits(const vb_model_desc& d, uint32_t rows, uint32_t clusters) {
-    static constexpr struct { uint32_t slices, clusters; } rule[] = {{8, 14}, {4, 32}, {3, 42}, {2, 74}};
+    static constexpr struct { uint32_t slices, clusters, from; } rule[] = {{8, 14, 1}, {6, 18, 1024}, {4, 32, 1}, {3, 44, 1}, {2, 74, 1}};
     if (d.max_seq_len >= 2048 && clusters <= 4) return 16;
     const uint32_t per_sm = d.head_dim <= 64 ? 2 : 1, most = rows == 1 ? (d.max_seq_len + 31) / 32 : std::max(2u, (d.max_seq_len + 95) / 96);
-    for (const auto& r : rule)
-        if (clusters <= r.clusters * per_sm && (rows == 1 || r.slices <= most) && !(r.slices == 3 && d.head_dim <= 64)) return std::min(r.slices, most);
+    for (const auto& r : rule) {
+        if (clusters > r.clusters * per_sm || d.max_seq_len < r.from || (r.slices % 3 == 0 && d.head_dim <= 64)) continue;
+        if (rows == 1 || r.slices <= most) return std::min(r.slices, most);
+    }
     return 1;
 }
 
