@@ -87,7 +87,7 @@ def test_reloaded_tensor_reaches_the_tensor_core_copies(spec):
 
 @pytest.mark.parametrize("fmt,batch,prefill_rows", [(L.FMT_Q4G32, 1, 160), (L.FMT_Q4G32, 1, 64), (L.FMT_I8PC, 1, 2048), (L.FMT_F16, 16, 100), (L.FMT_I8PC, 16, 100)])
 def test_a_wait_that_ran_out_ends_what_is_enqueued_behind_it(fmt, batch, prefill_rows):
-    """The stop word that such a wait sets, set by hand: a prompt of one or several chunks (pairs of blocks, operands in tensor memory) and a
+    """The stop word that such a wait sets, set by hand: a prompt of one or several chunks (both operands in shared memory, one in tensor memory) and a
     step of a batch (fp16 and int8 tensor-core products) start nothing and report a time-out at once; the context serves again afterwards."""
     spec = SPEC.scaled(name="stop", weight_fmt=fmt, head_fmt=fmt, embed_fmt=L.FMT_F16)
     eng = H.build_engine(spec, 5, 720, max_batch=batch)

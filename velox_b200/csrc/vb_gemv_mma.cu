@@ -2,11 +2,11 @@
 // short prompts, and batch 1 of the q4 group-64 format.
 //
 // Why mma.sync.  m16n8k16 issues every 8 clocks on each of an SM's four schedulers (measured; m16n8k32.s8 the same):
-// 128 weights a clock and SM for eight columns, where HBM delivers 41 int4 weights (11 of 16 bits).  So up to three
-// groups of eight columns cost no more time than the stream itself, without the detour through shared or tensor memory
+// 128 weights a clock and SM for eight columns, where HBM delivers 41 int4 weights (11 of 16 bits).  So the
+// products of up to three groups of eight columns take no longer than the stream, without the detour through shared or tensor memory
 // that tcgen05 operands take (dequantised hi + lo halves of int4 weights would be 164 bytes a clock of shared-memory
-// writes, more than an SM has).  What has to be kept down is instructions: 16 x 128 weights (1152 bytes) arrive every 50
-// clocks, 200 issue slots.
+// writes, more than an SM has).  What they cost is instructions and fragment reads (a step of 4 rows, one group: 1.82 ms, of 5, two
+// groups: 2.42): 16 x 128 weights (1152 bytes) arrive every 50 clocks, 200 issue slots.
 //
 // Weights.  A = 16 weight rows x 16 of K.  int4 group-32: a masked nibble IS an fp16 operand, the subnormal n * 2^-24 (bits 0-3)
 // or n * 2^-20 (bits 4-7, its x is stored divided by 16), exact: one AND per two weights and no conversion.  Groups keep their
