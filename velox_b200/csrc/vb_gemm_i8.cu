@@ -110,7 +110,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(bars + s * 8, 1); mbar_init(bars + (STAGES + s) * 8, 1); }
         mbar_init(bar_accum, 1);
-        *abort_flag = stop_set(p.stop) ? 1u : 0u;
+        *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -122,9 +122,8 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
 
-    if (warp == 0 && go) {
+    if (warp == 0) {
       if (elect_one()) {
         // weights do not depend on the kernel before this one: the whole ring of weight tiles is requested before the
         // dependency wait, the planes of x (written by the conversion kernel in front) after it
@@ -163,12 +162,14 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             tma_2d(st + W_TILES * I8_W_BYTES, &map_x, kx, 0, full);
         }
       }
-    } else if (warp == 1 && go) {
+    } else if (warp == 1) {
+        const bool stopped = stop_set(p.stop);  // an earlier kernel of this context gave up (looked at behind the first copies)
         // the warp waits together, an elected lane issues (vb_tma.cuh)
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
             if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
+            if (kb == 0 && __any_sync(0xFFFFFFFFu, stopped)) { *abort_flag = ABORT_STOPPED; break; }
             fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
@@ -198,7 +199,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, live);
         if (lane == 0) s_live_mask = m;
     }
-    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
+    const bool ok = wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
     fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     if (good) {
@@ -270,8 +271,7 @@ k_gemm_i8(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         }
     } else {
         if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x80u);
-        const long long t0 = clock64();
-        while (go && clock64() - t0 < 20000000LL) { }
+        abort_drain(abort_flag);
     }
     fence_before();
     __syncthreads();

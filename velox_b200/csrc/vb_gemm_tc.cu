@@ -124,7 +124,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(bars + s * 8, 1); mbar_init(bars + (STAGES + s) * 8, 1); }
         mbar_init(bar_accum, 1);
-        *abort_flag = stop_set(p.stop) ? 1u : 0u;
+        *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -136,12 +136,11 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
 
     pdl_wait();  // x (and converted weights) come from the kernels before this one
     pdl_launch_dependents();
 
-    if (warp == 0 && go) {
+    if (warp == 0) {
         // ---- producer: TMA copies into the ring ----
         if (elect_one())
         for (int kb = 0; kb < nk; ++kb) {
@@ -162,12 +161,14 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                 tma_load_2d(st + X_OFF + xp * X_BYTES, &map_x, kx, xr, full);
             }
         }
-    } else if (warp == 1 && go) {
+    } else if (warp == 1) {
+        const bool stopped = stop_set(p.stop);  // an earlier kernel of this context gave up (looked at behind the first copies)
         // ---- tensor-core issue: the warp waits together, an elected lane issues (see vb_tma.cuh) ----
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % STAGES;
             const uint32_t ph = (uint32_t)(kb / STAGES) & 1u;
             if (!__all_sync(0xFFFFFFFFu, wait_or_abort(bars + s * 8, ph, abort_flag, p.stop))) break;
+            if (kb == 0 && __any_sync(0xFFFFFFFFu, stopped)) { *abort_flag = ABORT_STOPPED; break; }
             tc_fence_after();
             const uint32_t st = base + s * STAGE_BYTES;
             if (elect_one()) {
@@ -194,7 +195,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     __syncwarp();
 
     // ---- epilogue: warp w owns tensor-memory lanes 32w..32w+31 = weight rows row0 + 32w + lane ----
-    const bool ok = go && wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
+    const bool ok = wait_or_abort(bar_accum, 0u, abort_flag, p.stop);
     tc_fence_after();
     const bool good = __syncthreads_and(ok && !*abort_flag);
     if (good) {
@@ -278,8 +279,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     } else {
         if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x40u);
         // let copies and products that are still in flight land before the memory they use is given back
-        const long long t0 = clock64();
-        while (go && clock64() - t0 < 20000000LL) { }
+        abort_drain(abort_flag);
     }
     tc_fence_before();
     __syncthreads();

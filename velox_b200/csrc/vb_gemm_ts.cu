@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     trace_mark(p.trace, 0);
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_AFULL && i < B_AEMPTY ? 4 : 1);
-        *abort_flag = stop_set(p.stop) ? 1u : 0u;
+        *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     // this block's part of K, in units
     const uint32_t n_units_all = p.K / F::unit, u0 = (uint32_t)((uint64_t)n_units_all * split / S), n_units = (uint32_t)((uint64_t)n_units_all * (split + 1) / S) - u0;
     constexpr int SPU = F::unit / 64;  // A stages per unit
-    uint32_t n_st = n_units * SPU;
+    const uint32_t n_st = n_units * SPU;
 
     // ---- dequantising warps: where this thread's weight row lies; the first units are requested before the dependency wait ----
     const uint32_t lg = warp & 3, row = lg * 32 + lane;  // tensor-memory lanes 32 * (warp % 4) .. + 31
@@ -222,8 +222,6 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     __syncthreads();
     ts_fence_after();
     const uint32_t tmem = *tmem_slot, tm_a = tmem + P::d_cols;
-    const bool go = !*abort_flag;  // an earlier kernel of this context gave up: nothing is started
-    if (!go) n_st = 0;
     pdl_wait();
     pdl_launch_dependents();
     trace_mark(p.trace, 1);
@@ -246,9 +244,11 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ---- tensor-core issue ----
+        const bool stopped = stop_set(p.stop);  // an earlier kernel of this context gave up (looked at behind the first copies)
         for (uint32_t i = 0; i < n_st; ++i) {
             const uint32_t xs = i % XS, as = i % AS;
             if (!ts_warp_wait(bar(B_XFULL + xs), (i / XS) & 1, abort_flag, p.stop) || !ts_warp_wait(bar(B_AFULL + as), (i / AS) & 1, abort_flag, p.stop)) break;
+            if (i == 0 && __any_sync(0xFFFFFFFFu, stopped)) { *abort_flag = ABORT_STOPPED; break; }
             ts_fence_after();
             if (elect_one()) {
                 const uint64_t bh = ts_desc(base + xs * P::x_stage), bl = ts_desc(base + xs * P::x_stage + NT * 128);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
         // ---- weights -> tensor memory ----
         const uint32_t lane_addr = (lg * 32u) << 16;
         uint32_t i = 0;
-        bool ok = go;
+        bool ok = true;
         for (uint32_t ub = 0; ub < n_units && ok; ub += F::depth) {
 #pragma unroll
             for (int d = 0; d < F::depth; ++d) {
@@ -377,8 +377,7 @@ __global__ void __launch_bounds__(TS_THREADS, 2) k_gemm_ts(const __grid_constant
     if (!good) {
         if (threadIdx.x == 0) report_wait(p.err, p.stop, 0x100u);
         // let copies and products that are still in flight land before the memory they use is given back
-        const long long c0 = clock64();
-        while (go && clock64() - c0 < 20000000LL) { }
+        abort_drain(abort_flag);
     }
     ts_fence_before();
     __syncthreads();

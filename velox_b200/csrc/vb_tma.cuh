@@ -65,7 +65,8 @@ __device__ __forceinline__ bool wait_or_stop(uint32_t bar, uint32_t parity, cons
         if (clock64() - t0 > (stop_set(stop) ? 20000000LL : 2000000000LL)) return false;
     }
 }
-// Bounded wait that also gives up as soon as another thread of the block has given up, or the stop word is set.
+// Bounded wait that also gives up as soon as another thread of the block has given up (abort_flag), or the stop word is set.
+constexpr uint32_t ABORT_WAITED = 1, ABORT_STOPPED = 2;
 __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, const uint32_t* stop) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
@@ -74,8 +75,15 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
         for (int i = 0; i < 128; ++i)
             if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
-        if (stop_set(stop) || clock64() - t0 > 2000000000LL) { *abort_flag = 1u; return false; }
+        if (stop_set(stop)) { *abort_flag = ABORT_STOPPED; return false; }
+        if (clock64() - t0 > 2000000000LL) { *abort_flag = ABORT_WAITED; return false; }
     }
+}
+// A block that gave up: what is still in flight lands before the memory that it uses is given back.  10 ms, 1 ms where only copies of its own
+// first stages can be (an earlier kernel gave up: no product was started).
+__device__ __forceinline__ void abort_drain(volatile uint32_t* abort_flag) {
+    const long long t0 = clock64(), limit = *abort_flag == ABORT_STOPPED ? 2000000LL : 20000000LL;
+    while (clock64() - t0 < limit) { }
 }
 // One lane of the (converged) warp, always the same one.  Tensor-core and TMA instructions take their operands from uniform
 // registers: under `lane == 0` the compiler has to make them uniform instruction by instruction (the latent attention's 36
