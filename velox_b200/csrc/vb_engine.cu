@@ -462,7 +462,8 @@ StepIO decode_io(vb_ctx* c) {
 // Slices of a context in the decode attention (the blocks of a cluster), by the model, the rows of the launch and the longest context alone:
 // the order of the merge, and with it the last bits, does not depend on the chip.  As many as run all their clusters at once on a chip
 // whose GPCs are of uneven size (one measured: 15 clusters of 8 blocks, 22 of 6, 33 of 4, 45 of 3, 74 of 2; heads of up to 64: two blocks an SM): a
-// cluster that waits for another to end costs a whole attention.  One for 32 tokens of the longest context, for several rows 96.
+// cluster that waits for another to end costs a whole attention.  One for 32 tokens of the longest context, but two; for several rows or heads of
+// 64 one for 96.
 // 8 layers and the head, us with 2 / 3 / 4 / 6 / 8 slices: 8B int4, contexts of 500, 1 sequence (8 clusters) 369 / 370 / 358 / 360 / 360, 2
 // 498 / 498 / 486 / 492 / 538, 4 526 / 527 / 518 / 570 / 608, 5 696 / 697 / 735 / 742 / 785, 8 701 / 763 / 743 / 800 / 886; of 3000, 1 447 / 421 / 400 /
 // 388 / 378, 2 576 / 549 / 529 / 521 / 578, 5 777 / 752 / 824 / 808 / 856; 7B int8, 3 sequences (12 clusters) of 500 703 / 716 / 701 / 710 / 704, of 3000
@@ -472,11 +473,9 @@ StepIO decode_io(vb_ctx* c) {
 uint32_t pick_attn_splits(const vb_model_desc& d, uint32_t rows, uint32_t clusters) {
     static constexpr struct { uint32_t slices, clusters, from; } rule[] = {{8, 14, 1}, {6, 18, 1024}, {4, 32, 1}, {3, 44, 1}, {2, 74, 1}};
     if (d.max_seq_len >= 2048 && clusters <= 4) return 16;
-    const uint32_t per_sm = d.head_dim <= 64 ? 2 : 1, most = rows == 1 ? (d.max_seq_len + 31) / 32 : std::max(2u, (d.max_seq_len + 95) / 96);
-    for (const auto& r : rule) {
-        if (clusters > r.clusters * per_sm || d.max_seq_len < r.from || (r.slices % 3 == 0 && d.head_dim <= 64)) continue;
-        if (rows == 1 || r.slices <= most) return std::min(r.slices, most);
-    }
+    const uint32_t per_sm = d.head_dim <= 64 ? 2 : 1, each = rows == 1 && d.head_dim > 64 ? 32 : 96, most = std::max(2u, (d.max_seq_len + each - 1) / each);
+    for (const auto& r : rule)
+        if (r.slices <= most && clusters <= r.clusters * per_sm && d.max_seq_len >= r.from && !(r.slices % 3 == 0 && d.head_dim <= 64)) return r.slices;
     return 1;
 }
 
