@@ -6,7 +6,7 @@
 // products of up to three groups of eight columns take no longer than the stream, without the detour through shared or tensor memory
 // that tcgen05 operands take (dequantised hi + lo halves of int4 weights would be 164 bytes a clock of shared-memory
 // writes, more than an SM has).  What they cost is instructions and fragment reads (a step of 4 rows, one group: 1.82 ms, of 5, two
-// groups: 2.42): 16 x 128 weights (1152 bytes) arrive every 50 clocks, 200 issue slots.
+// groups: 2.45): 16 x 128 weights (1152 bytes) arrive every 50 clocks, 200 issue slots.
 //
 // Weights.  A = 16 weight rows x 16 of K.  int4 group-32: a masked nibble IS an fp16 operand, the subnormal n * 2^-24 (bits 0-3)
 // or n * 2^-20 (bits 4-7, its x is stored divided by 16), exact: one AND per two weights and no conversion.  Groups keep their
@@ -40,8 +40,8 @@
 // step: one wait, one set of addresses, one loop for both.
 //
 // Measured, a step of the 8B shape, ms (as above with int4 weights too, 2..4 int4 rows on vb_gemv_imma.cu -> now): int4, 2 / 3 / 4 / 5 / 8 rows
-// 2.13 / 2.24 / 2.04 / 2.75 / 2.81 -> 1.73 / 1.78 / 1.82 / 2.42 / 2.46; group-64, 1 / 2 / 4 / 8 rows 2.08 / 2.27 / 2.51 / 4.56 -> 1.61 / 1.72 / 2.22 /
-// 4.26 (0.1..0.2 of it at 2 and 3 rows is the attention's).  fp16 gate/up with 4 rows 46.6 us (235 MB: 5.0 TB/s; fp32 kernel 72).
+// 2.16 / 2.24 / 2.06 / 2.74 / 2.79 -> 1.73 / 1.80 / 1.82 / 2.45 / 2.46; group-64, 1 / 2 / 4 / 8 rows 2.09 / 2.26 / 2.52 / 4.55 -> 1.64 / 1.73 / 2.24 /
+// 4.24 (0.1..0.2 of it at 2 and 3 rows is the attention's).  fp16 gate/up with 4 rows 46.6 us (235 MB: 5.0 TB/s; fp32 kernel 72).
 // What bounds the int4 products is issue and latency: ~115 instructions a weight block and 8 columns, IPC 1.9 of 4 in gate/up.
 #include <cooperative_groups.h>
 
