@@ -467,15 +467,16 @@ StepIO decode_io(vb_ctx* c) {
 // 8 layers and the head, us with 2 / 3 / 4 / 6 / 8 slices: 8B int4, contexts of 500, 1 sequence (8 clusters) 369 / 370 / 358 / 360 / 360, 2
 // 498 / 498 / 486 / 492 / 538, 4 526 / 527 / 518 / 570 / 608, 5 696 / 697 / 735 / 742 / 785, 8 701 / 763 / 743 / 800 / 886; of 3000, 1 447 / 421 / 400 /
 // 388 / 378, 2 576 / 549 / 529 / 521 / 578, 5 777 / 752 / 824 / 808 / 856; 7B int8, 3 sequences (12 clusters) of 500 703 / 716 / 701 / 710 / 704, of 3000
-// 778 / 764 / 741 / 736 / 722.  The 135M model, 8 sequences (24 clusters), 2 / 4 / 8: 250 rows 933 / 937 / 957, 3000 1230 / 1081 / 1034; three
-// and six slices of a head of 64 are slower than two and four.  Sixteen for four clusters at most (each takes most of a GPC, and how many GPCs have so many SMs
+// 778 / 764 / 741 / 736 / 722.  The 135M model, 8 sequences (24 clusters), 2 / 4 / 8: 250 rows 933 / 937 / 957, 3000 1230 / 1081 / 1034, 32
+// (96 clusters), 1 / 2: 60 rows 2098 / 2210, 1000 2302 / 2324 (more than a block an SM does not pay there); three and six slices of a head of 64
+// are slower than two and four.  Sixteen for four clusters at most (each takes most of a GPC, and how many GPCs have so many SMs
 // differs from chip to chip): 3000 rows, 8 / 16, 7B int8 572 / 564, 135M 595 / 587; 1000 rows 548 / 559.
 uint32_t pick_attn_splits(const vb_model_desc& d, uint32_t rows, uint32_t clusters) {
     static constexpr struct { uint32_t slices, clusters, from; } rule[] = {{8, 14, 1}, {6, 18, 1024}, {4, 32, 1}, {3, 44, 1}, {2, 74, 1}};
     if (d.max_seq_len >= 2048 && clusters <= 4) return 16;
     const uint32_t per_sm = d.head_dim <= 64 ? 2 : 1, each = rows == 1 && d.head_dim > 64 ? 32 : 96, most = std::max(2u, (d.max_seq_len + each - 1) / each);
     for (const auto& r : rule)
-        if (r.slices <= most && clusters <= r.clusters * per_sm && d.max_seq_len >= r.from && !(r.slices % 3 == 0 && d.head_dim <= 64)) return r.slices;
+        if (r.slices <= most && clusters <= r.clusters * (r.slices > 2 ? per_sm : 1) && d.max_seq_len >= r.from && !(r.slices % 3 == 0 && d.head_dim <= 64)) return r.slices;
     return 1;
 }
 
